@@ -40,14 +40,47 @@ template <typename V>
 __device__ __forceinline__ V csub(V a, V b) {
   return cmk<V>(a.x - b.x, a.y - b.y);
 }
+// FP64 products are written with explicit multiply-adds.  The FP64 kernels are
+// built without contraction (the sweep's decisions round like the oracle's),
+// but the transforms only have to be accurate, and GB300 issues 1.7 FP64
+// operations per SM and cycle (measured; FP32: 118), so an FP64 pass takes as
+// long as its operation count: 4 instead of 6 per complex product, 6 instead
+// of 10 per butterfly with a twiddle (Goedecker, SIAM J. Sci. Comput. 18,
+// 1997), each rounding once less.
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 template <typename V>
 __device__ __forceinline__ V cmul(V a, V b) {
+  if constexpr (sizeof(a.x) == 8) return cmk<V>(fma_rn(a.x, b.x, -(a.y * b.y)), fma_rn(a.x, b.y, a.y * b.x));
   return cmk<V>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 // a * conj(b)
 template <typename V>
 __device__ __forceinline__ V cmulc(V a, V b) {
+  if constexpr (sizeof(a.x) == 8) return cmk<V>(fma_rn(a.x, b.x, a.y * b.y), fma_rn(a.y, b.x, -(a.x * b.y)));
   return cmk<V>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+}
+// acc + a * b, acc + a * conj(b)
+template <typename V>
+__device__ __forceinline__ V cmac(V acc, V a, V b) {
+  if constexpr (sizeof(a.x) == 8)
+    return cmk<V>(fma_rn(-a.y, b.y, fma_rn(a.x, b.x, acc.x)), fma_rn(a.y, b.x, fma_rn(a.x, b.y, acc.y)));
+  return cadd(acc, cmul(a, b));
+}
+template <typename V>
+__device__ __forceinline__ V cmacc(V acc, V a, V b) {
+  if constexpr (sizeof(a.x) == 8)
+    return cmk<V>(fma_rn(a.y, b.y, fma_rn(a.x, b.x, acc.x)), fma_rn(-a.x, b.y, fma_rn(a.y, b.x, acc.y)));
+  return cadd(acc, cmulc(a, b));
+}
+
+// K^ . M^ at one frequency (src/demag_cu.cu:98-111): the real and imaginary
+// parts of sum_b K_ab M_b for a = x, y, z, from the six tensor blocks.
+template <typename V>
+__device__ __forceinline__ V tensor_row(V mx, V my, V mz, V k0, V k1, V k2) {
+  if constexpr (sizeof(mx.x) == 8) return cmac(cmac(cmul(mx, k0), my, k1), mz, k2);
+  return cmk<V>((mx.x * k0.x - mx.y * k0.y) + (my.x * k1.x - my.y * k1.y) + (mz.x * k2.x - mz.y * k2.y),
+                (mx.x * k0.y + mx.y * k0.x) + (my.x * k1.y + my.y * k1.x) + (mz.x * k2.y + mz.y * k2.x));
 }
 
 template <typename T>
@@ -183,7 +216,7 @@ __device__ __noinline__ C<T>* fft_lines(C<T>* a, C<T>* b, int nlines, int stride
           for (int t = 1; t < R; ++t) {
             e += q;
             if (e >= R) e -= R;
-            acc = INV ? cadd(acc, cmulc(v[t], RT[e])) : cadd(acc, cmul(v[t], RT[e]));
+            acc = INV ? cmacc(acc, v[t], RT[e]) : cmac(acc, v[t], RT[e]);
           }
           out[q * Ns] = acc;
         }
@@ -263,6 +296,11 @@ struct RegDft {
       } else {
         const T wr = (T)w32_re(k * (32 / N));
         const T wi = INV ? (T)-w32_im(k * (32 / N)) : (T)w32_im(k * (32 / N));
+        if constexpr (sizeof(T) == 8) {  // e + w o, and e - w o as 2 e - (e + w o)
+          v[k] = cmac(e[k], o[k], cmk<V>(wr, wi));
+          v[k + N / 2] = cmk<V>(fma_rn((T)2, e[k].x, -v[k].x), fma_rn((T)2, e[k].y, -v[k].y));
+          continue;
+        }
         t = cmk<V>(o[k].x * wr - o[k].y * wi, o[k].x * wi + o[k].y * wr);
       }
       v[k] = cadd(e[k], t);
@@ -464,7 +502,7 @@ struct ThreadDft {
             acc = cadd(acc, x[j]);
           } else {
             const V w = rt[e * RS];
-            acc = cadd(acc, INV ? cmulc(x[j], w) : cmul(x[j], w));
+            acc = INV ? cmacc(acc, x[j], w) : cmac(acc, x[j], w);
           }
         }
         v[k] = acc;

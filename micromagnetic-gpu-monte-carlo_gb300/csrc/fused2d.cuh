@@ -232,15 +232,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_const
         V* qy = cur + (size_t)(2 + t) * (Ly + 1) + pos;
         V* qz = cur + (size_t)(4 + t) * (Ly + 1) + pos;
         const V mx = *qx, my = *qy, mz = *qz;
-        T hxr = (mx.x * kxx.x - mx.y * kxx.y) + (my.x * kxy.x - my.y * kxy.y) + (mz.x * kxz.x - mz.y * kxz.y);
-        T hxi = (mx.x * kxx.y + mx.y * kxx.x) + (my.x * kxy.y + my.y * kxy.x) + (mz.x * kxz.y + mz.y * kxz.x);
-        T hyr = (mx.x * kxy.x - mx.y * kxy.y) + (my.x * kyy.x - my.y * kyy.y) + (mz.x * kyz.x - mz.y * kyz.y);
-        T hyi = (mx.x * kxy.y + mx.y * kxy.x) + (my.x * kyy.y + my.y * kyy.x) + (mz.x * kyz.y + mz.y * kyz.x);
-        T hzr = (mx.x * kxz.x - mx.y * kxz.y) + (my.x * kyz.x - my.y * kyz.y) + (mz.x * kzz.x - mz.y * kzz.y);
-        T hzi = (mx.x * kxz.y + mx.y * kxz.x) + (my.x * kyz.y + my.y * kyz.x) + (mz.x * kzz.y + mz.y * kzz.x);
-        *qx = cmk<V>(hxr * P.inv_n, hxi * P.inv_n);
-        *qy = cmk<V>(hyr * P.inv_n, hyi * P.inv_n);
-        *qz = cmk<V>(hzr * P.inv_n, hzi * P.inv_n);
+        const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
+        const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
+        const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
+        *qx = cmk<V>(hx_.x * P.inv_n, hx_.y * P.inv_n);
+        *qy = cmk<V>(hy_.x * P.inv_n, hy_.y * P.inv_n);
+        *qz = cmk<V>(hz_.x * P.inv_n, hz_.y * P.inv_n);
       }
       __syncthreads();
       V* r = fft_run<T, true>(cur, oth, 6, Ly + 1, P.py, twy);

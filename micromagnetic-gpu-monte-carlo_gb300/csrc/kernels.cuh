@@ -421,16 +421,12 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
       V* py = cur + (long long)(1 * ntx + t) * stride + pos;
       V* pz = cur + (long long)(2 * ntx + t) * stride + pos;
       const V mx = *px, my = *py, mz = *pz;
-      // src/demag_cu.cu:98-111: real and imaginary parts of sum_b K_ab M_b, divided by N
-      T hxr = (mx.x * kxx.x - mx.y * kxx.y) + (my.x * kxy.x - my.y * kxy.y) + (mz.x * kxz.x - mz.y * kxz.y);
-      T hxi = (mx.x * kxx.y + mx.y * kxx.x) + (my.x * kxy.y + my.y * kxy.x) + (mz.x * kxz.y + mz.y * kxz.x);
-      T hyr = (mx.x * kxy.x - mx.y * kxy.y) + (my.x * kyy.x - my.y * kyy.y) + (mz.x * kyz.x - mz.y * kyz.y);
-      T hyi = (mx.x * kxy.y + mx.y * kxy.x) + (my.x * kyy.y + my.y * kyy.x) + (mz.x * kyz.y + mz.y * kyz.x);
-      T hzr = (mx.x * kxz.x - mx.y * kxz.y) + (my.x * kyz.x - my.y * kyz.y) + (mz.x * kzz.x - mz.y * kzz.y);
-      T hzi = (mx.x * kxz.y + mx.y * kxz.x) + (my.x * kyz.y + my.y * kyz.x) + (mz.x * kzz.y + mz.y * kzz.x);
-      *px = cmk<V>(hxr * inv_n, hxi * inv_n);
-      *py = cmk<V>(hyr * inv_n, hyi * inv_n);
-      *pz = cmk<V>(hzr * inv_n, hzi * inv_n);
+      const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
+      const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
+      const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
+      *px = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
+      *py = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
+      *pz = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
     }
     __syncthreads();
   }
@@ -559,7 +555,7 @@ __global__ void __launch_bounds__(CR_TX * A) k_col_reg(FftPlan p, C<T>* __restri
     }
   __syncthreads();  // roots
   col_reg_transform3<T, false, A>(v, tb, roots, t, b, true);
-  // src/demag_cu.cu:98-111: real and imaginary parts of sum_b K_ab M_b, divided by N
+  // K^ . M^ / N
 #pragma unroll
   for (int kb = 0; kb < A; ++kb) {
     const int pos = b + A * kb;
@@ -568,15 +564,12 @@ __global__ void __launch_bounds__(CR_TX * A) k_col_reg(FftPlan p, C<T>* __restri
     V kyy = kk[3 * nspec], kyz = kk[4 * nspec], kzz = kk[5 * nspec];
     if (flags & PASS_SYM) kxx.y = kxy.y = kxz.y = kyy.y = kyz.y = kzz.y = (T)0;
     const V mx = v[0][kb], my = v[1][kb], mz = v[2][kb];
-    T hxr = (mx.x * kxx.x - mx.y * kxx.y) + (my.x * kxy.x - my.y * kxy.y) + (mz.x * kxz.x - mz.y * kxz.y);
-    T hxi = (mx.x * kxx.y + mx.y * kxx.x) + (my.x * kxy.y + my.y * kxy.x) + (mz.x * kxz.y + mz.y * kxz.x);
-    T hyr = (mx.x * kxy.x - mx.y * kxy.y) + (my.x * kyy.x - my.y * kyy.y) + (mz.x * kyz.x - mz.y * kyz.y);
-    T hyi = (mx.x * kxy.y + mx.y * kxy.x) + (my.x * kyy.y + my.y * kyy.x) + (mz.x * kyz.y + mz.y * kyz.x);
-    T hzr = (mx.x * kxz.x - mx.y * kxz.y) + (my.x * kyz.x - my.y * kyz.y) + (mz.x * kzz.x - mz.y * kzz.y);
-    T hzi = (mx.x * kxz.y + mx.y * kxz.x) + (my.x * kyz.y + my.y * kyz.x) + (mz.x * kzz.y + mz.y * kzz.x);
-    v[0][kb] = cmk<V>(hxr * inv_n, hxi * inv_n);
-    v[1][kb] = cmk<V>(hyr * inv_n, hyi * inv_n);
-    v[2][kb] = cmk<V>(hzr * inv_n, hzi * inv_n);
+    const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
+    const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
+    const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
+    v[0][kb] = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
+    v[1][kb] = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
+    v[2][kb] = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
   }
   col_reg_transform3<T, true, A>(v, tb, roots, t, b, false);
   if (!ok) return;
@@ -658,7 +651,7 @@ __global__ void __launch_bounds__(3 * CR_TX * A)
   // row c of K^: (xx, xy, xz), (xy, yy, yz) or (xz, yz, zz) in the six blocks
   // xx, xy, xz, yy, yz, zz
   const int o0 = c, o1 = c == 0 ? 1 : c == 1 ? 3 : 4, o2 = c == 0 ? 2 : c == 1 ? 4 : 5;
-  // src/demag_cu.cu:98-111: real and imaginary parts of sum_b K_ab M_b, divided by N
+  // K^ . M^ / N
 #pragma unroll
   for (int kb = 0; kb < A; ++kb) {
     const int pos = b + A * kb;
@@ -667,9 +660,8 @@ __global__ void __launch_bounds__(3 * CR_TX * A)
     if (flags & PASS_SYM) k0.y = k1.y = k2.y = (T)0;
     const int q = kb * RW + b * CR_TX + t;
     const V mx = tb[q], my = tb[A * RW + q], mz = tb[2 * A * RW + q];
-    const T hr = (mx.x * k0.x - mx.y * k0.y) + (my.x * k1.x - my.y * k1.y) + (mz.x * k2.x - mz.y * k2.y);
-    const T hi = (mx.x * k0.y + mx.y * k0.x) + (my.x * k1.y + my.y * k1.x) + (mz.x * k2.y + mz.y * k2.x);
-    v[kb] = cmk<V>(hr * inv_n, hi * inv_n);
+    const V hc = tensor_row(mx, my, mz, k0, k1, k2);
+    v[kb] = cmk<V>(hc.x * inv_n, hc.y * inv_n);
   }
   col_reg_transform1<T, true, A>(v, tbc, roots, t, b, false);
   if (!ok) return;
@@ -719,15 +711,12 @@ __global__ void __launch_bounds__(128) k_col_short(FftPlan p, C<T>* __restrict__
       V kyy = kk[3 * nspec], kyz = kk[4 * nspec], kzz = kk[5 * nspec];
       if (flags & PASS_SYM) kxx.y = kxy.y = kxz.y = kyy.y = kyz.y = kzz.y = (T)0;
       const V mx = v[0][z], my = v[1][z], mz = v[2][z];
-      T hxr = (mx.x * kxx.x - mx.y * kxx.y) + (my.x * kxy.x - my.y * kxy.y) + (mz.x * kxz.x - mz.y * kxz.y);
-      T hxi = (mx.x * kxx.y + mx.y * kxx.x) + (my.x * kxy.y + my.y * kxy.x) + (mz.x * kxz.y + mz.y * kxz.x);
-      T hyr = (mx.x * kxy.x - mx.y * kxy.y) + (my.x * kyy.x - my.y * kyy.y) + (mz.x * kyz.x - mz.y * kyz.y);
-      T hyi = (mx.x * kxy.y + mx.y * kxy.x) + (my.x * kyy.y + my.y * kyy.x) + (mz.x * kyz.y + mz.y * kyz.x);
-      T hzr = (mx.x * kxz.x - mx.y * kxz.y) + (my.x * kyz.x - my.y * kyz.y) + (mz.x * kzz.x - mz.y * kzz.y);
-      T hzi = (mx.x * kxz.y + mx.y * kxz.x) + (my.x * kyz.y + my.y * kyz.x) + (mz.x * kzz.y + mz.y * kzz.x);
-      v[0][z] = cmk<V>(hxr * inv_n, hxi * inv_n);
-      v[1][z] = cmk<V>(hyr * inv_n, hyi * inv_n);
-      v[2][z] = cmk<V>(hzr * inv_n, hzi * inv_n);
+      const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
+      const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
+      const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
+      v[0][z] = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
+      v[1][z] = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
+      v[2][z] = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
     }
   }
   if (flags & PASS_INV) {
