@@ -36,6 +36,7 @@ GXX_COMMON = ["g++", "-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall",
 UNITS = [
     ("kernels_f32.cu", ["-fmad=true"], "nvcc"),
     ("kernels_f64.cu", ["-fmad=false"], "nvcc"),
+    ("kernels_f64s.cu", ["-fmad=false"], "nvcc"),
     ("newell.cu", ["-fmad=false"], "nvcc"),
     ("demag_static.cu", [], "nvcc"),
     ("runtime.cpp", [], "g++"),

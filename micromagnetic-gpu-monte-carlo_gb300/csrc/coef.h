@@ -28,6 +28,37 @@ struct McParams {
 #define MMC_COEF_HD
 #endif
 
+// The FP32 filter's coefficients from the FP64 ones.  |F_a| of a trial is at
+// most (2 sum wex + 2 sum |wdm| + 3 k0h (1 + 1) + 2 can (1 + 1)) max(1, |m|) +
+// |cz| + cd |h|, components at most max(1, |m|) and |h|.
+MMC_COEF_HD inline McFilter mc_filter_from(const McCoef<double>& k) {
+  McFilter f;
+  double g = 0, kmax = 0, cmax = 0;
+  for (int a = 0; a < 3; ++a) {
+    f.wex[a] = (float)k.wex[a];
+    f.u[a] = (float)k.u[a];
+    f.cz[a] = (float)k.cz[a];
+    g += 2.0 * (k.wex[a] < 0 ? -k.wex[a] : k.wex[a]);
+    const double z = k.cz[a] < 0 ? -k.cz[a] : k.cz[a];
+    if (!(z <= cmax)) cmax = z;
+  }
+  for (int a = 0; a < 2; ++a) {
+    f.wdm[a] = (float)k.wdm[a];
+    g += 2.0 * (k.wdm[a] < 0 ? -k.wdm[a] : k.wdm[a]);
+  }
+  for (int q = 0; q < 6; ++q) {
+    f.k0h[q] = (float)k.k0h[q];
+    const double z = k.k0h[q] < 0 ? -k.k0h[q] : k.k0h[q];
+    if (!(z <= kmax)) kmax = z;
+  }
+  f.can = (float)k.can;
+  f.cd = (float)k.cd;
+  g += 6.0 * kmax + 4.0 * (k.can < 0 ? -k.can : k.can);
+  f.gm = (float)(1.001 * g);
+  f.gc = (float)(1.001 * cmax);
+  return f;
+}
+
 template <typename T>
 MMC_COEF_HD inline McCoef<T> mc_coef_from(const McParams& p, double T_K) {
   const double kB = 1.3806488e-23;  // src/constant.h:22
@@ -46,6 +77,7 @@ MMC_COEF_HD inline McCoef<T> mc_coef_from(const McParams& p, double T_K) {
   for (int q = 0; q < 6; ++q) k.k0h[q] = (T)(p.demag ? 0.5 * (p.mu0 * p.ms * p.ms * p.v / kT) * p.k0[q] : 0.0);
   k.key0 = p.key0;
   k.key1 = p.key1;
+  if constexpr (sizeof(T) == 8) k.f = mc_filter_from(k);
   return k;
 }
 

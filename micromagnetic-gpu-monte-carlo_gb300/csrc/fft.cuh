@@ -22,8 +22,31 @@ template <>
 struct Cplx<double> {
   using type = double2;
 };
+// FP64 whose products are never contracted into multiply-adds: the transforms
+// of the relaxation (see launch_demag_sym) use it in place of double.
+struct f64s {
+  double v;
+  f64s() = default;
+  __host__ __device__ __forceinline__ f64s(double d) : v(d) {}
+};
+#if defined(__CUDACC__)
+__device__ __forceinline__ f64s operator+(f64s a, f64s b) { return __dadd_rn(a.v, b.v); }
+__device__ __forceinline__ f64s operator-(f64s a, f64s b) { return __dadd_rn(a.v, -b.v); }
+__device__ __forceinline__ f64s operator*(f64s a, f64s b) { return __dmul_rn(a.v, b.v); }
+__device__ __forceinline__ f64s operator-(f64s a) { return -a.v; }
+#endif
+struct alignas(16) f64s2 {
+  f64s x, y;
+};
+template <>
+struct Cplx<f64s> {
+  using type = f64s2;
+};
 template <typename T>
 using C = typename Cplx<T>::type;
+// double proper: products written with explicit multiply-adds
+template <typename V>
+constexpr bool fused_mul = sizeof(V) == sizeof(double2) && !__is_same(V, f64s2);
 
 template <typename V>
 __device__ __forceinline__ V cmk(decltype(V::x) a, decltype(V::x) b) {
@@ -48,28 +71,27 @@ __device__ __forceinline__ V csub(V a, V b) {
 // of 10 per butterfly with a twiddle (Goedecker, SIAM J. Sci. Comput. 18,
 // 1997), each rounding once less.
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 template <typename V>
 __device__ __forceinline__ V cmul(V a, V b) {
-  if constexpr (sizeof(a.x) == 8) return cmk<V>(fma_rn(a.x, b.x, -(a.y * b.y)), fma_rn(a.x, b.y, a.y * b.x));
+  if constexpr (fused_mul<V>) return cmk<V>(fma_rn(a.x, b.x, -(a.y * b.y)), fma_rn(a.x, b.y, a.y * b.x));
   return cmk<V>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 // a * conj(b)
 template <typename V>
 __device__ __forceinline__ V cmulc(V a, V b) {
-  if constexpr (sizeof(a.x) == 8) return cmk<V>(fma_rn(a.x, b.x, a.y * b.y), fma_rn(a.y, b.x, -(a.x * b.y)));
+  if constexpr (fused_mul<V>) return cmk<V>(fma_rn(a.x, b.x, a.y * b.y), fma_rn(a.y, b.x, -(a.x * b.y)));
   return cmk<V>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 // acc + a * b, acc + a * conj(b)
 template <typename V>
 __device__ __forceinline__ V cmac(V acc, V a, V b) {
-  if constexpr (sizeof(a.x) == 8)
+  if constexpr (fused_mul<V>)
     return cmk<V>(fma_rn(-a.y, b.y, fma_rn(a.x, b.x, acc.x)), fma_rn(a.y, b.x, fma_rn(a.x, b.y, acc.y)));
   return cadd(acc, cmul(a, b));
 }
 template <typename V>
 __device__ __forceinline__ V cmacc(V acc, V a, V b) {
-  if constexpr (sizeof(a.x) == 8)
+  if constexpr (fused_mul<V>)
     return cmk<V>(fma_rn(a.y, b.y, fma_rn(a.x, b.x, acc.x)), fma_rn(-a.x, b.y, fma_rn(a.y, b.x, acc.y)));
   return cadd(acc, cmulc(a, b));
 }
@@ -78,7 +100,7 @@ __device__ __forceinline__ V cmacc(V acc, V a, V b) {
 // parts of sum_b K_ab M_b for a = x, y, z, from the six tensor blocks.
 template <typename V>
 __device__ __forceinline__ V tensor_row(V mx, V my, V mz, V k0, V k1, V k2) {
-  if constexpr (sizeof(mx.x) == 8) return cmac(cmac(cmul(mx, k0), my, k1), mz, k2);
+  if constexpr (fused_mul<V>) return cmac(cmac(cmul(mx, k0), my, k1), mz, k2);
   return cmk<V>((mx.x * k0.x - mx.y * k0.y) + (my.x * k1.x - my.y * k1.y) + (mz.x * k2.x - mz.y * k2.y),
                 (mx.x * k0.y + mx.y * k0.x) + (my.x * k1.y + my.y * k1.x) + (mz.x * k2.y + mz.y * k2.x));
 }
@@ -92,6 +114,10 @@ __device__ __forceinline__ const float2* plan_tw<float>(const FftPlan& p) {
 template <>
 __device__ __forceinline__ const double2* plan_tw<double>(const FftPlan& p) {
   return p.tw64;
+}
+template <>
+__device__ __forceinline__ const f64s2* plan_tw<f64s>(const FftPlan& p) {
+  return reinterpret_cast<const f64s2*>(p.tw64);
 }
 
 // Copies the plan's twiddle table into shared memory (call before the FFT,
@@ -296,7 +322,7 @@ struct RegDft {
       } else {
         const T wr = (T)w32_re(k * (32 / N));
         const T wi = INV ? (T)-w32_im(k * (32 / N)) : (T)w32_im(k * (32 / N));
-        if constexpr (sizeof(T) == 8) {  // e + w o, and e - w o as 2 e - (e + w o)
+        if constexpr (fused_mul<V>) {  // e + w o, and e - w o as 2 e - (e + w o)
           v[k] = cmac(e[k], o[k], cmk<V>(wr, wi));
           v[k + N / 2] = cmk<V>(fma_rn((T)2, e[k].x, -v[k].x), fma_rn((T)2, e[k].y, -v[k].y));
           continue;

@@ -805,15 +805,24 @@ struct Prop;
 
 template <>
 struct Prop<double> {
-  __device__ static void draw(mmcm::u32x4 r, double& px, double& py, double& pz, double& ua) {
-    pz = 2.0 * mmcm::u01_f64(r.x) - 1.0;
-    double t = 1.0 - pz * pz;
-    if (t < 0) t = 0;
-    double s = mmcm::dsqrt(t), sn, cs;
-    mmcm::sincospi(2.0 * mmcm::u01_f64(r.y), &sn, &cs);
+  static __device__ __forceinline__ double ticks(int j) {  // j 2^-32, exact
+    return __longlong_as_double(0x4138000000000000ll + (long long)j) - 0x1.8p20;
+  }
+  // The direction of the random words rx, ry: z = 2 u0 - 1, phi = 2 pi u1 with
+  // u = (r + 1/2) 2^-32.  The steps of mmcm::u01_f64 and mmcm::sincospi, bit
+  // for bit; what they do exactly (the uniforms, the split of 2 u1 into
+  // quadrants) is done on the integers, which leaves 60 FP64 operations.
+  static __device__ __forceinline__ void direction(uint32_t rx, uint32_t ry, double& px, double& py, double& pz) {
+    // (2 rx + 1 - 2^32) 2^-32: twice the signed word, 33 bits wide
+    pz = __longlong_as_double(0x4138000000000000ll + 2 * (long long)(int)(rx ^ 0x80000000u) + 1) - 0x1.8p20;
+    const double t = 1.0 - pz * pz;  // >= 0: |pz| < 1
+    const double s = mmcm::dsqrt(t);
+    const uint32_t n2 = (ry >> 30) + ((ry >> 29) & 1u);
+    const double r = ticks((int)(2u * ry + 1u - (n2 << 31)));
+    double sn, cs;
+    mmcm::sincospi_reduced((int)(n2 & 3u), r, &sn, &cs);
     px = s * cs;
     py = s * sn;
-    ua = mmcm::u01_f64(r.z);
   }
   __device__ static bool accept(double dE, double ua) { return dE <= 0.0 || ua < mmcm::exp(-dE); }
 };
@@ -846,10 +855,23 @@ struct Nbrs {
 };
 
 // Proposal of one trial: Philox4x32-10(key = seed; counter = (cell, sweep,
-// stage, 0)) -> direction m' and acceptance uniform ua.
+// stage, 0)).  FP32: the direction m' and the acceptance uniform; FP64: the
+// random words, from which the direction is made for accepted trials only.
 template <typename T>
 struct Proposal {
   T x, y, z, ua;
+  __device__ __forceinline__ void get(T& px, T& py, T& pz) const {
+    px = x;
+    py = y;
+    pz = z;
+  }
+};
+template <>
+struct Proposal<double> {
+  uint32_t rx, ry, rz;
+  __device__ __forceinline__ void get(double& px, double& py, double& pz) const {
+    Prop<double>::direction(rx, ry, px, py, pz);
+  }
 };
 
 template <typename T>
@@ -857,16 +879,113 @@ __device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t c
   mmcm::u32x4 ctr = {cell, sweep, stage, mmcm::STREAM_SWEEP};
   mmcm::u32x4 r = mmcm::philox4x32_10(ctr, c.key0, c.key1);
   Proposal<T> p;
-  Prop<T>::draw(r, p.x, p.y, p.z, p.ua);
+  if constexpr (sizeof(T) == 8) {
+    p.rx = r.x;
+    p.ry = r.y;
+    p.rz = r.z;
+  } else {
+    Prop<T>::draw(r, p.x, p.y, p.z, p.ua);
+  }
   return p;
+}
+
+// ---------------------------------------------- the FP64 trial's FP32 filter
+// GB300 issues 1.7 FP64 operations per SM and cycle, so an FP64 trial costs
+// what its FP64 operations cost: about 230 when everything is evaluated
+// (60 for the direction, 110 for dE, 50 for the exponential).  The filter
+// evaluates the same trial in FP32 with a bound on the distance from what the
+// FP64 formula gives and decides when the bound allows only one answer; the
+// FP64 formula decides the rest.  The decisions are the FP64 formula's, all of
+// them.
+//
+// The bound: with M >= every |component| of m involved (at least 1), H the
+// same for h, and G = gm M + gc + |cd| H >= |F_a| for each component of the
+// field (McFilter), dE = -d . F with |d_a| <= 1 + M, evaluated in the regrouped
+// form of mc_accept<float>.  Its FP32 evaluation sums at most 40 roundings of
+// 2^-24 on any path from an input to dE (2 for a truncated input, 1 for a
+// coefficient, at most 30 in the sums of F and of the dot product), each on
+// terms that add up to at most 3 (1 + M) G: 7.2e-6 (1 + M) G.  The direction's
+// components are off by less than 1e-6 (hardware sine and cosine: 2^-21.19 on
+// [-pi, pi], the angle's own rounding 2e-7; the rest rounds to a few 2^-24),
+// which changes dE by less than 3 x 1e-6 x 2 G.  FP64 rounding is 1e-9 of
+// either.  MC_FILTER_EPS = 1.6e-5 times (1 + M) G covers the sum 1.4e-5.
+// exp: the hardware's is within 2 + 1.173 |x| ulp, 4.5e-6 for x >= -30; below
+// that the smallest uniform (2^-33) decides alone.  MC_FILTER_EXP = 2e-5 covers
+// it and the rounding of the uniform.  NaN or infinity anywhere leaves both
+// comparisons false: unsure.
+constexpr float MC_FILTER_EPS = 1.6e-5f;
+constexpr float MC_FILTER_EXP = 2e-5f;
+enum McVerdict : int { MC_REJECT = 0, MC_ACCEPT = 1, MC_UNSURE = 2 };
+
+// x truncated to FP32 by integer operations (a conversion instruction runs at
+// the FP64 rate): below 2^-126 a denormal or 0, from 2^128 on NaN or infinity.
+__device__ __forceinline__ float f32_trunc(double x) {
+  const int hi = __double2hiint(x);
+  const int e = __vimin_s32_relu((hi & 0x7fffffff) - 0x38000000, 0x0fffffff);
+  const unsigned b = __funnelshift_l((unsigned)__double2loint(x), (unsigned)e, 3);
+  return __uint_as_float(b | ((unsigned)hi & 0x80000000u));
+}
+__device__ __forceinline__ float f32_trunc(float x) { return x; }
+
+// Neighbour values v (meaningful where has is true) and their flags, own cell
+// o, demag field h (0 when the demag term is off).
+__device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&v)[3][2][3], const bool (&has)[3][2],
+                                               float ox, float oy, float oz, float hx, float hy, float hz,
+                                               uint32_t rx, uint32_t ry, uint32_t rz) {
+  float Fx = c.cz[0], Fy = c.cz[1], Fz = c.cz[2];
+  float M = fmaxf(fmaxf(fabsf(ox), fabsf(oy)), fmaxf(fabsf(oz), 1.0f));
+  // NaN does not survive fmaxf: a sum that it does survive joins the bound
+  float nan0 = 0.0f * (ox + oy + oz);
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      if (!has[a][s]) continue;
+      const float x = v[a][s][0], y = v[a][s][1], z = v[a][s][2];
+      Fx = fmaf(c.wex[a], x, Fx);
+      Fy = fmaf(c.wex[a], y, Fy);
+      Fz = fmaf(c.wex[a], z, Fz);
+      M = fmaxf(M, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))));
+      if (a < 2) {  // DMI: (d_x m_z, d_y m_z, -d_x m_x - d_y m_y)
+        const float w = s ? c.wdm[a] : -c.wdm[a];
+        if (a == 0) Fx = fmaf(w, z, Fx);
+        if (a == 1) Fy = fmaf(w, z, Fy);
+        Fz = fmaf(-w, a == 0 ? x : y, Fz);
+      }
+    }
+  const float a0 = fmaf((float)rx, 0x1p-31f, 0x1p-32f), a1 = fmaf((float)~rx, 0x1p-31f, 0x1p-32f);  // 1 + z, 1 - z
+  const float t = a0 * a1;
+  const float r = t * rsqrtf(t);
+  float sn, cs;
+  __sincosf((float)(int)(ry ^ 0x80000000u) * (3.14159265358979323846f * 0x1p-31f), &sn, &cs);
+  const float px = -(r * cs), py = -(r * sn), pz = (float)(int)(rx ^ 0x80000000u) * 0x1p-31f;
+  const float dx = px - ox, dy = py - oy, dz = pz - oz;
+  Fx = fmaf(c.cd, hx, Fx) + fmaf(c.k0h[0], dx, fmaf(c.k0h[1], dy, c.k0h[2] * dz));
+  Fy = fmaf(c.cd, hy, Fy) + fmaf(c.k0h[1], dx, fmaf(c.k0h[3], dy, c.k0h[4] * dz));
+  Fz = fmaf(c.cd, hz, Fz) + fmaf(c.k0h[2], dx, fmaf(c.k0h[4], dy, c.k0h[5] * dz));
+  const float su = fmaf(px + ox, c.u[0], fmaf(py + oy, c.u[1], (pz + oz) * c.u[2]));
+  const float cu = c.can * su;
+  Fx = fmaf(cu, c.u[0], Fx);
+  Fy = fmaf(cu, c.u[1], Fy);
+  Fz = fmaf(cu, c.u[2], Fz);
+  const float mdE = fmaf(dx, Fx, fmaf(dy, Fy, dz * Fz));  // -dE
+  const float H = fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz)));
+  nan0 += 0.0f * mdE;
+  const float eps = fmaf(MC_FILTER_EPS * (1.0f + M), fmaf(c.gm, M, fmaf(fabsf(c.cd), H, c.gc)), nan0);
+  const float ua = fmaf((float)rz, 0x1p-32f, 0x1p-33f);
+  const float lo = mdE - eps, hi = fmaxf(mdE + eps, -30.0f);
+  if (lo >= 0.0f || ua * (1.0f + MC_FILTER_EXP) < __expf(lo)) return MC_ACCEPT;
+  // fmaxf drops a NaN: ask for a finite bound as well
+  if (eps < 1e30f && ua > (1.0f + MC_FILTER_EXP) * __expf(hi)) return MC_REJECT;
+  return MC_UNSURE;
 }
 
 // The Metropolis decision for one cell from its neighbour values, its own m,
 // its demag field h and its proposal.  Shared by every sweep kernel so that
 // all paths round identically.
 template <typename T>
-__device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy, T hz,
-                                          const Proposal<T>& p) {
+__device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy,
+                                                  T hz, T px, T py, T pz, T ua) {
   T Fx = 0, Fy = 0, Fz = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -893,18 +1012,18 @@ __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb,
     //   dE = -d . [F_local + cd h + (cd / 2) K0 d + can (s . u) u],
     // where F_local is the exchange, DMI and Zeeman part of F: the terms in
     // K0 m cancel, and the quadratic forms need no difference of squares.
-    const T ddx = p.x - ox, ddy = p.y - oy, ddz = p.z - oz;
+    const T ddx = px - ox, ddy = py - oy, ddz = pz - oz;
     if (c.cd != (T)0) {
       Fx = Fx + c.cd * hx + (c.k0h[0] * ddx + c.k0h[1] * ddy + c.k0h[2] * ddz);
       Fy = Fy + c.cd * hy + (c.k0h[1] * ddx + c.k0h[3] * ddy + c.k0h[4] * ddz);
       Fz = Fz + c.cd * hz + (c.k0h[2] * ddx + c.k0h[4] * ddy + c.k0h[5] * ddz);
     }
-    const T su = (p.x + ox) * c.u[0] + (p.y + oy) * c.u[1] + (p.z + oz) * c.u[2];
+    const T su = (px + ox) * c.u[0] + (py + oy) * c.u[1] + (pz + oz) * c.u[2];
     const T cs = c.can * su;
     Fx = Fx + cs * c.u[0];
     Fy = Fy + cs * c.u[1];
     Fz = Fz + cs * c.u[2];
-    return Prop<T>::accept(-(ddx * Fx + ddy * Fy + ddz * Fz), p.ua);
+    return Prop<T>::accept(-(ddx * Fx + ddy * Fy + ddz * Fz), ua);
   }
   if (c.cd != (T)0) {
     const T sx = c.k0[0] * ox + c.k0[1] * oy + c.k0[2] * oz;
@@ -914,7 +1033,6 @@ __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb,
     Fy = Fy + c.cd * (hy - sy);
     Fz = Fz + c.cd * (hz - sz);
   }
-  const T px = p.x, py = p.y, pz = p.z;
   const T ddx = px - ox, ddy = py - oy, ddz = pz - oz;
   T dE = -(ddx * Fx + ddy * Fy + ddz * Fz);
   const T pun = px * c.u[0] + py * c.u[1] + pz * c.u[2];
@@ -927,17 +1045,61 @@ __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb,
                  oz * (c.k0[2] * ox + c.k0[4] * oy + c.k0[5] * oz);
     dE = dE - (T)0.5 * c.cd * (qn - qo);
   }
-  return Prop<T>::accept(dE, p.ua);
+  return Prop<T>::accept(dE, ua);
 }
 
+// The decision; p's direction is the new m where it is true.
 template <typename T>
-__device__ __forceinline__ bool mc_decide(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy, T hz,
-                                          uint32_t cell, uint32_t stage, uint32_t sweep, T& px, T& py, T& pz) {
-  const Proposal<T> p = mc_propose<T>(c, cell, stage, sweep);
-  px = p.x;
-  py = p.y;
-  pz = p.z;
-  return mc_accept<T>(c, nb, ox, oy, oz, hx, hy, hz, p);
+__device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy, T hz,
+                                          const Proposal<T>& p) {
+  if constexpr (sizeof(T) == 8) {
+    float v[3][2][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[a][s][k] = f32_trunc(nb.v[a][s][k]);
+    const McVerdict w = mc_filter(c.f, v, nb.has, f32_trunc(ox), f32_trunc(oy), f32_trunc(oz), f32_trunc(hx),
+                                  f32_trunc(hy), f32_trunc(hz), p.rx, p.ry, p.rz);
+    if (w != MC_UNSURE) return w == MC_ACCEPT;
+    T px, py, pz;
+    p.get(px, py, pz);
+    return mc_accept_formula<T>(c, nb, ox, oy, oz, hx, hy, hz, px, py, pz, mmcm::u01_f64(p.rz));
+  } else {
+    return mc_accept_formula<T>(c, nb, ox, oy, oz, hx, hy, hz, p.x, p.y, p.z, p.ua);
+  }
+}
+
+// The neighbours of cell i = (x, y, z), read as U (T, or float for the filter).
+template <typename T, typename U>
+__device__ __forceinline__ U mc_read(const T* p) {
+  if constexpr (sizeof(T) == sizeof(U)) return *p;
+  else return f32_trunc(*p);
+}
+template <typename T, typename U>
+__device__ __forceinline__ void mc_nbrs(const Geom& g, const T* __restrict__ m, long long i, int x, int y, int z,
+                                        Nbrs<U>& nb) {
+  const T* mx = m;
+  const T* my = m + g.n;
+  const T* mz = m + 2 * g.n;
+  const bool film = g.nz == 1;  // no z bonds: skip their index work and loads
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      if (a == 2 && film) {
+        nb.has[a][s] = false;
+        nb.v[a][s][0] = nb.v[a][s][1] = nb.v[a][s][2] = (U)0;
+        continue;
+      }
+      const long long j = nbr_step(g, i, x, y, z, a, s ? 1 : -1);
+      nb.has[a][s] = j >= 0;
+      const long long jj = j >= 0 ? j : i;
+      nb.v[a][s][0] = mc_read<T, U>(mx + jj);
+      nb.v[a][s][1] = mc_read<T, U>(my + jj);
+      nb.v[a][s][2] = mc_read<T, U>(mz + jj);
+    }
 }
 
 template <typename T>
@@ -951,33 +1113,17 @@ __device__ __forceinline__ bool mc_trial(const Geom& g, const McCoef<T>& c, T* _
   const long long i = x + (long long)g.nx * (y + (long long)g.ny * z);
   const T ox = mx[i], oy = my[i], oz = mz[i];
   Nbrs<T> nb;
-  const bool film = g.nz == 1;  // no z bonds: skip their index work and loads
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      if (a == 2 && film) {
-        nb.has[a][s] = false;
-        nb.v[a][s][0] = ox;
-        nb.v[a][s][1] = oy;
-        nb.v[a][s][2] = oz;
-        continue;
-      }
-      const long long j = nbr_step(g, i, x, y, z, a, s ? 1 : -1);
-      nb.has[a][s] = j >= 0;
-      const long long jj = j >= 0 ? j : i;
-      nb.v[a][s][0] = mx[jj];
-      nb.v[a][s][1] = my[jj];
-      nb.v[a][s][2] = mz[jj];
-    }
+  mc_nbrs<T, T>(g, m, i, x, y, z, nb);
   T hx = 0, hy = 0, hz = 0;
   if (c.cd != (T)0) {
     hx = h[i];
     hy = h[n + i];
     hz = h[2 * n + i];
   }
-  T px, py, pz;
-  if (mc_decide<T>(c, nb, ox, oy, oz, hx, hy, hz, (uint32_t)i, stage, sweep, px, py, pz)) {
+  const Proposal<T> p = mc_propose<T>(c, (uint32_t)i, stage, sweep);
+  if (mc_accept<T>(c, nb, ox, oy, oz, hx, hy, hz, p)) {
+    T px, py, pz;
+    p.get(px, py, pz);
     mx[i] = px;
     my[i] = py;
     mz[i] = pz;
@@ -1030,6 +1176,112 @@ __global__ void __launch_bounds__(256, 4) k_mc_general(Geom g, const McCoef<T>* 
     if (cell_color(g, x, y, z) == color) accepted = mc_trial<T>(g, c, m, h, ctr->stage, ctr->sweep, x, y, z);
   }
   count_accepts(accepted, acc);
+}
+
+// One colour of an FP64 sweep (any lattice).  A thread judges MCL_TPT trials by
+// the FP32 filter (mc_filter); the accepted and the unsure ones go to a list
+// in shared memory, and the CTA then takes the list with full warps: the
+// direction (60 FP64 operations) is made for those trials only, and the FP64
+// formula decides the unsure ones.  Cells of one colour do not see each other,
+// so the stores may come after all of the CTA's decisions.  Bound by FP64
+// issue (1.7 operations per SM and cycle): per trial 60 x the acceptance rate
+// instead of the 230 that every lane of a warp paid.
+constexpr int MCL_THREADS = 128;
+template <int TPT>
+__global__ void __launch_bounds__(MCL_THREADS) k_mc_list(Geom g, const McCoef<double>* __restrict__ cp,
+                                                         double* __restrict__ m, const double* __restrict__ h,
+                                                         const SweepCounters* __restrict__ ctr, int color,
+                                                         unsigned long long* acc) {
+  __shared__ uint4 list[MCL_THREADS * TPT];  // cell (top bit: unsure), random words
+  __shared__ int count;
+  if (threadIdx.x == 0) count = 0;
+  pdl_wait();
+  const McCoef<double>& c = cp[blockIdx.z];
+  const long long n = g.n;
+  m += blockIdx.z * 3 * n;
+  h += blockIdx.z * 3 * n;
+  const uint32_t stage = ctr->stage, sweep = ctr->sweep;
+  const bool dm = c.cd != 0.0;
+  const bool two = g.ncolors == 2;
+  const int hxc = (g.nx + 1) >> 1;
+  const int total = two ? g.ny * g.nz * hxc : (int)n;  // fits: n < 2^31
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < TPT; ++u) {
+    const long long tl = ((long long)blockIdx.x * TPT + u) * MCL_THREADS + threadIdx.x;
+    McVerdict w = MC_REJECT;
+    Proposal<double> p{};
+    int cell = 0;
+    if (tl < total) {
+      const int t = (int)tl;
+      int x, y, z, row;
+      bool mine;
+      if (two) {
+        row = g.dhxc.div(t);
+        z = g.dny.div(row);
+        y = row - z * g.ny;
+        x = 2 * (t - row * hxc) + ((color + y + z) & 1);
+        mine = x < g.nx;
+      } else {
+        row = g.dnx.div(t);
+        x = t - row * g.nx;
+        z = g.dny.div(row);
+        y = row - z * g.ny;
+        mine = cell_color(g, x, y, z) == color;
+      }
+      if (mine) {
+        cell = x + g.nx * row;
+        Nbrs<float> nb;
+        mc_nbrs<double, float>(g, m, cell, x, y, z, nb);
+        float hx = 0, hy = 0, hz = 0;
+        if (dm) {
+          hx = f32_trunc(h[cell]);
+          hy = f32_trunc(h[n + cell]);
+          hz = f32_trunc(h[2 * n + cell]);
+        }
+        p = mc_propose<double>(c, (uint32_t)cell, stage, sweep);
+        w = mc_filter(c.f, nb.v, nb.has, f32_trunc(m[cell]), f32_trunc(m[n + cell]), f32_trunc(m[2 * n + cell]), hx,
+                      hy, hz, p.rx, p.ry, p.rz);
+      }
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, w != MC_REJECT);
+    if (mask) {
+      const int lane = threadIdx.x & 31;
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&count, __popc(mask));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (w != MC_REJECT)
+        list[base + __popc(mask & ((1u << lane) - 1u))] =
+            make_uint4((uint32_t)cell | (w == MC_UNSURE ? 0x80000000u : 0u), p.rx, p.ry, p.rz);
+    }
+  }
+  __syncthreads();
+  const int cnt = count;
+  for (int i0 = 0; i0 < cnt; i0 += MCL_THREADS) {
+    const int i = i0 + threadIdx.x;
+    bool ok = i < cnt;
+    if (ok) {
+      const uint4 e = list[i];
+      const int cell = (int)(e.x & 0x7fffffffu);
+      double px, py, pz;
+      Prop<double>::direction(e.y, e.z, px, py, pz);
+      if (e.x >> 31) {
+        const int row = g.dnx.div(cell), x = cell - row * g.nx;
+        const int z = g.dny.div(row), y = row - z * g.ny;
+        Nbrs<double> nb;
+        mc_nbrs<double, double>(g, m, cell, x, y, z, nb);
+        ok = mc_accept_formula<double>(c, nb, m[cell], m[n + cell], m[2 * n + cell], dm ? h[cell] : 0.0,
+                                       dm ? h[n + cell] : 0.0, dm ? h[2 * n + cell] : 0.0, px, py, pz,
+                                       mmcm::u01_f64(e.w));
+      }
+      if (ok) {
+        m[cell] = px;
+        m[n + cell] = py;
+        m[2 * n + cell] = pz;
+      }
+    }
+    count_accepts(ok, acc + blockIdx.z);
+  }
 }
 
 // One colour of a two-colour film sweep (nz = 1, nx a multiple of 4) with
@@ -1103,9 +1355,7 @@ __device__ __forceinline__ bool quad_cells(const McCoef<T>& c, Vec4<T> (&own)[3]
     }
     const Proposal<T> pr = mc_propose<T>(c, cell0 + (uint32_t)o, stage, sweep);
     if (mc_accept<T>(c, nb, own[0].v[o], own[1].v[o], own[2].v[o], hh[0].v[o], hh[1].v[o], hh[2].v[o], pr)) {
-      own[0].v[o] = pr.x;
-      own[1].v[o] = pr.y;
-      own[2].v[o] = pr.z;
+      pr.get(own[0].v[o], own[1].v[o], own[2].v[o]);
       changed = true;
       ++mine;
     }
@@ -1666,9 +1916,7 @@ __global__ void __launch_bounds__(256) k_mc_tile(Geom g, const McCoef<T>* __rest
     const T* hp = sh + (by - 1) * MCT_H + (bx - 1);
     const Proposal<T> p = mc_propose<T>(c, (uint32_t)(gx + g.nx * gy), stage, sweep);
     if (mc_accept<T>(c, nb, own[0], own[BB], own[2 * BB], hp[0], hp[HH], hp[2 * HH], p)) {
-      own[0] = p.x;
-      own[BB] = p.y;
-      own[2 * BB] = p.z;
+      p.get(own[0], own[BB], own[2 * BB]);
       return true;
     }
     return false;
@@ -1789,9 +2037,7 @@ __device__ __forceinline__ bool strip_trial(const Geom& g, const McCoef<T>& c, T
   }
   const Proposal<T> p = mc_propose<T>(c, (uint32_t)(y * nx + x), stage, sweep);
   if (mc_accept<T>(c, nb, ov[0], ov[1], ov[2], hx, hy, hz, p)) {
-    own[0] = p.x;
-    own[nx] = p.y;
-    own[2 * nx] = p.z;
+    p.get(own[0], own[nx], own[2 * nx]);
     return true;
   }
   return false;
@@ -2247,7 +2493,7 @@ inline size_t x_pass_w_smem(const FftPlan& p, int rows, size_t csize) {
 // device's opt-in maximum.  Called once per device at handle creation, never
 // inside a stream capture.
 template <typename T>
-cudaError_t prepare_impl(int max_dyn_smem) {
+cudaError_t prepare_passes(int max_dyn_smem) {
   const void* fns[] = {(const void*)k_x_forward<T, false, 3>, (const void*)k_x_forward<T, true, 3>,
                        (const void*)k_x_forward<T, false, 6>, (const void*)k_x_forward<T, true, 6>,
                        (const void*)k_x_inverse<T, false>, (const void*)k_x_inverse<T, true>,
@@ -2263,12 +2509,6 @@ cudaError_t prepare_impl(int max_dyn_smem) {
     MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
     MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
   }
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)mc_tile_smem<T>()));
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_band<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)MC_BAND_SMEM_MAX));
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_band<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)MC_BAND_SMEM_MAX));
   MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)col_reg_smem<T, 16>()));
   MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2277,6 +2517,17 @@ cudaError_t prepare_impl(int max_dyn_smem) {
                                     (int)col_reg_smem<T, 16>()));
   MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)col_reg_smem<T, 8>()));
+  return cudaSuccess;
+}
+template <typename T>
+cudaError_t prepare_impl(int max_dyn_smem) {
+  MMC_TRY_ATTR(prepare_passes<T>(max_dyn_smem));
+  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)mc_tile_smem<T>()));
+  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_band<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)MC_BAND_SMEM_MAX));
+  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_band<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)MC_BAND_SMEM_MAX));
   MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_strip<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     max_dyn_smem));
   MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_mc_strip<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2495,7 +2746,15 @@ cudaError_t mc_impl(const Geom& g, const McCoef<T>* c, T* m, const T* h, const S
                          : (mc_all_bonds(g) ? k_mc_quad<T, true, false> : k_mc_quad<T, false, false>);
     return launch_pdl(kern, grid, dim3(qthreads), 0, st, g, c, m, h, ctr, color, acc);
   }
-  if (g.ncolors == 2) {
+  if constexpr (sizeof(T) == 8) {
+    // one trial per thread; two (fuller warps of accepted trials) once the
+    // launch has more CTAs than the SMs hold at a time
+    const long long total = g.ncolors == 2 ? (long long)g.ny * g.nz * ((g.nx + 1) / 2) : g.n;
+    const int tpt = total * nrep >= 2LL * MCL_THREADS * 152 * 8 ? 2 : 1;
+    dim3 grid((unsigned)((total + tpt * MCL_THREADS - 1) / (tpt * MCL_THREADS)), 1, nrep);
+    return launch_pdl(tpt == 2 ? k_mc_list<2> : k_mc_list<1>, grid, dim3(MCL_THREADS), 0, st, g, c, m, h, ctr, color,
+                      acc);
+  } else if (g.ncolors == 2) {
     const long long total = (long long)g.ny * g.nz * ((g.nx + 1) / 2);
     dim3 grid((unsigned)((total + threads - 1) / threads), 1, nrep);
     MMC_TRY(launch_pdl(k_mc_checker<T>, grid, dim3(threads), 0, st, g, c, m, h, ctr, color, acc));

@@ -91,27 +91,6 @@ int mc_pipe_error_take() {
   return v;
 }
 
-// Forward transform of the six real tensor blocks k6[c][z][y][x] (padded
-// grid) into spec64[c][kz][ky][kx] (src/main.cu:593-642 ran cuFFT D2Z here).
-cudaError_t launch_tensor_fft(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
-                              const DemagTuning& tun, const double* k6, double2* spec64, cudaStream_t st) {
-  const long long ns = g.nspec;
-  MMC_TRY(cudaMemsetAsync(spec64, 0, 6 * (size_t)ns * sizeof(double2), st));
-  MMC_TRY(run_x_forward<double>(px, 6, g.nxp, g.nyp, g.nyp * g.nzp, k6, g.np, spec64, ns, g.nyp, g.hx, g.hxp, 1,
-                                tun.x_threads, st, 1, 0, 0));
-  const long long ystride = g.hxp, yplane = (long long)g.nyp * g.hxp;
-  for (int half = 0; half < 2; ++half) {
-    double2* S = spec64 + 3 * half * ns;
-    if (g.nyp > 1)
-      MMC_TRY(run_col_pass<double>(py, 3, S, ns, nullptr, g.hx, g.nzp, yplane, ystride, g.nyp, g.nyp, PASS_FWD, 1.0,
-                                   tun.col_tx, tun.col_threads, st));
-    if (g.nzp > 1)
-      MMC_TRY(run_col_pass<double>(pz, 3, S, ns, nullptr, g.hx, g.nyp, ystride, yplane, g.nzp, g.nzp, PASS_FWD, 1.0,
-                                   tun.col_tx, tun.col_threads, st));
-  }
-  return cudaSuccess;
-}
-
 __global__ void k_advance(SweepCounters* ctr, uint32_t delta, int count) {
   pdl_wait();  // the previous kernels read the counters
   if ((int)threadIdx.x < count) ctr[threadIdx.x].sweep += delta;

@@ -96,6 +96,20 @@ struct alignas(16) McCoef {
   uint32_t key0, key1;  // Philox key = seed
 };
 
+// The FP32 copy of the coefficients with which an FP64 trial is first judged
+// (mc_filter), and the weights of that judgement's error bound.
+struct McFilter {
+  float wex[3], wdm[2], can, u[3], cz[3], cd, k0h[6];
+  float gm;  // per-component bound on the field F of a trial: gm max|m| + gc + |cd| max|h|
+  float gc;
+};
+template <>
+struct alignas(16) McCoef<double> {
+  double wex[3], wdm[2], can, u[3], cz[3], cd, k0[6], k0h[6];
+  uint32_t key0, key1;
+  McFilter f;
+};
+
 // Energy prefactors (SI, J).
 struct EnCoef {
   double aexV_d2[3];  // Aex V / d_a^2
@@ -217,6 +231,14 @@ cudaError_t launch_init(const Geom& g, uint64_t seed, T* m, cudaStream_t st);
 template <typename T>
 cudaError_t launch_demag_sym(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
                              const DemagTuning& tun, const T* m, T* h, void* spec, const void* khat, cudaStream_t st);
+// The same in FP64 with every product and sum rounded by itself: a relaxation's
+// Barzilai-Borwein steps amplify the last bit of the field along the path (a
+// few hundred steps change the seventh digit), so its path is kept independent
+// of how the other passes contract their products.
+cudaError_t launch_demag_sym_relax(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
+                                   const DemagTuning& tun, const double* m, double* h, void* spec, const void* khat,
+                                   cudaStream_t st);
+cudaError_t launch_prepare_f64s(int max_dyn_smem);
 template <typename T>
 cudaError_t launch_grad(const Geom& g, const HCoef& c, const EnCoef& eu, double gscale, const T* m, const T* hs,
                         double* grad, double* partials, int npartials, double* out, cudaStream_t st);

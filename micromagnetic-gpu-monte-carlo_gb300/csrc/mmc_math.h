@@ -255,13 +255,9 @@ MMC_HD double exp(double x) {
   return p * bitsd((uint64_t)(k + 1023) << 52);
 }
 
-// sin(pi t) and cos(pi t): t = n/2 + r with |r| <= 1/4, then Taylor sums in
-// y = pi r (|y| <= pi/4) and a quadrant swap.
-MMC_HD void sincospi(double t, double* sp, double* cp) {
-  double n2 = dfloor(2.0 * t + 0.5);
-  double r = t - 0.5 * n2;
-  double q4 = n2 - 4.0 * dfloor(n2 * 0.25);
-  int q = (int)q4;
+// sin(pi t) and cos(pi t) from t = n/2 + r with |r| <= 1/4 and q = n mod 4:
+// Taylor sums in y = pi r (|y| <= pi/4) and a quadrant swap.
+MMC_HD void sincospi_reduced(int q, double r, double* sp, double* cp) {
   double y = r * MMCM_PI_HI + r * MMCM_PI_LO;
   double w = y * y;
   double s = 0x1.71b8ef6dcf572p-66;    // +1/21!
@@ -293,6 +289,14 @@ MMC_HD void sincospi(double t, double* sp, double* cp) {
     case 2: *sp = -s; *cp = -c; break;
     default: *sp = -c; *cp = s; break;
   }
+}
+
+// sin(pi t) and cos(pi t).
+MMC_HD void sincospi(double t, double* sp, double* cp) {
+  double n2 = dfloor(2.0 * t + 0.5);
+  double r = t - 0.5 * n2;
+  double q4 = n2 - 4.0 * dfloor(n2 * 0.25);
+  sincospi_reduced((int)q4, r, sp, cp);
 }
 
 // ------------------------------------------------------------------ Philox

@@ -231,9 +231,7 @@ __device__ __forceinline__ unsigned int row_sweep(const RowPhase<T>& R, const Mc
       const T* hr = R.hsm + (size_t)(slot - 1) * mstride;
       const Proposal<T> p = R.prop[k * half + j];
       if (mc_accept<T>(c, nbv, row[x], row[nx + x], row[2 * nx + x], hr[x], hr[nx + x], hr[2 * nx + x], p)) {
-        row[x] = p.x;
-        row[nx + x] = p.y;
-        row[2 * nx + x] = p.z;
+        p.get(row[x], row[nx + x], row[2 * nx + x]);
         if (slot >= 2 && slot < 2 + R.nb) acc += 1;
       }
     }

@@ -835,8 +835,13 @@ int set_m_impl(mmc_handle* h, const double* mx, const double* my, const double* 
 
 // ------------------------------------------------------------ gradient
 // The demag field with the symmetrised tensor, into h->hsym.
-int demag_sym(mmc_handle* h) {
+int demag_sym(mmc_handle* h, bool relax = false) {
   if (!h->hsym) CU(cudaMalloc(&h->hsym, 3 * (size_t)h->g.n * h->tsize));
+  if (relax && h->prec == 64) {
+    CU(launch_demag_sym_relax(h->g, h->px.p, h->py.p, h->pz.p, h->tun, (const double*)h->m, (double*)h->hsym, h->spec,
+                              h->khat, h->st));
+    return MMC_OK;
+  }
   CU(h->prec == 32 ? launch_demag_sym<float>(h->g, h->px.p, h->py.p, h->pz.p, h->tun, (const float*)h->m,
                                              (float*)h->hsym, h->spec, h->khat, h->st)
                    : launch_demag_sym<double>(h->g, h->px.p, h->py.p, h->pz.p, h->tun, (const double*)h->m,
@@ -897,7 +902,7 @@ int relax_impl(mmc_handle* h, double tol, long long max_iter, long long* iters, 
   long long it = 0;
   for (;; ++it) {
     if (h->stop.load()) return fail(MMC_ERR_INTERRUPTED, "stop requested");
-    if (dm) TRY(demag_sym(h));
+    if (dm) TRY(demag_sym(h, true));
     CU(h->prec == 32 ? launch_relax_eval<float>(h->g, k, inv_ms, (const float*)h->m,
                                                 dm ? (const float*)h->hsym : nullptr, h->relax_p, h->relax_s,
                                                 it == 0, h->partials, h->npartials, h->red, h->st)
@@ -1039,7 +1044,8 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   int nsm = 148, optin = 48 * 1024;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  if (launch_prepare<float>(optin) != cudaSuccess || launch_prepare<double>(optin) != cudaSuccess)
+  if (launch_prepare<float>(optin) != cudaSuccess || launch_prepare<double>(optin) != cudaSuccess ||
+      launch_prepare_f64s(optin) != cudaSuccess)
     return bail(fail(MMC_ERR_CUDA, "kernel attribute setup failed"));
   const size_t csize = 2 * h->tsize;
   h->tun = choose_tuning(g, h->px.p, h->py.p, h->pz.p, csize, nsm, 1);
