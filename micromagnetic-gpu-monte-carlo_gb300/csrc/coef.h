@@ -33,12 +33,12 @@ struct McParams {
 // |cz| + cd |h|, components at most max(1, |m|) and |h|.
 MMC_COEF_HD inline McFilter mc_filter_from(const McCoef<double>& k) {
   McFilter f;
-  double g = 0, kmax = 0, cmax = 0;
+  double g = 0, gz = 0, kmax = 0, cmax = 0;
   for (int a = 0; a < 3; ++a) {
     f.wex[a] = (float)k.wex[a];
     f.u[a] = (float)k.u[a];
     f.cz[a] = (float)k.cz[a];
-    g += 2.0 * (k.wex[a] < 0 ? -k.wex[a] : k.wex[a]);
+    (a < 2 ? g : gz) += 2.0 * (k.wex[a] < 0 ? -k.wex[a] : k.wex[a]);
     const double z = k.cz[a] < 0 ? -k.cz[a] : k.cz[a];
     if (!(z <= cmax)) cmax = z;
   }
@@ -55,6 +55,7 @@ MMC_COEF_HD inline McFilter mc_filter_from(const McCoef<double>& k) {
   f.cd = (float)k.cd;
   g += 6.0 * kmax + 4.0 * (k.can < 0 ? -k.can : k.can);
   f.gm = (float)(1.001 * g);
+  f.gz = (float)(1.001 * gz);
   f.gc = (float)(1.001 * cmax);
   return f;
 }

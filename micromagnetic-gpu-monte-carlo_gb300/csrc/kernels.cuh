@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "fft.cuh"
+#include "lines64.cuh"
 #include "mmc_internal.h"
 #include "mmc_math.h"
 
@@ -805,26 +806,40 @@ struct Prop;
 
 template <>
 struct Prop<double> {
-  static __device__ __forceinline__ double ticks(int j) {  // j 2^-32, exact
-    return __longlong_as_double(0x4138000000000000ll + (long long)j) - 0x1.8p20;
-  }
   // The direction of the random words rx, ry: z = 2 u0 - 1, phi = 2 pi u1 with
   // u = (r + 1/2) 2^-32.  The steps of mmcm::u01_f64 and mmcm::sincospi, bit
   // for bit; what they do exactly (the uniforms, the split of 2 u1 into
   // quadrants) is done on the integers, which leaves 60 FP64 operations.
+  static __device__ __forceinline__ double height(uint32_t rx) {  // (2 rx + 1 - 2^32) 2^-32
+    return __longlong_as_double(0x4138000000000000ll + 2 * (long long)(int)(rx ^ 0x80000000u) + 1) - 0x1.8p20;
+  }
+  static __device__ __forceinline__ double radius(double z) {
+    const double t = 1.0 - z * z;  // >= 0: |z| < 1
+    return mmcm::dsqrt(t);
+  }
+  static __device__ __forceinline__ uint32_t halves(uint32_t ry) { return (ry >> 30) + ((ry >> 29) & 1u); }
+  static __device__ __forceinline__ int quadrant(uint32_t ry) { return (int)(halves(ry) & 3u); }
+  static __device__ __forceinline__ double quarter(uint32_t ry) {  // 2 u1 less its nearest half
+    const int j = (int)(2u * ry + 1u - (halves(ry) << 31));
+    return __longlong_as_double(0x4138000000000000ll + (long long)j) - 0x1.8p20;
+  }
   static __device__ __forceinline__ void direction(uint32_t rx, uint32_t ry, double& px, double& py, double& pz) {
-    // (2 rx + 1 - 2^32) 2^-32: twice the signed word, 33 bits wide
-    pz = __longlong_as_double(0x4138000000000000ll + 2 * (long long)(int)(rx ^ 0x80000000u) + 1) - 0x1.8p20;
-    const double t = 1.0 - pz * pz;  // >= 0: |pz| < 1
-    const double s = mmcm::dsqrt(t);
-    const uint32_t n2 = (ry >> 30) + ((ry >> 29) & 1u);
-    const double r = ticks((int)(2u * ry + 1u - (n2 << 31)));
+    pz = height(rx);
+    const double s = radius(pz);
     double sn, cs;
-    mmcm::sincospi_reduced((int)(n2 & 3u), r, &sn, &cs);
+    mmcm::sincospi_reduced(quadrant(ry), quarter(ry), &sn, &cs);
     px = s * cs;
     py = s * sn;
   }
-  __device__ static bool accept(double dE, double ua) { return dE <= 0.0 || ua < mmcm::exp(-dE); }
+  // The exponential's 50 operations only where the hardware's (see mc_filter)
+  // cannot tell: dE is known to 2^-52 here, so the sides differ by 1e-5.
+  __device__ static bool accept(double dE, double ua) {
+    if (dE <= 0.0) return true;
+    const float x = fminf((float)dE, 30.0f), e = __expf(-x), u = (float)ua;
+    if (u > 1.00002f * e) return false;
+    if (dE < 30.0 && u * 1.00002f < e) return true;
+    return ua < mmcm::exp(-dE);
+  }
 };
 
 template <>
@@ -900,20 +915,20 @@ __device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t c
 //
 // The bound: with M >= every |component| of m involved (at least 1), H the
 // same for h, and G = gm M + gc + |cd| H >= |F_a| for each component of the
-// field (McFilter), dE = -d . F with |d_a| <= 1 + M, evaluated in the regrouped
-// form of mc_accept<float>.  Its FP32 evaluation sums at most 40 roundings of
-// 2^-24 on any path from an input to dE (2 for a truncated input, 1 for a
-// coefficient, at most 30 in the sums of F and of the dot product), each on
-// terms that add up to at most 3 (1 + M) G: 7.2e-6 (1 + M) G.  The direction's
-// components are off by less than 1e-6 (hardware sine and cosine: 2^-21.19 on
-// [-pi, pi], the angle's own rounding 2e-7; the rest rounds to a few 2^-24),
-// which changes dE by less than 3 x 1e-6 x 2 G.  FP64 rounding is 1e-9 of
-// either.  MC_FILTER_EPS = 1.6e-5 times (1 + M) G covers the sum 1.4e-5.
+// field (McFilter), dE = -d . F in the regrouped form of mc_accept<float>.  On
+// any path from an input to dE its FP32 evaluation makes at most 32 roundings of
+// 2^-24 (2 for a truncated input, 1 for a coefficient, 16 in a component of F, 3
+// in d and 3 in the dot product), each on terms that add up to at most |d|_1 G:
+// 1.9e-6 |d|_1 G.  The direction's components are off by at most 2.5e-7 (the
+// angle's rounding 9e-8, sincospif 1 ulp, 1 - z^2 as a product of two rounded
+// factors, its square root through rsqrtf), and dE changes by at most 2 G per
+// unit of each: 1.5e-6 G.  FP64 rounding is 1e-9 of either.  MC_FILTER_EPS =
+// 2.2e-6 times (|d|_1 + 1) G covers both.
 // exp: the hardware's is within 2 + 1.173 |x| ulp, 4.5e-6 for x >= -30; below
 // that the smallest uniform (2^-33) decides alone.  MC_FILTER_EXP = 2e-5 covers
 // it and the rounding of the uniform.  NaN or infinity anywhere leaves both
 // comparisons false: unsure.
-constexpr float MC_FILTER_EPS = 1.6e-5f;
+constexpr float MC_FILTER_EPS = 2.2e-6f;
 constexpr float MC_FILTER_EXP = 2e-5f;
 enum McVerdict : int { MC_REJECT = 0, MC_ACCEPT = 1, MC_UNSURE = 2 };
 
@@ -928,10 +943,10 @@ __device__ __forceinline__ float f32_trunc(double x) {
 __device__ __forceinline__ float f32_trunc(float x) { return x; }
 
 // Neighbour values v (meaningful where has is true) and their flags, own cell
-// o, demag field h (0 when the demag term is off).
+// o, demag field h (0 when the demag term is off); film: no z neighbours.
 __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&v)[3][2][3], const bool (&has)[3][2],
                                                float ox, float oy, float oz, float hx, float hy, float hz,
-                                               uint32_t rx, uint32_t ry, uint32_t rz) {
+                                               uint32_t rx, uint32_t ry, uint32_t rz, bool film) {
   float Fx = c.cz[0], Fy = c.cz[1], Fz = c.cz[2];
   float M = fmaxf(fmaxf(fabsf(ox), fabsf(oy)), fmaxf(fabsf(oz), 1.0f));
   // NaN does not survive fmaxf: a sum that it does survive joins the bound
@@ -957,7 +972,7 @@ __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&
   const float t = a0 * a1;
   const float r = t * rsqrtf(t);
   float sn, cs;
-  __sincosf((float)(int)(ry ^ 0x80000000u) * (3.14159265358979323846f * 0x1p-31f), &sn, &cs);
+  sincospif((float)(int)(ry ^ 0x80000000u) * 0x1p-31f, &sn, &cs);
   const float px = -(r * cs), py = -(r * sn), pz = (float)(int)(rx ^ 0x80000000u) * 0x1p-31f;
   const float dx = px - ox, dy = py - oy, dz = pz - oz;
   Fx = fmaf(c.cd, hx, Fx) + fmaf(c.k0h[0], dx, fmaf(c.k0h[1], dy, c.k0h[2] * dz));
@@ -971,7 +986,8 @@ __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&
   const float mdE = fmaf(dx, Fx, fmaf(dy, Fy, dz * Fz));  // -dE
   const float H = fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz)));
   nan0 += 0.0f * mdE;
-  const float eps = fmaf(MC_FILTER_EPS * (1.0f + M), fmaf(c.gm, M, fmaf(fabsf(c.cd), H, c.gc)), nan0);
+  const float D = fabsf(dx) + fabsf(dy) + fabsf(dz);
+  const float eps = fmaf(MC_FILTER_EPS * (D + 1.0f), fmaf(film ? c.gm : c.gm + c.gz, M, fmaf(fabsf(c.cd), H, c.gc)), nan0);
   const float ua = fmaf((float)rz, 0x1p-32f, 0x1p-33f);
   const float lo = mdE - eps, hi = fmaxf(mdE + eps, -30.0f);
   if (lo >= 0.0f || ua * (1.0f + MC_FILTER_EXP) < __expf(lo)) return MC_ACCEPT;
@@ -1061,7 +1077,8 @@ __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb,
 #pragma unroll
         for (int k = 0; k < 3; ++k) v[a][s][k] = f32_trunc(nb.v[a][s][k]);
     const McVerdict w = mc_filter(c.f, v, nb.has, f32_trunc(ox), f32_trunc(oy), f32_trunc(oz), f32_trunc(hx),
-                                  f32_trunc(hy), f32_trunc(hz), p.rx, p.ry, p.rz);
+                                  f32_trunc(hy), f32_trunc(hz), p.rx, p.ry, p.rz,
+                                  !nb.has[2][0] && !nb.has[2][1]);
     if (w != MC_UNSURE) return w == MC_ACCEPT;
     T px, py, pz;
     p.get(px, py, pz);
@@ -1193,6 +1210,7 @@ __global__ void __launch_bounds__(MCL_THREADS) k_mc_list(Geom g, const McCoef<do
                                                          const SweepCounters* __restrict__ ctr, int color,
                                                          unsigned long long* acc) {
   __shared__ uint4 list[MCL_THREADS * TPT];  // cell (top bit: unsure), random words
+  __shared__ double part[3][MCL_THREADS * TPT];
   __shared__ int count;
   if (threadIdx.x == 0) count = 0;
   pdl_wait();
@@ -1241,7 +1259,7 @@ __global__ void __launch_bounds__(MCL_THREADS) k_mc_list(Geom g, const McCoef<do
         }
         p = mc_propose<double>(c, (uint32_t)cell, stage, sweep);
         w = mc_filter(c.f, nb.v, nb.has, f32_trunc(m[cell]), f32_trunc(m[n + cell]), f32_trunc(m[2 * n + cell]), hx,
-                      hy, hz, p.rx, p.ry, p.rz);
+                      hy, hz, p.rx, p.ry, p.rz, g.nz == 1);
       }
     }
     const unsigned mask = __ballot_sync(0xffffffffu, w != MC_REJECT);
@@ -1257,14 +1275,34 @@ __global__ void __launch_bounds__(MCL_THREADS) k_mc_list(Geom g, const McCoef<do
   }
   __syncthreads();
   const int cnt = count;
+  // the listed trials' directions, in three pieces of about 25 FP64 operations
+  // on warps of their own: a warp's FP64 instructions issue one per 64 cycles
+  const int lane = threadIdx.x & 31, groups = (cnt + 31) >> 5;
+  for (int task = threadIdx.x >> 5; task < 3 * groups; task += MCL_THREADS / 32) {
+    const int piece = task / groups, i = (task - piece * groups) * 32 + lane;
+    if (i >= cnt) continue;
+    const uint4 e = list[i];
+    double v;
+    if (piece == 2) {
+      v = Prop<double>::radius(Prop<double>::height(e.y));
+    } else {
+      double y, w;
+      mmcm::pi_angle(Prop<double>::quarter(e.z), &y, &w);
+      v = piece == 0 ? mmcm::sin_taylor(y, w) : mmcm::cos_taylor(w);
+    }
+    part[piece][i] = v;
+  }
+  __syncthreads();
   for (int i0 = 0; i0 < cnt; i0 += MCL_THREADS) {
     const int i = i0 + threadIdx.x;
     bool ok = i < cnt;
     if (ok) {
       const uint4 e = list[i];
       const int cell = (int)(e.x & 0x7fffffffu);
-      double px, py, pz;
-      Prop<double>::direction(e.y, e.z, px, py, pz);
+      double sn, cs;
+      mmcm::sincos_quadrant(Prop<double>::quadrant(e.z), part[0][i], part[1][i], &sn, &cs);
+      const double s = part[2][i];
+      const double px = s * cs, py = s * sn, pz = Prop<double>::height(e.y);
       if (e.x >> 31) {
         const int row = g.dnx.div(cell), x = cell - row * g.nx;
         const int z = g.dny.div(row), y = row - z * g.ny;
@@ -2473,6 +2511,8 @@ struct XPassW {
 };
 template <typename T>
 XPassW<T> x_pass_w(const FftPlan& p) {
+  if constexpr (__is_same(T, double)) return {nullptr, nullptr};  // lines64.cuh
+  else {
 #define MMC_XW(A_, B_) \
   if (p.warp_a == A_ && p.warp_b == B_) return {k_x_forward_w<T, A_, B_>, k_x_inverse_w<T, A_, B_>};
   MMC_XW(32, 32)
@@ -2484,6 +2524,7 @@ XPassW<T> x_pass_w(const FftPlan& p) {
   MMC_XW(8, 4)
 #undef MMC_XW
   return {nullptr, nullptr};
+  }
 }
 inline size_t x_pass_w_smem(const FftPlan& p, int rows, size_t csize) {
   return ((size_t)p.n + 2 * (size_t)rows * (p.n + p.warp_a)) * csize;
@@ -2495,29 +2536,34 @@ inline size_t x_pass_w_smem(const FftPlan& p, int rows, size_t csize) {
 template <typename T>
 cudaError_t prepare_passes(int max_dyn_smem) {
   const void* fns[] = {(const void*)k_x_forward<T, false, 3>, (const void*)k_x_forward<T, true, 3>,
-                       (const void*)k_x_forward<T, false, 6>, (const void*)k_x_forward<T, true, 6>,
-                       (const void*)k_x_inverse<T, false>, (const void*)k_x_inverse<T, true>,
-                       (const void*)k_col_pass<T, false>,      (const void*)k_col_pass<T, true>,
-                       (const void*)k_col_pass_wide<T, false>, (const void*)k_col_pass_wide<T, true>};
+                       (const void*)k_x_inverse<T, false>,    (const void*)k_x_inverse<T, true>,
+                       (const void*)k_col_pass<T, false>,     (const void*)k_col_pass<T, true>};
   for (const void* f : fns) MMC_TRY_ATTR(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
-  for (int s = 0; s < 7; ++s) {
-    FftPlan p{};
-    const int ab[7][2] = {{32, 32}, {32, 16}, {16, 16}, {16, 8}, {8, 8}, {16, 2}, {8, 4}};
-    p.warp_a = ab[s][0];
-    p.warp_b = ab[s][1];
-    const XPassW<T> w = x_pass_w<T>(p);
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+  if constexpr (__is_same(T, double)) return l64_prepare(max_dyn_smem);
+  else {
+    const void* wide[] = {(const void*)k_col_pass_wide<T, false>, (const void*)k_col_pass_wide<T, true>};
+    for (const void* f : wide) MMC_TRY_ATTR(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+    if constexpr (__is_same(T, f64s))  // the tensor's six blocks
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_x_forward<T, false, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+    for (int s = 0; s < 7; ++s) {
+      FftPlan p{};
+      const int ab[7][2] = {{32, 32}, {32, 16}, {16, 16}, {16, 8}, {8, 8}, {16, 2}, {8, 4}};
+      p.warp_a = ab[s][0];
+      p.warp_b = ab[s][1];
+      const XPassW<T> w = x_pass_w<T>(p);
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+    }
+    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)col_reg_smem<T, 16>()));
+    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)col_reg_smem<T, 8>()));
+    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)col_reg_smem<T, 16>()));
+    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)col_reg_smem<T, 8>()));
+    return cudaSuccess;
   }
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)col_reg_smem<T, 16>()));
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)col_reg_smem<T, 8>()));
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)col_reg_smem<T, 16>()));
-  MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)col_reg_smem<T, 8>()));
-  return cudaSuccess;
 }
 template <typename T>
 cudaError_t prepare_impl(int max_dyn_smem) {
@@ -2559,9 +2605,11 @@ cudaError_t run_x_forward(const FftPlan& p, int ncomp, int xdata, int ydata, int
   const int lines = (ncomp + 1) / 2;
   size_t sm = x_pass_smem(p, lines, rpc, sizeof(C<T>));
   dim3 grid((nrows + rpc - 1) / rpc, 1, nrep);
-  if (ncomp != 3 && ncomp != 6) return cudaErrorInvalidValue;
-  auto kern = ncomp == 3 ? (inl ? k_x_forward<T, true, 3> : k_x_forward<T, false, 3>)
-                         : (inl ? k_x_forward<T, true, 6> : k_x_forward<T, false, 6>);
+  auto kern = inl ? k_x_forward<T, true, 3> : k_x_forward<T, false, 3>;
+  if constexpr (__is_same(T, f64s)) {
+    if (ncomp == 6) kern = k_x_forward<T, false, 6>;  // the tensor's six blocks
+  }
+  if (ncomp != 3 && !(ncomp == 6 && __is_same(T, f64s))) return cudaErrorInvalidValue;
   kern<<<grid, threads, sm, st>>>(p, xdata, FastDiv((uint32_t)ydata), nrows, in, in_cstride, S, nspec, nyp,
                                   FastDiv((uint32_t)hx), pitch, rpc, in_rstride, s_rstride);
   return cudaGetLastError();
@@ -2583,6 +2631,16 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
                         store_lim, flags, inv_n, s_rstride);
     }
   }
+  if constexpr (__is_same(T, double)) {
+    L64Fns f;
+    if (ncomp == 3 && l64_pick(p, (long long)hx * planes * nrep, f)) {
+      const int mode = (flags & PASS_MUL) ? 2 : (flags & PASS_INV) ? 1 : 0;
+      return launch_pdl(f.col[mode], dim3((hx + f.tile - 1) / f.tile, planes, nrep), dim3(f.threads), f.smem, st, p, S,
+                        nspec, khat, hx, plane_stride, pos_stride, load_lim, store_lim, (flags & PASS_SYM) ? 1 : 0,
+                        inv_n, s_rstride);
+    }
+  }
+  if constexpr (!__is_same(T, double))
   if (regs && ncomp == 3 && planes == 1 && (flags & ~PASS_SYM) == (PASS_FWD | PASS_MUL | PASS_INV) &&
       pos_stride < (1LL << 31) && p.warp_a == p.warp_b && (p.warp_a == 16 || p.warp_a == 8)) {
     dim3 grid((hx + CR_TX - 1) / CR_TX, 1, nrep);
@@ -2616,8 +2674,10 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
     }
   }
   dim3 grid((hx + tx - 1) / tx, planes, nrep);
-  auto kern = p.warp_a == 32 ? (inl ? k_col_pass_wide<T, true> : k_col_pass_wide<T, false>)
-                             : (inl ? k_col_pass<T, true> : k_col_pass<T, false>);
+  auto kern = inl ? k_col_pass<T, true> : k_col_pass<T, false>;
+  if constexpr (!__is_same(T, double)) {
+    if (p.warp_a == 32) kern = inl ? k_col_pass_wide<T, true> : k_col_pass_wide<T, false>;
+  }
   // no more threads than the kernel's registers allow (the split of the work
   // does not change the results)
   cudaFuncAttributes fa;
@@ -2643,10 +2703,22 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   const C<T>* K = reinterpret_cast<const C<T>*>(khat);
   const long long ns = g.nspec;
   const long long mr = 3 * g.n, sr = 3 * ns;  // replica strides
-  const T inv_n = (T)(1.0 / (double)g.np);
+  T inv_n = (T)(1.0 / (double)g.np);
   const int rows = g.ny * g.nz;
   if (ev) MMC_TRY(cudaEventRecord(ev[0], st));
-  MMC_TRY(run_x_forward<T>(px, 3, g.nx, g.ny, rows, m, g.n, S, ns, g.nyp, g.hx, g.hxp, tun.x_rows_per_cta,
+  bool x64 = false;  // the FP64 x passes of lines64.cuh
+  if constexpr (__is_same(T, double)) {
+    L64Fns f;
+    x64 = l64_pick(px, (long long)((rows + 1) / 2) * nrep, f);
+    if (x64) {
+      dim3 grid(((rows + 1) / 2 + f.tile - 1) / f.tile, 1, nrep);
+      MMC_TRY(launch_pdl(f.xf, grid, dim3(f.threads), f.smem, st, px, g.nx, g.dny, rows, m, g.n, S, ns, g.nyp, g.hxp,
+                         mr, sr));
+      inv_n *= 0.5;  // the forward pass leaves the spectra doubled
+    }
+  }
+  if (!x64)
+    MMC_TRY(run_x_forward<T>(px, 3, g.nx, g.ny, rows, m, g.n, S, ns, g.nyp, g.hx, g.hxp, tun.x_rows_per_cta,
                            tun.x_threads, st, nrep, mr, sr, tun.fft_inline != 0));
   if (ev) MMC_TRY(cudaEventRecord(ev[1], st));
   const long long ystride = g.hxp, yplane = (long long)g.nyp * g.hxp;
@@ -2667,7 +2739,14 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   const int rpc = tun.x_rows_per_cta;
   dim3 grid((rows + rpc - 1) / rpc, 1, nrep);
   const XPassW<T> w = x_pass_w<T>(px);
-  if (w.inv) {
+  if (x64) {
+    if constexpr (__is_same(T, double)) {
+      L64Fns f;
+      l64_pick(px, (long long)((rows + 1) / 2) * nrep, f);
+      MMC_TRY(launch_pdl(f.xi, dim3(((rows + 1) / 2 + f.tile - 1) / f.tile, 1, nrep), dim3(f.threads), f.smem, st, px,
+                         (const double2*)S, ns, g.nyp, g.hxp, g.nx, g.dny, rows, h, g.n, sr, mr));
+    }
+  } else if (w.inv) {
     MMC_TRY(launch_pdl(w.inv, grid, dim3(tun.x_threads), x_pass_w_smem(px, rpc, sizeof(C<T>)), st, px,
                        (const C<T>*)S, ns, g.nyp, g.hx, g.hxp, g.dnx, g.dny, rows, h, g.n, rpc, sr, mr));
   } else {

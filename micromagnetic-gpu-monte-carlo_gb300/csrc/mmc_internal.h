@@ -100,8 +100,9 @@ struct alignas(16) McCoef {
 // (mc_filter), and the weights of that judgement's error bound.
 struct McFilter {
   float wex[3], wdm[2], can, u[3], cz[3], cd, k0h[6];
-  float gm;  // per-component bound on the field F of a trial: gm max|m| + gc + |cd| max|h|
-  float gc;
+  // per-component bound on the field F of a trial: (gm + gz) max|m| + gc + |cd| max|h|, gz the
+  // part of the z neighbours
+  float gm, gz, gc;
 };
 template <>
 struct alignas(16) McCoef<double> {

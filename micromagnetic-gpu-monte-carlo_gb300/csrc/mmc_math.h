@@ -256,10 +256,12 @@ MMC_HD double exp(double x) {
 }
 
 // sin(pi t) and cos(pi t) from t = n/2 + r with |r| <= 1/4 and q = n mod 4:
-// Taylor sums in y = pi r (|y| <= pi/4) and a quadrant swap.
-MMC_HD void sincospi_reduced(int q, double r, double* sp, double* cp) {
-  double y = r * MMCM_PI_HI + r * MMCM_PI_LO;
-  double w = y * y;
+// Taylor sums in y = pi r (|y| <= pi/4), w = y^2, and a quadrant swap.
+MMC_HD void pi_angle(double r, double* y, double* w) {
+  *y = r * MMCM_PI_HI + r * MMCM_PI_LO;
+  *w = *y * *y;
+}
+MMC_HD double sin_taylor(double y, double w) {
   double s = 0x1.71b8ef6dcf572p-66;    // +1/21!
   s = s * w - 0x1.2f49b46814157p-57;   // -1/19!
   s = s * w + 0x1.952c77030ad4ap-49;   // +1/17!
@@ -271,7 +273,9 @@ MMC_HD void sincospi_reduced(int q, double r, double* sp, double* cp) {
   s = s * w + 0x1.1111111111111p-7;    // +1/5!
   s = s * w - 0x1.5555555555555p-3;    // -1/3!
   s = s * w + 1.0;
-  s = s * y;
+  return s * y;
+}
+MMC_HD double cos_taylor(double w) {
   double c = 0x1.e542ba4020225p-62;    // +1/20!
   c = c * w - 0x1.6827863b97d97p-53;   // -1/18!
   c = c * w + 0x1.ae7f3e733b81fp-45;   // +1/16!
@@ -283,12 +287,20 @@ MMC_HD void sincospi_reduced(int q, double r, double* sp, double* cp) {
   c = c * w + 0x1.5555555555555p-5;    // +1/4!
   c = c * w - 0.5;                     // -1/2!
   c = c * w + 1.0;
+  return c;
+}
+MMC_HD void sincos_quadrant(int q, double s, double c, double* sp, double* cp) {
   switch (q) {
     case 0: *sp = s; *cp = c; break;
     case 1: *sp = c; *cp = -s; break;
     case 2: *sp = -s; *cp = -c; break;
     default: *sp = -c; *cp = s; break;
   }
+}
+MMC_HD void sincospi_reduced(int q, double r, double* sp, double* cp) {
+  double y, w;
+  pi_angle(r, &y, &w);
+  sincos_quadrant(q, sin_taylor(y, w), cos_taylor(w), sp, cp);
 }
 
 // sin(pi t) and cos(pi t).
