@@ -57,7 +57,9 @@ enum mmc_term {
 enum mmc_ovf_format { MMC_OVF_BINARY4 = 0, MMC_OVF_BINARY8 = 1, MMC_OVF_TEXT = 2 };
 
 /* How sweeps are executed.  AUTO picks FUSED for films (nz = 1, demag on, two
- * sublattice colours) and KERNELS otherwise.  Both give bit-identical results. */
+ * sublattice colours) where it is the faster one -- in FP32 always, in FP64 for
+ * small films without a power-of-two transform -- and KERNELS otherwise.  Both
+ * give the same decisions. */
 enum mmc_engine {
   MMC_ENGINE_AUTO = 0,
   MMC_ENGINE_KERNELS = 1,  /* one kernel per transform pass and colour, replayed from CUDA graphs */

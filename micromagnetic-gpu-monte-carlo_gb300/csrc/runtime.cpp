@@ -548,7 +548,13 @@ int setup_engine(mmc_handle* h, int nsm) {
   const bool eligible = c.cal_demag_flag && g.nz == 1 && g.nzp == 1 && g.ncolors == 2 &&
                         ((size_t)g.nx * h->tsize) % 16 == 0 && g.ny >= 1 && h->px.p.warp_a != 32 &&
                         h->py.p.warp_a != 32;
-  if (c.sweep_engine == MMC_ENGINE_KERNELS || (c.sweep_engine == MMC_ENGINE_AUTO && !eligible)) {
+  // FP64 films: the film engine's CTAs transform and sweep their halo rows again
+  // and leave most of the SM's FP64 issue idle, while the pass kernels spread
+  // the operations (lines64.cuh).  us per sweep, pass kernels / film engine: 32^2
+  // 20 / 32, 64^2 22 / 36, 128^2 27 / 70; without a power-of-two transform 24^2
+  // 37 / 28, 48^2 39 / 32, 96^2 43 / 46, 192^2 56 / 85.
+  const bool f64_kernels = h->prec == 64 && ((h->px.p.warp_a && h->py.p.warp_a) || g.n >= 8192);
+  if (c.sweep_engine == MMC_ENGINE_KERNELS || (c.sweep_engine == MMC_ENGINE_AUTO && (!eligible || f64_kernels))) {
     h->engine = MMC_ENGINE_KERNELS;
     return MMC_OK;
   }
