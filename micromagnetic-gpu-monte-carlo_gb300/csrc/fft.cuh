@@ -63,6 +63,37 @@ template <typename V>
 __device__ __forceinline__ V csub(V a, V b) {
   return cmk<V>(a.x - b.x, a.y - b.y);
 }
+// The same as padd and psub where neither operand is a product the compiler
+// contracts with the sum: in FP32 one packed instruction for the real and the
+// imaginary part, the same two sums in one issue slot.
+template <typename V>
+__device__ __forceinline__ V padd(V a, V b) {
+  return cadd(a, b);
+}
+template <typename V>
+__device__ __forceinline__ V psub(V a, V b) {
+  return csub(a, b);
+}
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_of(unsigned long long r) {
+  float2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ float2 padd(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+__device__ __forceinline__ float2 psub(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
 // FP64 products are written with explicit multiply-adds.  The FP64 kernels are
 // built without contraction (the sweep's decisions round like the oracle's),
 // but the transforms only have to be accurate, and GB300 issues 1.7 FP64
@@ -329,8 +360,8 @@ struct RegDft {
         }
         t = cmk<V>(o[k].x * wr - o[k].y * wi, o[k].x * wi + o[k].y * wr);
       }
-      v[k] = cadd(e[k], t);
-      v[k + N / 2] = csub(e[k], t);
+      v[k] = padd(e[k], t);
+      v[k + N / 2] = psub(e[k], t);
     }
   }
 };
