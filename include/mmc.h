@@ -57,9 +57,9 @@ enum mmc_term {
 enum mmc_ovf_format { MMC_OVF_BINARY4 = 0, MMC_OVF_BINARY8 = 1, MMC_OVF_TEXT = 2 };
 
 /* How sweeps are executed.  AUTO picks FUSED for films (nz = 1, demag on, two
- * sublattice colours) where it is the faster one -- in FP32 always, in FP64 for
- * small films without a power-of-two transform -- and KERNELS otherwise.  Both
- * give the same decisions. */
+ * sublattice colours) where it is the faster one -- small films, and FP32 films
+ * without power-of-two transforms -- and KERNELS otherwise.  Both give the same
+ * decisions. */
 enum mmc_engine {
   MMC_ENGINE_AUTO = 0,
   MMC_ENGINE_KERNELS = 1,  /* one kernel per transform pass and colour, replayed from CUDA graphs */
@@ -399,9 +399,9 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
  * fetched by bulk asynchronous copies (as 3; a run whose buffer wait runs out
  * of its time limit returns MMC_ERR_TIMEOUT), whether the pass kernels expand their transforms in
  * line (1) or call them out of line (0), whether the column passes
- * transform in place reading the tensor from global memory (1; 2 the same,
- * with film y lines of length 64 or 256 held in registers, other lines as 1;
- * 3 as 2 with one component per thread),
+ * transform in place reading the tensor from global memory (1; 2 and 3 the
+ * same, with FP32 film y lines of length 32 to 256 by the pipelined pass, other
+ * lines as 1),
  * and the number of streams (1-4) the batch's replicas are split over. */
 int mmc_batch_launch_shape(mmc_batch* b, int out[10]);
 /* Autotuner: times each launch shape this batch can run with (the film row

@@ -127,13 +127,32 @@ __device__ __forceinline__ V cmacc(V acc, V a, V b) {
   return cadd(acc, cmulc(a, b));
 }
 
+// The products of the power-of-two transforms and of the tensor with the
+// contraction written out in FP32, the one the compiler chose for cmul and
+// cmulc in the first passes: which product of a sum it fuses depends on the code
+// around, and every pass has to round alike.
+template <typename V>
+__device__ __forceinline__ V tmul(V a, V b) {
+  return cmul(a, b);
+}
+template <typename V>
+__device__ __forceinline__ V tmulc(V a, V b) {
+  return cmulc(a, b);
+}
+__device__ __forceinline__ float2 tmul(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float2 tmulc(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, -__fmul_rn(a.x, b.y)));
+}
+
 // K^ . M^ at one frequency (src/demag_cu.cu:98-111): the real and imaginary
 // parts of sum_b K_ab M_b for a = x, y, z, from the six tensor blocks.
 template <typename V>
 __device__ __forceinline__ V tensor_row(V mx, V my, V mz, V k0, V k1, V k2) {
   if constexpr (fused_mul<V>) return cmac(cmac(cmul(mx, k0), my, k1), mz, k2);
-  return cmk<V>((mx.x * k0.x - mx.y * k0.y) + (my.x * k1.x - my.y * k1.y) + (mz.x * k2.x - mz.y * k2.y),
-                (mx.x * k0.y + mx.y * k0.x) + (my.x * k1.y + my.y * k1.x) + (mz.x * k2.y + mz.y * k2.x));
+  const V p0 = tmul(mx, k0), p1 = tmul(my, k1), p2 = tmul(mz, k2);
+  return padd(padd(p0, p1), p2);
 }
 
 template <typename T>
@@ -374,22 +393,23 @@ struct RegDft<T, INV, 1> {
 // group), with the input already in registers: v[a] = x[b + B a].
 //   x[b + B a] --(A-point DFT over a)--> Y[b][ka] --(* W_N^(b ka))-->
 //   transpose in the line --(B-point DFT over b)--> X[ka + A kb].
-// Lp is the line in shared memory, used for the transpose; it holds X in
-// natural order on return.  All lanes of the warp must call it (inactive
-// groups with active = false); `roots` holds exp(-2 pi i j / N), j < N.
+// On return lane b holds the columns ka = b Q + t, t < Q = A / B: v[t B + kb] =
+// X[ka + A kb].  Lp is the line's room in shared memory for the transpose.  All
+// lanes of the warp must call it (inactive groups with active = false).
+// roots: exp(-2 pi i j / N), j < N, or (LANES) the same roots as [ka][b].
 // The transpose goes through rows of B + 1 elements when PAD (row ka at
 // ka (B + 1): every address is the lane's base plus a compile-time offset,
 // and the line then needs N + A - 1 elements of room), else through rows of
 // B with the columns rotated by ka (N elements of room).
-template <typename T, bool INV, int A, int B, bool PAD = false>
-__device__ __forceinline__ void fft_line_regs(C<T> (&v)[A], C<T>* Lp, int b, bool active, const C<T>* roots) {
+template <typename T, bool INV, int A, int B, bool PAD = false, bool LANES = false>
+__device__ __forceinline__ void fft_line_cols(C<T> (&v)[A], C<T>* Lp, int b, bool active, const C<T>* roots) {
   using V = C<T>;
   constexpr int Q = A / B;
   RegDft<T, INV, A>::run(v);
 #pragma unroll
   for (int ka = 1; ka < A; ++ka) {
-    const V w = roots[b * ka];
-    v[ka] = INV ? cmulc(v[ka], w) : cmul(v[ka], w);
+    const V w = LANES ? roots[ka * B + b] : roots[b * ka];
+    v[ka] = INV ? tmulc(v[ka], w) : tmul(v[ka], w);
   }
   __syncwarp();
   if (active) {
@@ -422,6 +442,13 @@ __device__ __forceinline__ void fft_line_regs(C<T> (&v)[A], C<T>* Lp, int b, boo
   }
 #pragma unroll
   for (int t = 0; t < Q; ++t) RegDft<T, INV, B>::run(v + t * B);
+}
+
+// The same with X left in Lp in natural order.
+template <typename T, bool INV, int A, int B, bool PAD = false>
+__device__ __forceinline__ void fft_line_regs(C<T> (&v)[A], C<T>* Lp, int b, bool active, const C<T>* roots) {
+  constexpr int Q = A / B;
+  fft_line_cols<T, INV, A, B, PAD>(v, Lp, b, active, roots);
   __syncwarp();
   if (active) {
 #pragma unroll

@@ -124,7 +124,7 @@ __host__ __device__ inline Fused2DLayout fused2d_layout(const Geom& g, const Fft
                                                         int nblocks) {
   Fused2DLayout L;
   const size_t cs = sizeof(C<T>);
-  L.npairs = g.hxp / 2;
+  L.npairs = (g.hx + 1) / 2;
   L.items = (L.npairs + nblocks - 1) / nblocks;
   L.resident = L.items <= FUSED_MAX_RES ? L.items : 0;
   L.rowph = row_phase_bytes<T>(g, px, band, true, (size_t)6 * (py.n + 1));

@@ -44,6 +44,13 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// 16-byte asynchronous copy from global to shared memory.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // =========================================================== demag passes
 //
 // The reference computes H^ = K^ . M^ / N with three cuFFT R2C transforms and
@@ -317,6 +324,167 @@ __global__ void __launch_bounds__(256, x_w_min_blocks<T, A>()) k_x_inverse_w(Fft
   }
 }
 
+// The FP32 x passes.  The same lines, transforms and splits as k_x_forward_w /
+// k_x_inverse_w, bit for bit, with each line finished by the warp that holds
+// it: the split needs X[L - k] beside X[k], which sits in the mirrored lane's
+// registers (two shuffles per value instead of a line written to shared memory
+// and read back twice), and the inverse's rows go straight to global memory.
+// Shared memory carries the transposes only, so the kernel has no barrier after
+// its table of roots, which it holds in the lanes' order (the products b ka of
+// the plain order meet in the same banks).  What bounded k_x_forward_w was the
+// shared-memory pipe (84 % busy at 64 x 256^2).
+// SPLIT: m and h rows in the colour-split order (see k_mc_split): cell x of row
+// (y, z) at split_pos(x, y + z, nx); a lane's values have one parity (B and A
+// are even), so its addresses stay a base plus a compile-time step.
+__host__ __device__ __forceinline__ int split_pos(int x, int yz, int nx) {
+  return ((x + yz) & 1) * (nx >> 1) + (x >> 1);
+}
+template <int A>
+constexpr int x_r_min_blocks() {
+  return A >= 32 ? 2 : 4;
+}
+template <int A, int B>
+__device__ __forceinline__ void load_lane_roots(const FftPlan& p, float2* dst) {
+  const float2* src = p.tw32 + p.lane_off;
+  for (int i = threadIdx.x; i < A * B; i += blockDim.x) dst[i] = src[i];
+}
+template <int A, int B, bool SPLIT>
+__global__ void __launch_bounds__(256, x_r_min_blocks<A>())
+    k_x_forward_r(FftPlan p, int xdata, FastDiv dyd, int nrows, const float* __restrict__ in, long long in_cstride,
+                  float2* __restrict__ S, long long nspec, int nyp, int hx, int pitch, int rows_per_cta,
+                  long long in_rstride, long long s_rstride) {
+  using V = float2;
+  constexpr int L = A * B, GPW = 32 / B, Q = A / B, LS = L + A;
+  const int ydata = (int)dyd.d;
+  in += blockIdx.z * in_rstride;
+  S += blockIdx.z * s_rstride;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V* roots = reinterpret_cast<V*>(smem_raw);
+  load_lane_roots<A, B>(p, roots);
+  pdl_wait();
+  __syncthreads();
+  const int row0 = blockIdx.x * rows_per_cta;
+  const int nr = min(rows_per_cta, nrows - row0);
+  const int nlines = 2 * nr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int grp = lane / B, b = lane - grp * B;
+  V* Lp = roots + L + (warp * GPW + grp) * LS;
+  for (int line0 = warp * GPW; line0 < nlines; line0 += nwarps * GPW) {
+    const int line = line0 + grp;
+    const bool active = line < nlines;
+    const int pr = line >= nr ? 1 : 0, row = row0 + (active ? line - pr * nr : 0);
+    const int z = dyd.div(row), y = row - z * ydata;
+    V v[A];
+    if (active) {
+      const float* re = in + (long long)(2 * pr) * in_cstride + (long long)row * xdata +
+                        (SPLIT ? split_pos(b, y + z, xdata) : b);
+#pragma unroll
+      for (int a = 0; a < A; ++a) {
+        const int o = SPLIT ? B / 2 * a : B * a;
+        const bool ok = b + B * a < xdata;
+        v[a] = make_float2(ok ? re[o] : 0.0f, (ok && pr == 0) ? re[in_cstride + o] : 0.0f);
+      }
+    }
+    fft_line_cols<float, false, A, B, true, true>(v, Lp, b, active, roots);
+    V* so = S + (long long)(2 * pr) * nspec + ((long long)z * nyp + y) * pitch;
+    // this lane's columns ka = b Q + t, the half kb < B / 2 (k < L / 2): the mirror
+    // of X[ka + A kb] is X[A - ka + A (B - 1 - kb)] in lane B - b (t = 0) or
+    // B - 1 - b (column Q - t there); lane 0's column 0 mirrors onto itself, kb to B - kb
+#pragma unroll
+    for (int kb = 0; kb < B / 2; ++kb) {
+#pragma unroll
+      for (int t = 0; t < Q; ++t) {
+        const V a = v[t * B + kb];
+        V m;
+        if (t == 0) {
+          const V s0 = v[(B - kb) & (B - 1)], s1 = v[B - 1 - kb];
+          m.x = __shfl_sync(0xffffffffu, b == 0 ? s0.x : s1.x, (B - b) & (B - 1), B);
+          m.y = __shfl_sync(0xffffffffu, b == 0 ? s0.y : s1.y, (B - b) & (B - 1), B);
+        } else {
+          const V s1 = v[(Q - t) * B + B - 1 - kb];
+          m.x = __shfl_sync(0xffffffffu, s1.x, B - 1 - b, B);
+          m.y = __shfl_sync(0xffffffffu, s1.y, B - 1 - b, B);
+        }
+        const int k = b * Q + t + A * kb;
+        if (active) {
+          so[k] = make_float2(0.5f * (a.x + m.x), 0.5f * (a.y - m.y));
+          if (pr == 0) so[nspec + k] = make_float2(0.5f * (a.y + m.y), -0.5f * (a.x - m.x));
+        }
+      }
+    }
+    if (active && b == 0) {  // k = L / 2 mirrors onto itself
+      const V a = v[B / 2];
+      so[L / 2] = make_float2(0.5f * (a.x + a.x), 0.5f * (a.y - a.y));
+      if (pr == 0) so[nspec + L / 2] = make_float2(0.5f * (a.y + a.y), -0.5f * (a.x - a.x));
+    }
+  }
+}
+
+template <int A, int B, bool SPLIT>
+__global__ void __launch_bounds__(256, x_r_min_blocks<A>())
+    k_x_inverse_r(FftPlan p, const float2* __restrict__ S, long long nspec, int nyp, int hx, int pitch, FastDiv dxo,
+                  FastDiv dyo, int nrows, float* __restrict__ out, long long out_cstride, int rows_per_cta,
+                  long long s_rstride, long long out_rstride) {
+  using V = float2;
+  constexpr int L = A * B, GPW = 32 / B, Q = A / B, LS = L + A;
+  const int xout = (int)dxo.d, yout = (int)dyo.d;
+  S += blockIdx.z * s_rstride;
+  out += blockIdx.z * out_rstride;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V* roots = reinterpret_cast<V*>(smem_raw);
+  load_lane_roots<A, B>(p, roots);
+  pdl_wait();
+  __syncthreads();
+  const int row0 = blockIdx.x * rows_per_cta;
+  const int nr = min(rows_per_cta, nrows - row0);
+  const int nlines = 2 * nr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int grp = lane / B, b = lane - grp * B;
+  V* Lp = roots + L + (warp * GPW + grp) * LS;
+  for (int line0 = warp * GPW; line0 < nlines; line0 += nwarps * GPW) {
+    const int line = line0 + grp;
+    const bool active = line < nlines;
+    const int pr = line >= nr ? 1 : 0, row = row0 + (active ? line - pr * nr : 0);
+    const int z = dyo.div(row), y = row - z * yout;
+    V v[A];
+    if (active) {
+      const V* si = S + (long long)(2 * pr) * nspec + ((long long)z * nyp + y) * pitch;
+#pragma unroll
+      for (int a = 0; a < A; ++a) {
+        const int k = b + B * a;
+        const int kk = k < hx ? k : L - k;
+        V u0 = si[kk];
+        if (k >= hx) u0.y = -u0.y;
+        if (k == 0 || 2 * k == L) u0.y = 0;  // bins that are real for a real output
+        if (pr == 0) {
+          V u1 = si[nspec + kk];
+          if (k >= hx) u1.y = -u1.y;
+          if (k == 0 || 2 * k == L) u1.y = 0;
+          v[a] = make_float2(u0.x - u1.y, u0.y + u1.x);
+        } else {
+          v[a] = u0;
+        }
+      }
+    }
+    fft_line_cols<float, true, A, B, true, true>(v, Lp, b, active, roots);
+    if (active) {
+      float* o = out + (long long)(2 * pr) * out_cstride + (long long)row * xout;
+#pragma unroll
+      for (int t = 0; t < Q; ++t) {
+        const int x0 = b * Q + t;
+        float* ot = o + (SPLIT ? split_pos(x0, y + z, xout) : x0);
+#pragma unroll
+        for (int kb = 0; kb < B; ++kb) {
+          if (x0 + A * kb >= xout) continue;
+          const int d = SPLIT ? A / 2 * kb : A * kb;
+          ot[d] = v[t * B + kb].x;
+          if (pr == 0) ot[out_cstride + d] = v[t * B + kb].y;
+        }
+      }
+    }
+  }
+}
+
 // PASS_SYM (with PASS_MUL): multiply by the real part of K^ only, i.e. by the
 // spectrum of (K(r) + K(-r)) / 2 -- the symmetrised tensor of the energy's
 // adjoint.
@@ -465,212 +633,182 @@ __global__ void __launch_bounds__(256) k_col_pass_wide(FftPlan p, int ncomp, C<T
                               inv_n, tx, s_rstride, lean);
 }
 
-// Column pass of a film (the y lines, with the K^ product between the forward
-// and the inverse transform) for lengths A x A (64, 256) with the lines held
-// in registers.  A CTA takes CR_TX kx columns; thread (t, b), t = threadIdx.x
-// mod CR_TX, holds the values y = b + A a (a = 0 .. A-1) of the three
-// components of column kx0 + t, loaded straight from the spectrum (CR_TX
-// consecutive kx per row: whole sectors).  The forward transform is the
-// arithmetic of fft_line_regs<T, false, A, A>: an A-point DFT over a in
-// registers, the twiddles W^(b ka), a transpose among the A threads of the
-// column through shared memory, an A-point DFT -- after which thread (t, b)
-// holds the frequencies b + A kb, the layout the inverse starts from, so the
-// K^ product and the inverse (fft_line_regs<T, true, A, A>'s arithmetic) run
-// from the same registers and the results go straight back.  No line is
-// staged in shared memory, and the transform, the product and the loads
-// round exactly as in k_col_pass: the same results bit for bit, with about
-// 40 % fewer instructions (ncu: 9.9 M against 17.0 M warp instructions for 32
-// replicas of 256^2).  Holding three lines per thread takes 255 registers, so
-// 2 CTAs of 128 threads fit per SM (12 % of the warp slots) and the loads'
-// latency is exposed: at 256^2 it runs at k_col_pass's speed (32.2 against
-// 33.0 us per batched sweep).  Capping it at 168 registers (3 CTAs) spilled
-// and took 44.8 us; transforming one component at a time with the others
-// parked in shared memory (126 registers) took 36.3 us.  It is an autotuner
-// candidate (col_lean = 2).
-constexpr int CR_TX = 8;  // kx columns per CTA
-template <int A>
-__host__ __device__ constexpr int col_reg_row() {
-  return A * CR_TX + 8;  // transpose row (complex): conflict-free 8-byte accesses both ways
+// Column pass of FP32 films (the y lines, with the K^ product between the
+// forward and the inverse transform) for lengths A B = 32, 64, 128 and 256, by
+// persistent CTAs.  An item is a tile of TX kx columns of one replica; CTA i
+// takes `chunk` items, consecutive replicas of one tile, so K^'s tile stays in
+// shared memory (read once per CTA, before the wait on the x pass).  The next
+// item's columns arrive by asynchronous copies while the current one is
+// transformed, which is what the kernel is for: the register-held pass it
+// replaces (three components per thread, 255 registers, 8 warps per SM) spent
+// half of its time waiting for its loads.  Thread (c, b, t) of 3 B TX holds the
+// values y = b + B a of component c of column t: the arithmetic of
+// fft_line_cols forward, a meeting of the three components in shared memory
+// for the product, and fft_line_cols inverse; each rounds as in k_col_pass, so
+// the results are the same bit for bit.  Two CTAs of 192 threads per SM.
+// 64 x 256^2: 48.4 -> 41 us; 4 x 256^2, a whole sweep: 22.1 -> 18.8.
+template <int B>
+__host__ __device__ constexpr int cp_tx() {
+  return 64 / B;
 }
-template <typename T, int A>
-__host__ __device__ inline size_t col_reg_smem() {
-  return ((size_t)A * A + 3 * (size_t)A * col_reg_row<A>()) * sizeof(C<T>);
+template <int A, int B>
+__host__ __device__ constexpr int cp_row() {  // transpose row: conflict-free both ways
+  return B * cp_tx<B>() + (A == 8 ? 8 : 4);
 }
+template <int A, int B>
+__host__ __device__ constexpr int cp_region() {  // one component's room: the tile's lines, then the transposes
+  constexpr int L = A * B * cp_tx<B>(), T = A * cp_row<A, B>();
+  return L > T ? L : T;
+}
+template <int A, int B>
+__host__ __device__ constexpr size_t col_pipe_smem() {
+  return ((size_t)6 * A * B * cp_tx<B>() + 2 * 3 * cp_region<A, B>()) * sizeof(float2);
+}
+// The 64 threads of one component meet (two whole warps).
+__device__ __forceinline__ void cp_bar(int c) { asm volatile("bar.sync %0, 64;" ::"r"(c + 1) : "memory"); }
 
-// The three components' lines of column t: DFT over the thread's A values,
-// twiddles, transpose (tb: three buffers of A rows), DFT.  first: the
-// buffers are not being read by an earlier transform.
-template <typename T, bool INV, int A>
-__device__ __forceinline__ void col_reg_transform3(C<T> (&v)[3][A], C<T>* tb, const C<T>* roots, int t, int b,
-                                                   bool first) {
-  using V = C<T>;
-  constexpr int RW = col_reg_row<A>();
-#pragma unroll
-  for (int c = 0; c < 3; ++c) RegDft<T, INV, A>::run(v[c]);
+// The column's transform from v (positions b + B a) to v[t B + kb] = X[(b Q + t) + A kb].
+template <bool INV, int A, int B>
+__device__ __forceinline__ void cp_transform(float2 (&v)[A], float2* reg, const float2 (&tw)[A], int c, int b, int t) {
+  constexpr int Q = A / B, TX = cp_tx<B>(), RW = cp_row<A, B>();
+  RegDft<float, INV, A>::run(v);
 #pragma unroll
   for (int ka = 1; ka < A; ++ka) {
-    const V w = roots[b * ka];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) v[c][ka] = INV ? cmulc(v[c][ka], w) : cmul(v[c][ka], w);
+    v[ka] = INV ? tmulc(v[ka], tw[ka]) : tmul(v[ka], tw[ka]);
   }
-  if (!first) __syncthreads();
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int ka = 0; ka < A; ++ka) reg[ka * RW + b * TX + t] = v[ka];
+  cp_bar(c);
 #pragma unroll
-    for (int ka = 0; ka < A; ++ka) tb[(c * A + ka) * RW + b * CR_TX + t] = v[c][ka];
-  __syncthreads();
+  for (int q = 0; q < Q; ++q) {
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-#pragma unroll
-    for (int bb = 0; bb < A; ++bb) v[c][bb] = tb[(c * A + b) * RW + bb * CR_TX + t];
-    RegDft<T, INV, A>::run(v[c]);
+    for (int bb = 0; bb < B; ++bb) v[q * B + bb] = reg[(b * Q + q) * RW + bb * TX + t];
+    RegDft<float, INV, B>::run(v + q * B);
   }
 }
 
-template <typename T, int A>
-__global__ void __launch_bounds__(CR_TX * A) k_col_reg(FftPlan p, C<T>* __restrict__ S, long long nspec,
-                                                          const C<T>* __restrict__ khat, int hx, int pitch,
-                                                          int load_lim, int store_lim, int flags, T inv_n,
-                                                          long long s_rstride) {
-  using V = C<T>;
-  constexpr int L = A * A;
+template <int A, int B>
+__global__ void __launch_bounds__(192, 2)
+    k_col_pipe(const __grid_constant__ FftPlan p, float2* __restrict__ S, long long nspec,
+               const float2* __restrict__ khat, int hx, int pitch, int load_lim, int store_lim, int sym, float inv_n,
+               int nrep, int items, int chunk) {
+  using V = float2;
+  constexpr int L = A * B, Q = A / B, TX = cp_tx<B>(), RG = cp_region<A, B>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* roots = reinterpret_cast<V*>(smem_raw);  // exp(-2 pi i j / L), j < L
-  V* tb = roots + L;
-  S += blockIdx.z * s_rstride;
-  const int t = threadIdx.x % CR_TX, b = threadIdx.x / CR_TX;
-  const int kx = blockIdx.x * CR_TX + t;
-  const bool ok = kx < hx;
-  {
-    const V* src = plan_tw<T>(p) + p.full_off;
-    for (int i = threadIdx.x; i < L; i += blockDim.x) roots[i] = src[i];
-  }
-  pdl_wait();  // the spectrum is the x pass's output
-  V v[3][A];
+  V* kt = reinterpret_cast<V*>(smem_raw);  // K^ tile [block][pos][t]
+  V* buf0 = kt + 6 * L * TX;               // two buffers of three regions
+  const int c = threadIdx.x >> 6, u = threadIdx.x & 63, t = u & (TX - 1), b = u / TX;
+  const int i0 = blockIdx.x * chunk, i1 = min(items, i0 + chunk);
+  // copies: thread u of a component's 64 moves the 16-byte piece lt of rows lr, lr + LR, ...
+  constexpr int LR = 64 / (TX / 2);
+  const int lr = u / (TX / 2), lt = 2 * (u & (TX / 2 - 1));
+  auto load_k = [&](int tile) {
+    const int kx = tile * TX + lt;
+    if (kx < pitch) {
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int a = 0; a < A; ++a) {
-      const int row = b + A * a;
-      v[c][a] = (ok && row < load_lim) ? S[c * nspec + (long long)row * pitch + kx] : cmk<V>(0, 0);
+      for (int q = 0; q < 2; ++q) {
+        const V* src = khat + (2 * c + q) * nspec + (long long)lr * pitch + kx;
+        V* d = kt + ((2 * c + q) * L + lr) * TX + lt;
+#pragma unroll 4
+        for (int r = 0; r < L; r += LR) cp_async16(d + r * TX, src + (long long)r * pitch);
+      }
     }
-  __syncthreads();  // roots
-  col_reg_transform3<T, false, A>(v, tb, roots, t, b, true);
-  // K^ . M^ / N
+  };
+  // item i's columns, rows load_lim and above 0
+  auto load_item = [&](int i, V* buf) {
+    const int tile = i / nrep, kx = tile * TX + lt;
+    const V* src = S + ((long long)(i - tile * nrep) * 3 + c) * nspec + (long long)lr * pitch + kx;
+    V* d = buf + c * RG + lr * TX + lt;
 #pragma unroll
-  for (int kb = 0; kb < A; ++kb) {
-    const int pos = b + A * kb;
-    const V* kk = khat + (long long)pos * pitch + (ok ? kx : 0);
-    V kxx = kk[0], kxy = kk[nspec], kxz = kk[2 * nspec];
-    V kyy = kk[3 * nspec], kyz = kk[4 * nspec], kzz = kk[5 * nspec];
-    if (flags & PASS_SYM) kxx.y = kxy.y = kxz.y = kyy.y = kyz.y = kzz.y = (T)0;
-    const V mx = v[0][kb], my = v[1][kb], mz = v[2][kb];
-    const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
-    const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
-    const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
-    v[0][kb] = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
-    v[1][kb] = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
-    v[2][kb] = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
-  }
-  col_reg_transform3<T, true, A>(v, tb, roots, t, b, false);
-  if (!ok) return;
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int kb = 0; kb < A; ++kb) {
-      const int row = b + A * kb;
-      if (row < store_lim) S[c * nspec + (long long)row * pitch + kx] = v[c][kb];
+    for (int r = 0; r < L; r += LR) {
+      if (lr + r < load_lim && kx < pitch)
+        cp_async16(d + r * TX, src + (long long)r * pitch);
+      else
+        *reinterpret_cast<float4*>(d + r * TX) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-}
-
-// The same column pass with each component held by threads of its own:
-// thread (c, t, b) of 3 CR_TX A holds component c of column t (k_col_reg's
-// values y = b + A a).  Each component is transformed by exactly k_col_reg's
-// arithmetic (col_reg_transform1, its own transpose buffer); for the K^
-// product every thread writes its frequencies into its buffer in the
-// transposes' layout and reads the other two components' from theirs, then
-// forms its own component of sum_b K_ab M_b with k_col_reg's expressions.
-// The results equal k_col_reg's (and k_col_pass's) bit for bit.  At 256^2
-// (A = 16) it holds 168 registers per thread -- 12 warps per SM against
-// k_col_reg's 8 -- and takes 30.3-31.1 us per batch of 32 replicas against
-// 32.4; capped at 80 registers for two CTAs per SM it spilled and took 36.7,
-// and 4 columns per CTA (192 threads, two CTAs per SM at 168 registers, less
-// of the 129th column's tile wasted) took 30.6.  An autotuner candidate
-// (col_lean = 3).
-template <typename T, bool INV, int A>
-__device__ __forceinline__ void col_reg_transform1(C<T> (&v)[A], C<T>* tb, const C<T>* roots, int t, int b,
-                                                   bool first) {
-  using V = C<T>;
-  constexpr int RW = col_reg_row<A>();
-  RegDft<T, INV, A>::run(v);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  V tw[A];  // this thread's roots b ka
 #pragma unroll
-  for (int ka = 1; ka < A; ++ka) {
-    const V w = roots[b * ka];
-    v[ka] = INV ? cmulc(v[ka], w) : cmul(v[ka], w);
-  }
-  if (!first) __syncthreads();
-#pragma unroll
-  for (int ka = 0; ka < A; ++ka) tb[ka * RW + b * CR_TX + t] = v[ka];
-  __syncthreads();
-#pragma unroll
-  for (int bb = 0; bb < A; ++bb) v[bb] = tb[b * RW + bb * CR_TX + t];
-  RegDft<T, INV, A>::run(v);
-}
-
-template <typename T, int A>
-__global__ void __launch_bounds__(3 * CR_TX * A)
-    k_col_reg3(FftPlan p, C<T>* __restrict__ S, long long nspec, const C<T>* __restrict__ khat, int hx, int pitch,
-               int load_lim, int store_lim, int flags, T inv_n, long long s_rstride) {
-  using V = C<T>;
-  constexpr int L = A * A, RW = col_reg_row<A>(), NT = CR_TX * A;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* roots = reinterpret_cast<V*>(smem_raw);  // exp(-2 pi i j / L), j < L
-  V* tb = roots + L;                          // three buffers of A rows of RW
-  S += blockIdx.z * s_rstride;
-  const int c = threadIdx.x / NT, tt = threadIdx.x - c * NT;  // c is warp-uniform
-  const int t = tt % CR_TX, b = tt / CR_TX;
-  const int kx = blockIdx.x * CR_TX + t;
-  const bool ok = kx < hx;
-  {
-    const V* src = plan_tw<T>(p) + p.full_off;
-    for (int i = threadIdx.x; i < L; i += blockDim.x) roots[i] = src[i];
-  }
+  for (int ka = 1; ka < A; ++ka) tw[ka] = p.tw32[p.lane_off + ka * B + b];
+  int tile = i0 / nrep;
+  load_k(tile);
   pdl_wait();  // the spectrum is the x pass's output
-  V v[A];
-#pragma unroll
-  for (int a = 0; a < A; ++a) {
-    const int row = b + A * a;
-    v[a] = (ok && row < load_lim) ? S[c * nspec + (long long)row * pitch + kx] : cmk<V>(0, 0);
-  }
-  __syncthreads();  // roots
-  V* tbc = tb + (size_t)c * A * RW;
-  col_reg_transform1<T, false, A>(v, tbc, roots, t, b, true);
-  __syncthreads();  // every thread has read its transpose
-#pragma unroll
-  for (int kb = 0; kb < A; ++kb) tbc[kb * RW + b * CR_TX + t] = v[kb];
-  __syncthreads();
-  // row c of K^: (xx, xy, xz), (xy, yy, yz) or (xz, yz, zz) in the six blocks
-  // xx, xy, xz, yy, yz, zz
+  load_item(i0, buf0);
+  // row c of K^: (xx, xy, xz), (xy, yy, yz) or (xz, yz, zz) in the six blocks xx, xy, xz, yy, yz, zz
   const int o0 = c, o1 = c == 0 ? 1 : c == 1 ? 3 : 4, o2 = c == 0 ? 2 : c == 1 ? 4 : 5;
-  // K^ . M^ / N
+  for (int i = i0; i < i1; ++i) {
+    V* buf = buf0 + ((i - i0) & 1) * 3 * RG;
+    const int it = i / nrep;
+    if (it != tile) {  // the chunk runs on into the next tile: every thread is past the last product
+      tile = it;
+      load_k(tile);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    cp_async_wait_all();
+    __syncthreads();  // the item has landed; the other buffer is free
+    if (i + 1 < i1) load_item(i + 1, buf0 + ((i + 1 - i0) & 1) * 3 * RG);
+    V* reg = buf + c * RG;
+    V v[A];
 #pragma unroll
-  for (int kb = 0; kb < A; ++kb) {
-    const int pos = b + A * kb;
-    const V* kk = khat + (long long)pos * pitch + (ok ? kx : 0);
-    V k0 = kk[o0 * nspec], k1 = kk[o1 * nspec], k2 = kk[o2 * nspec];
-    if (flags & PASS_SYM) k0.y = k1.y = k2.y = (T)0;
-    const int q = kb * RW + b * CR_TX + t;
-    const V mx = tb[q], my = tb[A * RW + q], mz = tb[2 * A * RW + q];
-    const V hc = tensor_row(mx, my, mz, k0, k1, k2);
-    v[kb] = cmk<V>(hc.x * inv_n, hc.y * inv_n);
-  }
-  col_reg_transform1<T, true, A>(v, tbc, roots, t, b, false);
-  if (!ok) return;
+    for (int a = 0; a < A; ++a) v[a] = reg[(b + B * a) * TX + t];
+    cp_bar(c);
+    cp_transform<false, A, B>(v, reg, tw, c, b, t);
+    cp_bar(c);
 #pragma unroll
-  for (int kb = 0; kb < A; ++kb) {
-    const int row = b + A * kb;
-    if (row < store_lim) S[c * nspec + (long long)row * pitch + kx] = v[kb];
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int kb = 0; kb < B; ++kb) reg[(b * Q + q + A * kb) * TX + t] = v[q * B + kb];
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < A; ++a) {  // K^ . M^ / N
+      const int e = (b + B * a) * TX + t;
+      V k0 = kt[o0 * L * TX + e], k1 = kt[o1 * L * TX + e], k2 = kt[o2 * L * TX + e];
+      if (sym) k0.y = k1.y = k2.y = 0.0f;
+      V m0 = buf[e], m1 = buf[RG + e], m2 = buf[2 * RG + e];
+      const V h = tensor_row(m0, m1, m2, k0, k1, k2);
+      v[a] = make_float2(h.x * inv_n, h.y * inv_n);
+    }
+    __syncthreads();
+    cp_transform<true, A, B>(v, reg, tw, c, b, t);
+    const int kx = tile * TX + t;
+    if (kx < hx) {
+      V* dst = S + (long long)(i - it * nrep) * 3 * nspec + c * nspec + kx;
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int kb = 0; kb < B; ++kb) {
+          const int pos = b * Q + q + A * kb;
+          if (pos < store_lim) dst[(long long)pos * pitch] = v[q * B + kb];
+        }
+    }
   }
+}
+// Whether the pass has a k_col_pipe instance.
+inline bool col_pipe_ok(const FftPlan& p) {
+  return p.warp_a == 16 ? p.warp_b >= 8 : p.warp_a == 8;  // 256, 128, 64, 32
+}
+template <int A, int B>
+cudaError_t launch_col_pipe_ab(const FftPlan& p, float2* S, long long nspec, const float2* khat, int hx, int pitch,
+                               int load_lim, int store_lim, int sym, float inv_n, int nrep, cudaStream_t st) {
+  const int tiles = (hx + cp_tx<B>() - 1) / cp_tx<B>();
+  const long long items = (long long)tiles * nrep;
+  if (items > INT_MAX) return cudaErrorInvalidValue;
+  int dev = 0, nsm = 152;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int chunk = (int)((items + 2 * nsm - 1) / (2 * nsm));  // two CTAs per SM, all resident
+  return launch_pdl(k_col_pipe<A, B>, dim3((unsigned)((items + chunk - 1) / chunk)), dim3(192), col_pipe_smem<A, B>(),
+                    st, p, S, nspec, khat, hx, pitch, load_lim, store_lim, sym, inv_n, nrep, (int)items, chunk);
+}
+inline cudaError_t launch_col_pipe(const FftPlan& p, float2* S, long long nspec, const float2* khat, int hx, int pitch,
+                                   int load_lim, int store_lim, int sym, float inv_n, int nrep, cudaStream_t st) {
+  auto f = p.n == 256   ? launch_col_pipe_ab<16, 16>
+           : p.n == 128 ? launch_col_pipe_ab<16, 8>
+           : p.n == 64  ? launch_col_pipe_ab<8, 8>
+                        : launch_col_pipe_ab<8, 4>;
+  return f(p, S, nspec, khat, hx, pitch, load_lim, store_lim, sym, inv_n, nrep, st);
 }
 
 // Column pass for short lines (n <= 16: the padded z axis of thin 3-D
@@ -848,17 +986,29 @@ struct Prop<float> {
   // absolute error is about 4e-7, negated (exact), and sqrt(t) as t / sqrt(t)
   // from the hardware reciprocal square root; t = 1 - z^2 >= 2^-22 because
   // u01_f32 never returns 0 or 1.
+  // The flush-to-zero forms of rsqrt and ex2 skip the scaling of denormal
+  // arguments and results: t is normal, and a denormal exponential loses
+  // against every ua >= 2^-24 like 0 does.
+  // (r >> 9) + 1/2 in units of 2^-23, as mmcm::u01_f32: the word's upper bits
+  // become the mantissa of a number in [1, 2), and 1 - 2^-24 comes off exactly.
+  __device__ static float u01(uint32_t r) { return __uint_as_float((r >> 9) + 0x3f800000u) - 0x1.fffffep-1f; }
   __device__ static void draw(mmcm::u32x4 r, float& px, float& py, float& pz, float& ua) {
-    pz = 2.0f * mmcm::u01_f32(r.x) - 1.0f;
+    pz = 2.0f * u01(r.x) - 1.0f;
     const float t = 1.0f - pz * pz;
-    const float s = t * rsqrtf(t);
+    float q;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(t));
+    const float s = t * q;
     float sn, cs;
-    __sincosf(6.28318530717958647692f * mmcm::u01_f32(r.y) - 3.14159265358979323846f, &sn, &cs);
+    __sincosf(6.28318530717958647692f * u01(r.y) - 3.14159265358979323846f, &sn, &cs);
     px = -(s * cs);
     py = -(s * sn);
-    ua = mmcm::u01_f32(r.z);
+    ua = u01(r.z);
   }
-  __device__ static bool accept(float dE, float ua) { return dE <= 0.0f || ua < __expf(-dE); }
+  __device__ static bool accept(float dE, float ua) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-dE * 1.44269504088896340736f));
+    return dE <= 0.0f || ua < e;
+  }
 };
 
 // Neighbour values of one trial: v[a][s] is the neighbour along axis a on side
@@ -890,9 +1040,10 @@ struct Proposal<double> {
 };
 
 template <typename T>
-__device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t cell, uint32_t stage, uint32_t sweep) {
+__device__ __forceinline__ Proposal<T> mc_propose(uint32_t key0, uint32_t key1, uint32_t cell, uint32_t stage,
+                                                  uint32_t sweep) {
   mmcm::u32x4 ctr = {cell, sweep, stage, mmcm::STREAM_SWEEP};
-  mmcm::u32x4 r = mmcm::philox4x32_10(ctr, c.key0, c.key1);
+  mmcm::u32x4 r = mmcm::philox4x32_10(ctr, key0, key1);
   Proposal<T> p;
   if constexpr (sizeof(T) == 8) {
     p.rx = r.x;
@@ -902,6 +1053,11 @@ __device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t c
     Prop<T>::draw(r, p.x, p.y, p.z, p.ua);
   }
   return p;
+}
+
+template <typename T>
+__device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t cell, uint32_t stage, uint32_t sweep) {
+  return mc_propose<T>(c.key0, c.key1, cell, stage, sweep);
 }
 
 // ---------------------------------------------- the FP64 trial's FP32 filter
@@ -999,15 +1155,33 @@ __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&
 // The Metropolis decision for one cell from its neighbour values, its own m,
 // its demag field h and its proposal.  Shared by every sweep kernel so that
 // all paths round identically.
+// SEP (FP32): the products of the first two neighbours are rounded before they
+// are added, where the chain of multiply-adds rounds the second with the sum.
+// The vectorised forms have always taken the first of a thread's two cells this
+// way (see mc_sep), the others the chain; written out, it does not depend on
+// what the compiler makes of the code around.
 template <typename T>
 __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy,
-                                                  T hz, T px, T py, T pz, T ua) {
+                                                  T hz, T px, T py, T pz, T ua, bool sep = false) {
   T Fx = 0, Fy = 0, Fz = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       if (!nb.has[a][s]) continue;
+      if constexpr (sizeof(T) == 4) {
+        const float w = c.wex[a], x = nb.v[a][s][0], y = nb.v[a][s][1], z = nb.v[a][s][2];
+        if (sep && a == 0 && s == 1) {
+          Fx = __fadd_rn(Fx, __fmul_rn(w, x));
+          Fy = __fadd_rn(Fy, __fmul_rn(w, y));
+          Fz = __fadd_rn(Fz, __fmul_rn(w, z));
+        } else {
+          Fx = __fmaf_rn(w, x, Fx);
+          Fy = __fmaf_rn(w, y, Fy);
+          Fz = __fmaf_rn(w, z, Fz);
+        }
+        continue;
+      }
       Fx = Fx + c.wex[a] * nb.v[a][s][0];
       Fy = Fy + c.wex[a] * nb.v[a][s][1];
       Fz = Fz + c.wex[a] * nb.v[a][s][2];
@@ -1067,7 +1241,7 @@ __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs
 // The decision; p's direction is the new m where it is true.
 template <typename T>
 __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy, T hz,
-                                          const Proposal<T>& p) {
+                                          const Proposal<T>& p, bool sep = false) {
   if constexpr (sizeof(T) == 8) {
     float v[3][2][3];
 #pragma unroll
@@ -1084,7 +1258,7 @@ __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb,
     p.get(px, py, pz);
     return mc_accept_formula<T>(c, nb, ox, oy, oz, hx, hy, hz, px, py, pz, mmcm::u01_f64(p.rz));
   } else {
-    return mc_accept_formula<T>(c, nb, ox, oy, oz, hx, hy, hz, p.x, p.y, p.z, p.ua);
+    return mc_accept_formula<T>(c, nb, ox, oy, oz, hx, hy, hz, p.x, p.y, p.z, p.ua, sep);
   }
 }
 
@@ -1356,6 +1530,14 @@ __device__ __forceinline__ void st4(T* p, const Vec4<T>& r) {
   }
 }
 
+// Whether the vectorised forms round the first exchange products separately
+// (mc_accept_formula) for cell q of a thread's two: the first one, on thick
+// lattices with an open x or y axis only in the layer that has none above it.
+template <bool ALLB, bool Z3>
+__device__ __forceinline__ bool mc_sep(int q, bool hzu) {
+  return q == 0 && (!Z3 || ALLB || !hzu);
+}
+
 // The decisions of the two cells at offsets P0 and P0 + 2 of a segment.
 // ALLB: every x and y bond exists (both axes periodic, ny > 1), so the
 // availability flags are compile-time true.  Z3: a 3-D lattice, with the
@@ -1392,7 +1574,8 @@ __device__ __forceinline__ bool quad_cells(const McCoef<T>& c, Vec4<T> (&own)[3]
       nb.v[2][1][k] = hzu ? zu[k].v[o] : ov;
     }
     const Proposal<T> pr = mc_propose<T>(c, cell0 + (uint32_t)o, stage, sweep);
-    if (mc_accept<T>(c, nb, own[0].v[o], own[1].v[o], own[2].v[o], hh[0].v[o], hh[1].v[o], hh[2].v[o], pr)) {
+    if (mc_accept<T>(c, nb, own[0].v[o], own[1].v[o], own[2].v[o], hh[0].v[o], hh[1].v[o], hh[2].v[o], pr,
+                     mc_sep<ALLB, Z3>(q, hzu))) {
       pr.get(own[0].v[o], own[1].v[o], own[2].v[o]);
       changed = true;
       ++mine;
@@ -1510,6 +1693,158 @@ __global__ void __launch_bounds__(256) k_mc_quad(Geom g, const McCoef<T>* __rest
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, (unsigned long long)v);
 }
 
+// --------------------------------------------------- colour-split Metropolis
+// One colour of a two-colour FP32 sweep on rows stored colour by colour: the
+// nx / 2 cells of colour 0 of row (y, z) first, then those of colour 1
+// (split_pos).  The cells of a launch's colour are then contiguous, and so are
+// their neighbours, all of the other colour: cell j of the row sees cell j of the
+// rows above and below and cells j and j - 1 (or j + 1, by the row's parity) of
+// its own row.  A thread takes two cells: it reads 15 pairs and 3 side cells
+// where k_mc_quad read 12 vectors of 4 and 3 side cells for two trials, of which
+// half were cells of no use to it.  Runs of at least MC_SPLIT_SWEEPS sweeps
+// convert m once at either end (k_split_rows); the x passes read and write the
+// split order at no cost.  Decisions: mc_propose / mc_accept on the same inputs
+// as every other form.  Latency and issue share the bound (58 % issue, loads the
+// top stall): the coefficients stay in shared memory so that 80 registers hold 24
+// warps per SM (102 registers and 16 warps with them in registers: 29 us; one
+// cell per thread, 32 warps: 31 us for its index work).  128 x 64^2: 17.6 -> 13.3
+// us per sweep against k_mc_quad, 64 x 256^2: 53 -> 49.
+__host__ __device__ inline bool mc_split_geom_ok(const Geom& g) { return g.ncolors == 2 && g.nx % 4 == 0; }
+template <typename T>
+inline bool mc_split_ok(const Geom& g, const FftPlan& px) {
+  return sizeof(T) == 4 && mc_split_geom_ok(g) && px.warp_a != 0;
+}
+constexpr int MCSP_THREADS = 128;
+template <bool ALLB, bool Z3>
+__global__ void __launch_bounds__(MCSP_THREADS, 6) k_mc_split(Geom g, const McCoef<float>* __restrict__ cp,
+                                                           float* __restrict__ m, const float* __restrict__ h,
+                                                           const SweepCounters* __restrict__ ctr, int color,
+                                                           int upt, FastDiv dunit, unsigned long long* acc) {
+  // the coefficients stay in shared memory and are read again for each trial:
+  // 26 registers less
+  __shared__ McCoef<float> c;
+  pdl_wait();
+  if (threadIdx.x < sizeof(c) / 4)
+    reinterpret_cast<uint32_t*>(&c)[threadIdx.x] = reinterpret_cast<const uint32_t*>(cp + blockIdx.z)[threadIdx.x];
+  const long long n = g.n;
+  m += blockIdx.z * 3 * n;
+  h += blockIdx.z * 3 * n;
+  acc += blockIdx.z;
+  const uint32_t stage = ctr->stage, sweep = ctr->sweep;
+  __syncthreads();
+  const bool dm = c.cd != 0.0f;
+  const int half = g.nx >> 1, upr = g.nx >> 2;  // cells of a colour, units of a row
+  const int total = upr * g.ny * g.nz, tstride = gridDim.x * MCSP_THREADS;
+  const int own0 = color ? half : 0, oth0 = color ? 0 : half;
+  unsigned int mine = 0;
+  int t = blockIdx.x * MCSP_THREADS + threadIdx.x;
+  for (int u = 0; u < upt; ++u, t += tstride) {
+    if (t >= total) break;
+    const int row = dunit.div(t), j0 = 2 * (t - row * upr);
+    int z = 0, y = row;
+    if constexpr (Z3) {
+      z = g.dny.div(row);
+      y = row - z * g.ny;
+    }
+    const int p = (color + y + z) & 1;
+    int yu = y + 1, yd = y - 1;
+    bool hu = true, hd = true;
+    if (yu >= g.ny) { if (g.per[1]) yu -= g.ny; else hu = false; }
+    if (yd < 0) { if (g.per[1]) yd += g.ny; else hd = false; }
+    if (g.ny == 1) hu = hd = false;
+    int zu = z + 1, zd = z - 1;
+    bool hzu = Z3, hzd = Z3;
+    if constexpr (Z3) {
+      if (zu >= g.nz) { if (g.per[2]) zu -= g.nz; else hzu = false; }
+      if (zd < 0) { if (g.per[2]) zd += g.nz; else hzd = false; }
+    }
+    int js = p ? j0 + 2 : j0 - 1;  // the side cell
+    bool hs = true;
+    if (js < 0) { if (g.per[0]) js += half; else hs = false; }
+    if (js >= half) { if (g.per[0]) js -= half; else hs = false; }
+    if constexpr (ALLB) hu = hd = hs = true;
+    const int rb = row * g.nx, ro = rb + own0 + j0, rt = rb + oth0;
+    const int ru = (z * g.ny + yu) * g.nx + oth0 + j0, rd = (z * g.ny + yd) * g.nx + oth0 + j0;
+    const int rzu = (zu * g.ny + y) * g.nx + oth0 + j0, rzd = (zd * g.ny + y) * g.nx + oth0 + j0;
+    float2 own[3], oth[3], up[3], dn[3], zup[3], zdn[3], hh[3];
+    float side[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float* base = m + k * n;
+      own[k] = *reinterpret_cast<const float2*>(base + ro);
+      oth[k] = *reinterpret_cast<const float2*>(base + rt + j0);
+      side[k] = hs ? base[rt + js] : 0.0f;
+      up[k] = hu ? *reinterpret_cast<const float2*>(base + ru) : own[k];
+      dn[k] = hd ? *reinterpret_cast<const float2*>(base + rd) : own[k];
+      if constexpr (Z3) {
+        zup[k] = hzu ? *reinterpret_cast<const float2*>(base + rzu) : own[k];
+        zdn[k] = hzd ? *reinterpret_cast<const float2*>(base + rzd) : own[k];
+      } else {
+        zup[k] = zdn[k] = own[k];
+      }
+      hh[k] = dm ? *reinterpret_cast<const float2*>(h + k * n + ro) : make_float2(0.0f, 0.0f);
+    }
+    bool changed = false;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      asm volatile("" ::: "memory");
+      Nbrs<float> nb;
+      // q = 0: (side, oth.x) or (oth.x, oth.y); q = 1: (oth.x, oth.y) or (oth.y, side)
+      nb.has[0][0] = q == 0 ? (p || hs) : true;
+      nb.has[0][1] = q == 1 ? (!p || hs) : true;
+      if constexpr (ALLB) nb.has[0][0] = nb.has[0][1] = true;
+      nb.has[1][0] = hd;
+      nb.has[1][1] = hu;
+      nb.has[2][0] = hzd;
+      nb.has[2][1] = hzu;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        nb.v[0][0][k] = q == 0 ? (p ? oth[k].x : side[k]) : (p ? oth[k].y : oth[k].x);
+        nb.v[0][1][k] = q == 0 ? (p ? oth[k].y : oth[k].x) : (p ? side[k] : oth[k].y);
+        nb.v[1][0][k] = q ? dn[k].y : dn[k].x;
+        nb.v[1][1][k] = q ? up[k].y : up[k].x;
+        nb.v[2][0][k] = q ? zdn[k].y : zdn[k].x;
+        nb.v[2][1][k] = q ? zup[k].y : zup[k].x;
+      }
+      const Proposal<float> pr = mc_propose<float>(c, (uint32_t)(rb + 2 * (j0 + q) + p), stage, sweep);
+      float& ox = q ? own[0].y : own[0].x;
+      float& oy = q ? own[1].y : own[1].x;
+      float& oz = q ? own[2].y : own[2].x;
+      if (mc_accept<float>(c, nb, ox, oy, oz, q ? hh[0].y : hh[0].x, q ? hh[1].y : hh[1].x, q ? hh[2].y : hh[2].x,
+                           pr, mc_sep<ALLB, Z3>(q, hzu))) {
+        pr.get(ox, oy, oz);
+        changed = true;
+        ++mine;
+      }
+    }
+    if (changed) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<float2*>(m + k * n + ro) = own[k];
+    }
+  }
+  unsigned int v = mine;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, (unsigned long long)v);
+}
+
+// Rows of `a` (nrows rows of nx values, components and replicas back to back;
+// row r has y + z = yz of lattice row r mod nyz) between the natural and the
+// colour-split order, in place: a CTA holds a row in shared memory in between.
+static __global__ void k_split_rows(float* __restrict__ a, int nx, FastDiv dnyz, FastDiv dny, int to_split) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* line = reinterpret_cast<float*>(smem_raw);
+  const int r = blockIdx.x, row = r - dnyz.div(r) * (int)dnyz.d, z = dny.div(row), yz = row - z * (int)dny.d + z;
+  float* p = a + (long long)r * nx;
+  for (int x = threadIdx.x; x < nx; x += blockDim.x) line[x] = p[x];
+  __syncthreads();
+  for (int x = threadIdx.x; x < nx; x += blockDim.x) {
+    const int q = split_pos(x, yz, nx);
+    if (to_split) p[q] = line[x];
+    else p[x] = line[q];
+  }
+}
+
 // One colour of a two-colour film sweep (the k_mc_quad film cases) with the rows
 // a CTA needs staged in shared memory first: the CTA owns a band of `band`
 // rows of one replica, copies m rows y0-1 .. y0+band (wrapped on a periodic
@@ -1519,11 +1854,6 @@ __global__ void __launch_bounds__(256) k_mc_quad(Geom g, const McCoef<T>* __rest
 // registers per thread than k_mc_quad, whose vector loads all sit in
 // registers at once, so more warps per SM hide the copies' latency.
 // Shared memory: (band + 2) x 3 rows of m and band x 3 rows of h.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename T>
 __host__ __device__ inline size_t mc_band_smem(const Geom& g, int band) {
@@ -2307,9 +2637,11 @@ __global__ void __launch_bounds__(256) k_energy(Geom g, const EnCoef* __restrict
 // far below what a swap decision resolves (kT ~ 1e-3 of these energies), at
 // a small fraction of its cost on a GPU with a low FP64 rate.  q[5..8] are 0.
 constexpr int ENL_CELLS = 8;
-static __global__ void __launch_bounds__(256) k_energy_lean(Geom g, const EnCoef* __restrict__ ep,
-                                                            const float* __restrict__ m, const float* __restrict__ h,
-                                                            double* __restrict__ partials) {
+// SPLIT: m and h in the colour-split order.
+template <bool SPLIT>
+__global__ void __launch_bounds__(256) k_energy_lean(Geom g, const EnCoef* __restrict__ ep,
+                                                     const float* __restrict__ m, const float* __restrict__ h,
+                                                     double* __restrict__ partials) {
   const EnCoef e = ep[blockIdx.z];
   const int n = (int)g.n;
   m += blockIdx.z * 3 * g.n;
@@ -2327,15 +2659,26 @@ static __global__ void __launch_bounds__(256) k_energy_lean(Geom g, const EnCoef
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int row = g.dnx.div(i), x = i - row * g.nx;
     const int z = g.dny.div(row), y = row - z * g.ny;
-    const float ax = mx[i], ay = my[i], az = mz[i];
+    const auto at = [&](long long j) -> int {  // where cell j is stored
+      if constexpr (!SPLIT) return (int)j;
+      const int r = g.dnx.div((int)j), zz = g.dny.div(r);
+      return r * g.nx + split_pos((int)j - r * g.nx, r - zz * g.ny + zz, g.nx);
+    };
+    const int is = at(i);
+    const float ax = mx[is], ay = my[is], az = mz[is];
     for (int a = 0; a < 3; ++a) {
-      const long long j = nbr_idx(g, x, y, z, a, 1);
+      long long j = nbr_idx(g, x, y, z, a, 1);
       if (j < 0) continue;
+      j = at(j);
       const float ddx = mx[j] - ax, ddy = my[j] - ay, ddz = mz[j] - az;
       acc[0] += aex[a] * (ddx * ddx + ddy * ddy + ddz * ddz);
     }
-    const long long xp = nbr_idx(g, x, y, z, 0, 1), xm = nbr_idx(g, x, y, z, 0, -1);
-    const long long yp = nbr_idx(g, x, y, z, 1, 1), ym = nbr_idx(g, x, y, z, 1, -1);
+    long long xp = nbr_idx(g, x, y, z, 0, 1), xm = nbr_idx(g, x, y, z, 0, -1);
+    long long yp = nbr_idx(g, x, y, z, 1, 1), ym = nbr_idx(g, x, y, z, 1, -1);
+    xp = xp < 0 ? xp : at(xp);
+    xm = xm < 0 ? xm : at(xm);
+    yp = yp < 0 ? yp : at(yp);
+    ym = ym < 0 ? ym : at(ym);
     const float dxmz = (xp >= 0 ? mz[xp] : 0.f) - (xm >= 0 ? mz[xm] : 0.f);
     const float dxmx = (xp >= 0 ? mx[xp] : 0.f) - (xm >= 0 ? mx[xm] : 0.f);
     const float dymz = (yp >= 0 ? mz[yp] : 0.f) - (ym >= 0 ? mz[ym] : 0.f);
@@ -2344,7 +2687,7 @@ static __global__ void __launch_bounds__(256) k_energy_lean(Geom g, const EnCoef
     const float mu = ax * u0 + ay * u1 + az * u2;
     acc[2] -= kuv * mu * mu;
     acc[3] -= ax * b0 + ay * b1 + az * b2;
-    if (h) acc[4] -= dmg * (ax * h[i] + ay * h[n + i] + az * h[2 * n + i]);
+    if (h) acc[4] -= dmg * (ax * h[is] + ay * h[n + is] + az * h[2 * n + is]);
   }
   double q[NQ];
 #pragma unroll
@@ -2509,12 +2852,17 @@ struct XPassW {
   void (*inv)(FftPlan, const C<T>*, long long, int, int, int, FastDiv, FastDiv, int, T*, long long, int, long long,
               long long);
 };
-template <typename T>
+template <typename T, bool SPLIT = false>
 XPassW<T> x_pass_w(const FftPlan& p) {
   if constexpr (__is_same(T, double)) return {nullptr, nullptr};  // lines64.cuh
   else {
 #define MMC_XW(A_, B_) \
-  if (p.warp_a == A_ && p.warp_b == B_) return {k_x_forward_w<T, A_, B_>, k_x_inverse_w<T, A_, B_>};
+  if (p.warp_a == A_ && p.warp_b == B_) {                                                    \
+    if constexpr (sizeof(T) == 4)                                                           \
+      return {k_x_forward_r<A_, B_, SPLIT>, k_x_inverse_r<A_, B_, SPLIT>};                  \
+    else                                                                                    \
+      return {k_x_forward_w<T, A_, B_>, k_x_inverse_w<T, A_, B_>};                          \
+  }
   MMC_XW(32, 32)
   MMC_XW(32, 16)
   MMC_XW(16, 16)
@@ -2526,8 +2874,10 @@ XPassW<T> x_pass_w(const FftPlan& p) {
   return {nullptr, nullptr};
   }
 }
-inline size_t x_pass_w_smem(const FftPlan& p, int rows, size_t csize) {
-  return ((size_t)p.n + 2 * (size_t)rows * (p.n + p.warp_a)) * csize;
+inline size_t x_pass_w_smem(const FftPlan& p, int rows, int threads, size_t csize) {
+  // a line's room per row and pair, or (FP32) per line in flight
+  const size_t lines = csize == 8 ? (size_t)(threads / p.warp_b) : 2 * (size_t)rows;
+  return ((size_t)p.n + lines * (p.n + p.warp_a)) * csize;
 }
 
 // Raises the dynamic shared-memory limit of the FFT pass kernels to the
@@ -2553,15 +2903,22 @@ cudaError_t prepare_passes(int max_dyn_smem) {
       const XPassW<T> w = x_pass_w<T>(p);
       MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
       MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)w.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+      if constexpr (sizeof(T) == 4) {
+        const XPassW<T> ws = x_pass_w<T, true>(p);
+        MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)ws.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+        MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)ws.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+      }
     }
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)col_reg_smem<T, 16>()));
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)col_reg_smem<T, 8>()));
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)col_reg_smem<T, 16>()));
-    MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_reg3<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)col_reg_smem<T, 8>()));
+    if constexpr (sizeof(T) == 4) {
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_pipe<16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)col_pipe_smem<16, 16>()));
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_pipe<16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)col_pipe_smem<16, 8>()));
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_pipe<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)col_pipe_smem<8, 8>()));
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_col_pipe<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)col_pipe_smem<8, 4>()));
+    }
     return cudaSuccess;
   }
 }
@@ -2591,12 +2948,15 @@ template <typename T>
 cudaError_t run_x_forward(const FftPlan& p, int ncomp, int xdata, int ydata, int nrows, const T* in,
                           long long in_cstride, C<T>* S, long long nspec, int nyp, int hx, int pitch, int rpc,
                           int threads, cudaStream_t st, int nrep = 1, long long in_rstride = 0,
-                          long long s_rstride = 0, bool inl = false) {
+                          long long s_rstride = 0, bool inl = false, bool split = false) {
   if (ncomp == 3) {
-    const XPassW<T> w = x_pass_w<T>(p);
+    XPassW<T> w = x_pass_w<T>(p);
+    if constexpr (sizeof(T) == 4) {
+      if (split) w = x_pass_w<T, true>(p);
+    }
     if (w.fwd) {
       dim3 grid((nrows + rpc - 1) / rpc, 1, nrep);
-      return launch_pdl(w.fwd, grid, dim3(threads), x_pass_w_smem(p, rpc, sizeof(C<T>)), st, p, xdata,
+      return launch_pdl(w.fwd, grid, dim3(threads), x_pass_w_smem(p, rpc, threads, sizeof(C<T>)), st, p, xdata,
                         FastDiv((uint32_t)ydata), nrows, in, in_cstride, S, nspec, nyp, hx, pitch, rpc, in_rstride,
                         s_rstride);
     }
@@ -2615,9 +2975,8 @@ cudaError_t run_x_forward(const FftPlan& p, int ncomp, int xdata, int ydata, int
   return cudaGetLastError();
 }
 
-// The film column pass held in registers for a launch shape: 0 none, 1
-// k_col_reg (col_lean 2), 2 k_col_reg3 (col_lean 3).
-inline int col_regs(const DemagTuning& tun) { return tun.col_lean >= 2 ? tun.col_lean - 1 : 0; }
+// Whether a launch shape takes the pipelined film column pass (col_lean 2 or 3).
+inline int col_regs(const DemagTuning& tun) { return tun.col_lean >= 2 ? 1 : 0; }
 template <typename T>
 cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, const C<T>* khat, int hx,
                          int planes, long long plane_stride, long long pos_stride, int load_lim, int store_lim,
@@ -2640,22 +2999,11 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
                         inv_n, s_rstride);
     }
   }
-  if constexpr (!__is_same(T, double))
-  if (regs && ncomp == 3 && planes == 1 && (flags & ~PASS_SYM) == (PASS_FWD | PASS_MUL | PASS_INV) &&
-      pos_stride < (1LL << 31) && p.warp_a == p.warp_b && (p.warp_a == 16 || p.warp_a == 8)) {
-    dim3 grid((hx + CR_TX - 1) / CR_TX, 1, nrep);
-    if (regs == 2) {  // one component per thread
-      if (p.warp_a == 16)
-        return launch_pdl(k_col_reg3<T, 16>, grid, dim3(3 * CR_TX * 16), col_reg_smem<T, 16>(), st, p, S, nspec,
-                          khat, hx, (int)pos_stride, load_lim, store_lim, flags, inv_n, s_rstride);
-      return launch_pdl(k_col_reg3<T, 8>, grid, dim3(3 * CR_TX * 8), col_reg_smem<T, 8>(), st, p, S, nspec, khat,
-                        hx, (int)pos_stride, load_lim, store_lim, flags, inv_n, s_rstride);
-    }
-    if (p.warp_a == 16)
-      return launch_pdl(k_col_reg<T, 16>, grid, dim3(CR_TX * 16), col_reg_smem<T, 16>(), st, p, S, nspec, khat, hx,
-                        (int)pos_stride, load_lim, store_lim, flags, inv_n, s_rstride);
-    return launch_pdl(k_col_reg<T, 8>, grid, dim3(CR_TX * 8), col_reg_smem<T, 8>(), st, p, S, nspec, khat, hx,
-                      (int)pos_stride, load_lim, store_lim, flags, inv_n, s_rstride);
+  if constexpr (sizeof(T) == 4) {
+    if (regs && ncomp == 3 && planes == 1 && (flags & ~PASS_SYM) == (PASS_FWD | PASS_MUL | PASS_INV) &&
+        pos_stride < (1LL << 31) && (nrep == 1 || s_rstride == 3 * nspec) && col_pipe_ok(p))
+      return launch_col_pipe(p, S, nspec, khat, hx, (int)pos_stride, load_lim, store_lim, (flags & PASS_SYM) ? 1 : 0,
+                             inv_n, nrep, st);
   }
   if (tx < 1 || (tx & (tx - 1)) != 0 || threads % tx != 0) return cudaErrorInvalidValue;  // see k_col_pass
   // in-place transforms exist for the warp path only
@@ -2698,7 +3046,7 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
 template <typename T>
 cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
                        const DemagTuning& tun, const T* m, T* h, void* spec, const void* khat, cudaStream_t st,
-                       int nrep, cudaEvent_t* ev, int mul_flags = 0) {
+                       int nrep, cudaEvent_t* ev, int mul_flags = 0, bool split = false) {
   C<T>* S = reinterpret_cast<C<T>*>(spec);
   const C<T>* K = reinterpret_cast<const C<T>*>(khat);
   const long long ns = g.nspec;
@@ -2719,7 +3067,7 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   }
   if (!x64)
     MMC_TRY(run_x_forward<T>(px, 3, g.nx, g.ny, rows, m, g.n, S, ns, g.nyp, g.hx, g.hxp, tun.x_rows_per_cta,
-                           tun.x_threads, st, nrep, mr, sr, tun.fft_inline != 0));
+                           tun.x_threads, st, nrep, mr, sr, tun.fft_inline != 0, split));
   if (ev) MMC_TRY(cudaEventRecord(ev[1], st));
   const long long ystride = g.hxp, yplane = (long long)g.nyp * g.hxp;
   if (g.nzp == 1) {
@@ -2738,7 +3086,10 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   if (ev) MMC_TRY(cudaEventRecord(ev[2], st));
   const int rpc = tun.x_rows_per_cta;
   dim3 grid((rows + rpc - 1) / rpc, 1, nrep);
-  const XPassW<T> w = x_pass_w<T>(px);
+  XPassW<T> w = x_pass_w<T>(px);
+  if constexpr (sizeof(T) == 4) {
+    if (split) w = x_pass_w<T, true>(px);
+  }
   if (x64) {
     if constexpr (__is_same(T, double)) {
       L64Fns f;
@@ -2747,7 +3098,7 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
                          (const double2*)S, ns, g.nyp, g.hxp, g.nx, g.dny, rows, h, g.n, sr, mr));
     }
   } else if (w.inv) {
-    MMC_TRY(launch_pdl(w.inv, grid, dim3(tun.x_threads), x_pass_w_smem(px, rpc, sizeof(C<T>)), st, px,
+    MMC_TRY(launch_pdl(w.inv, grid, dim3(tun.x_threads), x_pass_w_smem(px, rpc, tun.x_threads, sizeof(C<T>)), st, px,
                        (const C<T>*)S, ns, g.nyp, g.hx, g.hxp, g.dnx, g.dny, rows, h, g.n, rpc, sr, mr));
   } else {
     if (px.warp_a == 32) return cudaErrorInvalidValue;  // the wide shapes have warp-shaped x passes
@@ -2815,6 +3166,19 @@ cudaError_t mc_impl(const Geom& g, const McCoef<T>* c, T* m, const T* h, const S
         g, c, m, h, ctr, color, band, FastDiv((uint32_t)(g.nx * sizeof(T) / 16)), FastDiv((uint32_t)(g.nx / 4)), acc);
     return cudaGetLastError();
   }
+  if (form == MC_FORM_SPLIT) {
+    if constexpr (sizeof(T) == 4) {
+      if (!mc_split_geom_ok(g)) return cudaErrorInvalidValue;
+      const long long total = (long long)g.ny * g.nz * (g.nx >> 2);
+      const int upt = 2;  // units per thread (1: 28.6 us at 64 x 256^2 instead of 24.3)
+      dim3 grid((unsigned)((total + upt * MCSP_THREADS - 1) / (upt * MCSP_THREADS)), 1, nrep);
+      auto kern = g.nz > 1 ? (mc_all_bonds(g) ? k_mc_split<true, true> : k_mc_split<false, true>)
+                           : (mc_all_bonds(g) ? k_mc_split<true, false> : k_mc_split<false, false>);
+      return launch_pdl(kern, grid, dim3(MCSP_THREADS), 0, st, g, c, m, h, ctr, color, upt,
+                        FastDiv((uint32_t)(g.nx >> 2)), acc);
+    }
+    return cudaErrorInvalidValue;
+  }
   if (form == MC_FORM_QUAD && mc_quad_ok(g)) {
     // 128-thread CTAs: the same warps per SM as 256 (the registers limit
     // them), in finer pieces, measured 2 us faster per batched sweep
@@ -2860,11 +3224,11 @@ cudaError_t energy_impl(const Geom& g, const EnCoef* e, const T* m, const T* h, 
 // with_q < 0: the energies for tempering swaps (k_energy_lean for FP32 replicas).
 template <typename T>
 cudaError_t energy_swap_impl(const Geom& g, const EnCoef* e, const T* m, const T* h, double* partials,
-                             int npartials, double* out, cudaStream_t st, int nrep) {
+                             int npartials, double* out, cudaStream_t st, int nrep, bool split) {
   if constexpr (sizeof(T) == 4) {
     const int nb = std::max(1, energy_blocks(g) / ENL_CELLS);
     if (nb > npartials || g.n >= (1LL << 31)) return cudaErrorInvalidValue;
-    k_energy_lean<<<dim3(nb, 1, nrep), 256, 0, st>>>(g, e, m, h, partials);
+    (split ? k_energy_lean<true> : k_energy_lean<false>)<<<dim3(nb, 1, nrep), 256, 0, st>>>(g, e, m, h, partials);
     MMC_TRY(cudaGetLastError());
     k_reduce_partials<<<nrep, 256, 0, st>>>(partials, nb, out);
     return cudaGetLastError();
@@ -2892,8 +3256,9 @@ cudaError_t init_impl(const Geom& g, uint64_t seed, T* m, cudaStream_t st) {
 template <typename T>
 cudaError_t launch_demag(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
                          const DemagTuning& tun, const T* m, T* h, void* spec, const void* khat, cudaStream_t st,
-                         int nrep, cudaEvent_t* ev) {
-  return demag_impl<T>(g, px, py, pz, tun, m, h, spec, khat, st, nrep, ev);
+                         int nrep, cudaEvent_t* ev, bool split) {
+  if (split && !mc_split_ok<T>(g, px)) return cudaErrorInvalidValue;
+  return demag_impl<T>(g, px, py, pz, tun, m, h, spec, khat, st, nrep, ev, 0, split);
 }
 template <typename T>
 cudaError_t launch_demag_sym(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
@@ -2917,8 +3282,9 @@ cudaError_t launch_mc_strip(const Geom& g, const McCoef<T>* c, const T* m_in, T*
 }
 template <typename T>
 cudaError_t launch_energy(const Geom& g, const EnCoef* e, const T* m, const T* h, double* partials, int npartials,
-                          double* out, cudaStream_t st, int nrep, int with_q) {
-  if (with_q < 0) return energy_swap_impl<T>(g, e, m, h, partials, npartials, out, st, nrep);
+                          double* out, cudaStream_t st, int nrep, int with_q, bool split) {
+  if (with_q < 0) return energy_swap_impl<T>(g, e, m, h, partials, npartials, out, st, nrep, split);
+  if (split) return cudaErrorInvalidValue;
   return energy_impl<T>(g, e, m, h, partials, npartials, out, st, nrep, with_q);
 }
 template <typename T>
@@ -2965,7 +3331,7 @@ cudaError_t launch_khat_store(long long count, const double2* spec64, void* khat
 #define MMC_INSTANTIATE_LAUNCHERS(T)                                                                          \
   template cudaError_t launch_demag<T>(const Geom&, const FftPlan&, const FftPlan&, const FftPlan&,           \
                                        const DemagTuning&, const T*, T*, void*, const void*, cudaStream_t, int, \
-                                       cudaEvent_t*);                                                          \
+                                       cudaEvent_t*, bool);                                                    \
   template cudaError_t launch_demag_sym<T>(const Geom&, const FftPlan&, const FftPlan&, const FftPlan&,       \
                                            const DemagTuning&, const T*, T*, void*, const void*, cudaStream_t); \
   template cudaError_t launch_mc<T>(const Geom&, const McCoef<T>*, T*, const T*, const SweepCounters*, int,   \
@@ -2973,7 +3339,7 @@ cudaError_t launch_khat_store(long long count, const double2* spec64, void* khat
   template cudaError_t launch_mc_strip<T>(const Geom&, const McCoef<T>*, const T*, T*, const T*,             \
                                           const SweepCounters*, unsigned long long*, cudaStream_t, int);       \
   template cudaError_t launch_energy<T>(const Geom&, const EnCoef*, const T*, const T*, double*, int, double*, \
-                                        cudaStream_t, int, int);                                               \
+                                        cudaStream_t, int, int, bool);                                         \
   template cudaError_t launch_field<T>(const Geom&, const HCoef&, int, const T*, const T*, double*,            \
                                        cudaStream_t);                                                          \
   template cudaError_t launch_init<T>(const Geom&, uint64_t, T*, cudaStream_t);                               \

@@ -51,6 +51,8 @@ struct FftPlan {
   // roots exp(-2 pi i j / n) at full_off.
   int warp_a, warp_b;
   int full_off;
+  int lane_off;  // the roots in the order the lanes of a line take them: [ka][b] = root b ka, ka < A, b < B
+                 // (behind tw_total: only the FP32 x passes load it)
   FastDiv dn;  // n
   FastDiv dnb[FFT_MAX_STAGES];  // n / radix[s]
   FastDiv dns[FFT_MAX_STAGES];  // ns[s]
@@ -63,8 +65,8 @@ struct FftPlan {
 // periodic n); the transform grid (nxp, nyp, nzp) equals it except that an
 // open axis of 2n - 1 > 16 is padded further to the next power of two up to
 // 1024, where the warp-level transforms apply.  The spectrum keeps the
-// kx half-axis: hx = nxp/2 + 1 columns stored with an even row pitch hxp (so
-// that pairs of FP32 columns are 16-byte aligned), layout [comp][kz][ky][kx],
+// kx half-axis: hx = nxp/2 + 1 columns stored with a row pitch hxp of whole
+// 32-byte sectors (even at least, so that pairs of FP32 columns are 16-byte aligned), layout [comp][kz][ky][kx],
 // nspec = hxp*nyp*nzp.  Pad columns hold zeros.
 struct Geom {
   int nx, ny, nz;
@@ -154,9 +156,8 @@ struct DemagTuning {
   int col_threads;
   int mc_form;     // MC_FORM_*
   int fft_inline;  // 1: the pass kernels expand the warp-level transforms in line
-  int col_lean;    // 1: column passes transform in place and read K^ from global memory; 2: as 1, and
-                   // film y passes of length 64 or 256 hold their lines in registers (k_col_reg); 3: as 2,
-                   // one component per thread (k_col_reg3)
+  int col_lean;    // 1: column passes transform in place and read K^ from global memory; 2 and 3: as 1, and FP32
+                   // film y passes of length 32 to 256 are the pipelined ones (k_col_pipe)
 };
 
 // Device counters read by the sweep kernels: [stage, sweep].
@@ -173,7 +174,8 @@ struct SweepCounters {
 template <typename T>
 cudaError_t launch_demag(const Geom& g, const FftPlan& px, const FftPlan& py, const FftPlan& pz,
                          const DemagTuning& tun, const T* m, T* h, void* spec, const void* khat,
-                         cudaStream_t st, int nrep = 1, cudaEvent_t* ev = nullptr);
+                         cudaStream_t st, int nrep = 1, cudaEvent_t* ev = nullptr, bool split = false);
+// (split: m and h in the colour-split order, see MC_FORM_SPLIT.)
 // Metropolis kernel forms (all make the same decisions): one scalar launch
 // per colour; both colours of a film in one tile launch; one vectorised launch
 // per colour for films with nx a multiple of 4.
@@ -190,8 +192,19 @@ enum : int {
   MC_FORM_QUAD = 2,
   MC_FORM_BAND = 3,
   MC_FORM_STRIP = 4,
-  MC_FORM_PIPE = 5
+  MC_FORM_PIPE = 5,
+  // what the vectorised form becomes in FP32 runs of MC_SPLIT_SWEEPS sweeps or
+  // more: m and h rows stored colour by colour (k_mc_split); not a launch shape
+  // of its own
+  MC_FORM_SPLIT = 6
 };
+constexpr int MC_SPLIT_SWEEPS = 16;
+// Whether a lattice's FP32 sweeps can run on the split order, and the
+// conversion of `count` fields of 3 n values in place.
+bool mc_split_eligible(const Geom& g, const FftPlan& px);
+// Whether an FP32 film's y pass can be the pipelined one.
+bool col_pipe_eligible(const FftPlan& py);
+cudaError_t launch_split_rows(const Geom& g, float* a, int count, bool to_split, cudaStream_t st);
 // color < 0: every colour of the sweep in the given form (falls back to the
 // scalar form where the lattice does not qualify).
 template <typename T>
@@ -219,7 +232,8 @@ template <typename T>
 // energies for tempering swaps (FP32 per cell, FP64 sums, for FP32 replicas;
 // as 0 for FP64 ones).
 cudaError_t launch_energy(const Geom& g, const EnCoef* e, const T* m, const T* h, double* partials,
-                          int npartials, double* out, cudaStream_t st, int nrep = 1, int with_q = 1);
+                          int npartials, double* out, cudaStream_t st, int nrep = 1, int with_q = 1,
+                          bool split = false);
 template <typename T>
 cudaError_t launch_field(const Geom& g, const HCoef& c, int term, const T* m, const T* h, double* out,
                          cudaStream_t st);

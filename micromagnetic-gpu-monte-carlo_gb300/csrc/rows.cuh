@@ -58,7 +58,7 @@ __host__ __device__ inline size_t row_phase_bytes(const Geom& g, const FftPlan& 
   auto a16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
   size_t b = a16((size_t)px.tw_total * cs);
   b += a16((size_t)(band + 4) * 3 * g.nx * sizeof(T));
-  b += a16((size_t)(band + 2) * 3 * g.hxp * cs);
+  b += a16((size_t)(band + 2) * 3 * (g.hx + (g.hx & 1)) * cs);
   b += a16((size_t)(band + 2) * 3 * g.nx * sizeof(T));
   b += a16((size_t)(2 * band + 2) * ((g.nx + 1) / 2) * 4 * sizeof(T));
   size_t fl = (size_t)2 * (band + 2) * px.n;
@@ -78,7 +78,7 @@ __device__ __forceinline__ void row_phase_carve(RowPhase<T>& R, unsigned char*& 
   R.msm = reinterpret_cast<T*>(ptr);
   ptr += a16((size_t)(band + 4) * 3 * R.g.nx * sizeof(T));
   R.specraw = reinterpret_cast<C<T>*>(ptr);
-  ptr += a16((size_t)(band + 2) * 3 * R.g.hxp * cs);
+  ptr += a16((size_t)(band + 2) * 3 * (R.g.hx + (R.g.hx & 1)) * cs);
   R.hsm = reinterpret_cast<T*>(ptr);
   ptr += a16((size_t)(band + 2) * 3 * R.g.nx * sizeof(T));
   R.prop = reinterpret_cast<Proposal<T>*>(ptr);
@@ -116,12 +116,12 @@ template <typename T>
 __device__ __forceinline__ void row_load(const RowPhase<T>& R, const McCoef<T>& c, uint32_t stage, uint32_t sweep,
                                          bool with_proposals = true) {
   using V = C<T>;
-  const int nx = R.g.nx, hxp = R.g.hxp;
+  const int nx = R.g.nx, hxp = R.g.hxp, hxs = R.g.hx + (R.g.hx & 1);  // hxs: the rows' pitch in shared memory
   const long long n = R.g.n, nspec = R.g.nspec;
   const int nslots = R.nb + 4, nwork = R.nb + 2;
   const size_t mstride = 3 * (size_t)nx;
   const int elems = 16 / (int)sizeof(T), per_m = nx / elems;
-  const int ve = 16 / (int)sizeof(V), per_s = hxp / ve;
+  const int ve = 16 / (int)sizeof(V), per_s = hxs / ve;
   const FastDiv d3m((uint32_t)(3 * per_m)), dm((uint32_t)per_m), d3s((uint32_t)(3 * per_s)), ds((uint32_t)per_s);
   for (int idx = threadIdx.x; idx < nslots * 3 * per_m; idx += blockDim.x) {
     const int slot = d3m.div(idx), rem = idx - slot * 3 * per_m;
@@ -135,7 +135,7 @@ __device__ __forceinline__ void row_load(const RowPhase<T>& R, const McCoef<T>& 
     const int r = R.rows[w + 1];
     if (r < 0) continue;
     const int cc = ds.div(rem), q = rem - cc * per_s;
-    cp_async16(R.specraw + ((size_t)w * 3 + cc) * hxp + q * ve, R.S + cc * nspec + (long long)r * hxp + q * ve);
+    cp_async16(R.specraw + ((size_t)w * 3 + cc) * hxs + q * ve, R.S + cc * nspec + (long long)r * hxp + q * ve);
   }
   if (with_proposals) row_proposals<T>(R, c, stage, sweep);
   cp_async_wait_all();
@@ -146,7 +146,7 @@ __device__ __forceinline__ void row_load(const RowPhase<T>& R, const McCoef<T>& 
 template <typename T>
 __device__ __forceinline__ void row_field(const RowPhase<T>& R) {
   using V = C<T>;
-  const int nx = R.g.nx, hx = R.g.hx, hxp = R.g.hxp, L = R.px->n;
+  const int nx = R.g.nx, hx = R.g.hx, hxp = R.g.hx + (R.g.hx & 1), L = R.px->n;
   const int nwork = R.nb + 2;
   const size_t mstride = 3 * (size_t)nx;
   for (int idx = threadIdx.x; idx < nwork * L; idx += blockDim.x) {

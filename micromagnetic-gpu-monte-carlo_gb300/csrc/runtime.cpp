@@ -174,6 +174,14 @@ int make_plan(int n, PlanHost* ph) {
     }
   }
   p.tw_total = (int)(tw.size() / 2);
+  p.lane_off = p.tw_total;
+  for (int ka = 0; ka < p.warp_a; ++ka)
+    for (int b = 0; b < p.warp_b; ++b) {
+      double c, sn;
+      unit_root((long long)b * ka, n, &c, &sn);
+      tw.push_back(c);
+      tw.push_back(sn);
+    }
   size_t cnt = tw.size() / 2;
   if (cnt == 0) cnt = 1, tw.push_back(1.0), tw.push_back(0.0);
   std::vector<float> tw32(tw.size());
@@ -243,13 +251,18 @@ DemagTuning choose_tuning(const Geom& g, const FftPlan& px, const FftPlan& py, c
   } else {
     r = 4;
   }
-  while (r > 1 && ((rows + r - 1) / r) * nrep < want) r /= 2;
+  // (FP32 warp-shaped passes: a CTA's warps work on their own, and full CTAs are
+  // as fast as single rows on one 64^2 film, faster from 32 of them on)
+  while (r > 1 && !(csize == 8 && px.warp_a) && ((rows + r - 1) / r) * nrep < want) r /= 2;
   while (r > 1 && xsm(r) > 96 * 1024) r /= 2;
   t.x_rows_per_cta = r;
   // in-place column passes reading K^ from global memory for the long
   // warp-shaped lines, where the copies of the tile and of K^ would leave room
   // for one column per CTA (the autotuner tries both forms)
   t.col_lean = py.warp_a != 0 && py.n >= 512 ? 1 : 0;
+  // FP32 films: the pipelined pass, the fastest one from a single 64^2 film
+  // (9.7 us per sweep, 12.1 in place, 13.2 with copies) to 64 x 256^2
+  if (csize == 8 && g.nzp == 1 && col_pipe_eligible(py)) t.col_lean = 2;
   // shared memory of a column pass: the in-place form holds the tile once,
   // the other twice plus the K^ tile when the pass multiplies
   auto csm = [&](const FftPlan& p, int tx, bool mul) {
@@ -271,8 +284,9 @@ DemagTuning choose_tuning(const Geom& g, const FftPlan& px, const FftPlan& py, c
   t.col_tx_z = pick(pz, g.nyp, true);
   t.col_threads = col_threads_for(g, py, pz, t.col_tx, t.col_tx_z);
   // FP32 with at least 8 x 256^2 trials per launch (batches of 8 films, a
-  // 512x512x8 slab): the vectorised per-colour sweep, measured faster there;
-  // smaller lattices and FP64 keep the scalar form (the autotuner tries every
+  // 512x512x8 slab): the vectorised per-colour sweep, measured faster there
+  // (16 x 128^2: 18.8 us per sweep and 21.0 with the scalar form; 2 x 256^2: 17.0
+  // and 16.6); smaller lattices keep the scalar form (the autotuner tries every
   // form)
   t.mc_form = csize == 8 && (long long)nrep * g.n >= 8LL * 65536 && mc_quad_eligible(g) ? MC_FORM_QUAD
                                                                                       : MC_FORM_SCALAR;
@@ -282,6 +296,11 @@ DemagTuning choose_tuning(const Geom& g, const FftPlan& px, const FftPlan& py, c
 
 
 }  // namespace
+
+// Sweep counters in device memory: slot q holds (stage, sweep + q); sweep q of a
+// run reads slot q mod CTR_SLOTS, and one launch advances them all after
+// CTR_SLOTS sweeps and after the last one.
+constexpr int CTR_SLOTS = 32;
 
 // =================================================================== handle
 struct mmc_handle {
@@ -305,7 +324,8 @@ struct mmc_handle {
   double* red = nullptr;     // NQ doubles, device
   double* red_host = nullptr;  // NQ doubles, pinned
   unsigned long long* acc = nullptr;
-  SweepCounters* ctr = nullptr;
+  SweepCounters* ctr = nullptr;  // CTR_SLOTS
+  SweepCounters ctr_host[CTR_SLOTS];
   double* stage64 = nullptr;  // 3n doubles, device (host <-> device staging)
   double* field64 = nullptr;  // 3n doubles, device
   bool demag_built = false;
@@ -317,6 +337,7 @@ struct mmc_handle {
   // graph of `graph_sweeps` sweeps
   cudaGraphExec_t gexec = nullptr;
   int graph_sweeps = 0;
+  bool graph_split = false;
   long long seed = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   double last_run_ms = 0;
@@ -328,6 +349,7 @@ struct mmc_handle {
   void* hsym = nullptr;      // 3n T, symmetrised demag field of the gradient (allocated on first use)
   double* relax_p = nullptr;  // 3n doubles, relaxation direction
   double* relax_s = nullptr;  // 3n doubles, last relaxation step
+  bool split = false;     // m and h are in the colour-split order (inside a run only)
   void* m2 = nullptr;     // film engine: second copy of m (3n T)
   void* spec2 = nullptr;  // film engine: second spectrum (3*nspec complex T)
   int nsm = 0;
@@ -432,41 +454,61 @@ HCoef make_h_coef(const mmc_handle* h) {
 cudaError_t demag(mmc_handle* h) {
   if (h->prec == 32)
     return launch_demag<float>(h->g, h->px.p, h->py.p, h->pz.p, h->tun, (const float*)h->m, (float*)h->h, h->spec,
-                               h->khat, h->st);
+                               h->khat, h->st, 1, nullptr, h->split);
   return launch_demag<double>(h->g, h->px.p, h->py.p, h->pz.p, h->tun, (const double*)h->m, (double*)h->h, h->spec,
                               h->khat, h->st);
 }
 
-cudaError_t mc_color(mmc_handle* h, int color) {
+cudaError_t mc_color(mmc_handle* h, int color, int slot = 0) {
   if (h->prec == 32)
-    return launch_mc<float>(h->g, (const McCoef<float>*)h->coef, (float*)h->m, (const float*)h->h, h->ctr, color,
-                            h->acc, h->st, 1, h->tun.mc_form);
-  return launch_mc<double>(h->g, (const McCoef<double>*)h->coef, (double*)h->m, (const double*)h->h, h->ctr, color,
+    return launch_mc<float>(h->g, (const McCoef<float>*)h->coef, (float*)h->m, (const float*)h->h, h->ctr + slot, color,
+                            h->acc, h->st, 1, h->split ? MC_FORM_SPLIT : h->tun.mc_form);
+  return launch_mc<double>(h->g, (const McCoef<double>*)h->coef, (double*)h->m, (const double*)h->h, h->ctr + slot, color,
                            h->acc, h->st, 1, h->tun.mc_form);
 }
 
-// Enqueues one full sweep: demag refresh, every colour, counter advance.
-cudaError_t enqueue_sweep(mmc_handle* h) {
-  cudaError_t e;
-  if (h->cfg.cal_demag_flag) {
-    e = demag(h);
-    if (e != cudaSuccess) return e;
+// Sets the counter slots to (stage, sweep0 + q).
+cudaError_t set_counters(mmc_handle* h, long long stage, long long sweep0) {
+  for (int q = 0; q < CTR_SLOTS; ++q) h->ctr_host[q] = SweepCounters{(uint32_t)stage, (uint32_t)(sweep0 + q)};
+  return cudaMemcpyAsync(h->ctr, h->ctr_host, sizeof h->ctr_host, cudaMemcpyHostToDevice, h->st);
+}
+
+// Enqueues k full sweeps: demag refresh, every colour; the counters advance
+// after every CTR_SLOTS sweeps and after the last one.
+cudaError_t enqueue_sweeps(mmc_handle* h, long long k) {
+  cudaError_t e = cudaSuccess;
+  for (long long q = 0; q < k && e == cudaSuccess; ++q) {
+    const int slot = (int)(q % CTR_SLOTS);
+    if (h->cfg.cal_demag_flag) e = demag(h);
+    if (e == cudaSuccess) e = mc_color(h, -1, slot);
+    if (e == cudaSuccess && (slot == CTR_SLOTS - 1 || q == k - 1))
+      e = launch_advance(h->ctr, (uint32_t)(slot + 1), h->st, CTR_SLOTS);
   }
-  e = mc_color(h, -1);
-  if (e != cudaSuccess) return e;
-  return launch_advance(h->ctr, 1, h->st);
+  return e;
+}
+
+// The order of m and h on the device for a run of `nsweeps` sweeps, and back.
+bool handle_split(const mmc_handle* h, long long nsweeps) {
+  return h->prec == 32 && h->tun.mc_form == MC_FORM_QUAD && nsweeps >= MC_SPLIT_SWEEPS && h->cfg.cal_demag_flag &&
+         mc_split_eligible(h->g, h->px.p);
+}
+cudaError_t set_split(mmc_handle* h, bool split) {
+  if (h->split == split) return cudaSuccess;
+  cudaError_t e = launch_split_rows(h->g, (float*)h->m, 1, split, h->st);
+  if (e == cudaSuccess) e = launch_split_rows(h->g, (float*)h->h, 1, split, h->st);
+  if (e == cudaSuccess) h->split = split;
+  return e;
 }
 
 int ensure_graph(mmc_handle* h, int nsw) {
-  if (h->gexec && h->graph_sweeps == nsw) return MMC_OK;
+  if (h->gexec && h->graph_sweeps == nsw && h->graph_split == h->split) return MMC_OK;
   if (h->gexec) {
     cudaGraphExecDestroy(h->gexec);
     h->gexec = nullptr;
   }
   cudaGraph_t graph;
   CU(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaSuccess;
-  for (int s = 0; s < nsw && e == cudaSuccess; ++s) e = enqueue_sweep(h);
+  cudaError_t e = enqueue_sweeps(h, nsw);
   cudaError_t e2 = cudaStreamEndCapture(h->st, &graph);
   if (e != cudaSuccess || e2 != cudaSuccess) cudaGetLastError();  // do not leak the capture error to later calls
   if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("sweep capture: ") + cudaGetErrorString(e));
@@ -475,6 +517,7 @@ int ensure_graph(mmc_handle* h, int nsw) {
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
   h->graph_sweeps = nsw;
+  h->graph_split = h->split;
   return MMC_OK;
 }
 
@@ -553,8 +596,12 @@ int setup_engine(mmc_handle* h, int nsm) {
   // the operations (lines64.cuh).  us per sweep, pass kernels / film engine: 32^2
   // 20 / 32, 64^2 22 / 36, 128^2 27 / 70; without a power-of-two transform 24^2
   // 37 / 28, 48^2 39 / 32, 96^2 43 / 46, 192^2 56 / 85.
-  const bool f64_kernels = h->prec == 64 && ((h->px.p.warp_a && h->py.p.warp_a) || g.n >= 8192);
-  if (c.sweep_engine == MMC_ENGINE_KERNELS || (c.sweep_engine == MMC_ENGINE_AUTO && (!eligible || f64_kernels))) {
+  // FP32 films from 64^2 on whose transforms have the warp-shaped x passes and
+  // the pipelined column pass: 64^2 9.7 / 11.8, 128^2 14.1 / 15.9, 256^2 15.5 / 22.5
+  // (32^2, and films with other transforms: the film engine).
+  const bool kernels = h->prec == 64 ? (h->px.p.warp_a && h->py.p.warp_a) || g.n >= 8192
+                                     : h->px.p.warp_a && col_pipe_eligible(h->py.p) && g.n >= 4096;
+  if (c.sweep_engine == MMC_ENGINE_KERNELS || (c.sweep_engine == MMC_ENGINE_AUTO && (!eligible || kernels))) {
     h->engine = MMC_ENGINE_KERNELS;
     return MMC_OK;
   }
@@ -595,18 +642,10 @@ int setup_engine(mmc_handle* h, int nsm) {
   return MMC_OK;
 }
 
-// Runs `nsweeps` sweeps with counters (stage, sweep0); graph replays for the bulk.
-int run_sweeps_impl(mmc_handle* h, double T_K, long long stage, long long sweep0, long long nsweeps) {
-  if (nsweeps <= 0) return MMC_OK;
-  TRY(ensure_demag(h));
-  TRY(upload_coef(h, T_K));
-  SweepCounters c0{(uint32_t)stage, (uint32_t)sweep0};
-  CU(cudaMemcpyAsync(h->ctr, &c0, sizeof c0, cudaMemcpyHostToDevice, h->st));
-  CU(cudaStreamSynchronize(h->st));
-  if (h->engine == MMC_ENGINE_FUSED) return run_fused(h, stage, sweep0, nsweeps);
+// Enqueues `nsweeps` sweeps of the pass kernels; graph replays for the bulk.
+int run_sweeps_kernels(mmc_handle* h, long long nsweeps) {
   const int G = 64;
   long long done = 0;
-  CU(cudaEventRecord(h->ev[0], h->st));
   if (nsweeps >= G) {
     TRY(ensure_graph(h, G));
     while (nsweeps - done >= G) {
@@ -617,7 +656,22 @@ int run_sweeps_impl(mmc_handle* h, double T_K, long long stage, long long sweep0
       if ((done / G) % 16 == 0) CU(cudaStreamSynchronize(h->st));
     }
   }
-  for (; done < nsweeps; ++done) CU(enqueue_sweep(h));
+  if (done < nsweeps) CU(enqueue_sweeps(h, nsweeps - done));
+  return MMC_OK;
+}
+
+// Runs `nsweeps` sweeps with counters (stage, sweep0).
+int run_sweeps_impl(mmc_handle* h, double T_K, long long stage, long long sweep0, long long nsweeps) {
+  if (nsweeps <= 0) return MMC_OK;
+  TRY(ensure_demag(h));
+  TRY(upload_coef(h, T_K));
+  if (h->engine == MMC_ENGINE_FUSED) return run_fused(h, stage, sweep0, nsweeps);
+  CU(set_counters(h, stage, sweep0));
+  CU(cudaEventRecord(h->ev[0], h->st));
+  CU(set_split(h, handle_split(h, nsweeps)));
+  const int status = run_sweeps_kernels(h, nsweeps);
+  CU(set_split(h, false));  // also after an error or a stop request
+  TRY(status);
   CU(cudaEventRecord(h->ev[1], h->st));
   CU(cudaStreamSynchronize(h->st));
   float ms = 0;
@@ -631,8 +685,7 @@ int profile_sweeps_impl(mmc_handle* h, double T_K, long long stage, long long sw
                         double out[3]) {
   TRY(ensure_demag(h));
   TRY(upload_coef(h, T_K));
-  SweepCounters c0{(uint32_t)stage, (uint32_t)sweep0};
-  CU(cudaMemcpyAsync(h->ctr, &c0, sizeof c0, cudaMemcpyHostToDevice, h->st));
+  CU(set_counters(h, stage, sweep0));
   CU(cudaStreamSynchronize(h->st));
   double tdem = 0, tmc = 0;
   cudaEvent_t a = h->ev[0], b = h->ev[1], c = h->ev[2], t0 = h->ev[3];
@@ -643,7 +696,7 @@ int profile_sweeps_impl(mmc_handle* h, double T_K, long long stage, long long sw
     CU(cudaEventRecord(b, h->st));
     CU(mc_color(h, -1));
     CU(cudaEventRecord(c, h->st));
-    CU(launch_advance(h->ctr, 1, h->st));
+    CU(launch_advance(h->ctr, 1, h->st, CTR_SLOTS));
     CU(cudaEventSynchronize(c));
     float x = 0, y = 0;
     CU(cudaEventElapsedTime(&x, a, b));
@@ -992,6 +1045,18 @@ void destroy_impl(mmc_handle* h) {
   delete h;
 }
 
+// Row pitch of the half spectrum: rows start on 32-byte sectors (4 FP32 or 2
+// FP64 values), or in FP32 on 16 bytes only where the wider rows would push the
+// spectrum beyond the static array of mmc_demag_apply_static.  The column
+// passes' 64-byte pieces of a row otherwise touch three sectors instead of two
+// in every odd row.
+int spectrum_pitch(const Geom& g, int prec) {
+  const int even = g.hx + (g.hx & 1), wide = (g.hx + 3) & ~3;
+  if (prec == 64) return even;
+  const size_t row = 3 * (size_t)g.nyp * g.nzp * 2 * sizeof(float), limit = MMC_DEMAG_STATIC_SCRATCH_BYTES;
+  return row * even <= limit && row * wide > limit ? even : wide;
+}
+
 int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   *out = nullptr;
   TRY(config_validate(cfg));
@@ -1024,7 +1089,7 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   g.nyp = transform_len(g.typ, cfg->pbc_y == 0);
   g.nzp = transform_len(g.tzp, cfg->pbc_z == 0);
   g.hx = g.nxp / 2 + 1;
-  g.hxp = g.hx + (g.hx & 1);
+  g.hxp = spectrum_pitch(g, h->prec);
   g.per[0] = cfg->pbc_x != 0;
   g.per[1] = cfg->pbc_y != 0;
   g.per[2] = cfg->pbc_z != 0;
@@ -1050,7 +1115,8 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   int nsm = 148, optin = 48 * 1024;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  if (launch_prepare<float>(optin) != cudaSuccess || launch_prepare<double>(optin) != cudaSuccess ||
+  // this lattice's kernels, and those of the tensor's transform
+  if ((h->prec == 32 ? launch_prepare<float>(optin) : launch_prepare<double>(optin)) != cudaSuccess ||
       launch_prepare_f64s(optin) != cudaSuccess)
     return bail(fail(MMC_ERR_CUDA, "kernel attribute setup failed"));
   const size_t csize = 2 * h->tsize;
@@ -1079,7 +1145,7 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   if ((st = alloc((void**)&h->partials, (size_t)h->npartials * NQ * sizeof(double))) != MMC_OK) return bail(st);
   if ((st = alloc((void**)&h->red, NQ * sizeof(double))) != MMC_OK) return bail(st);
   if ((st = alloc((void**)&h->acc, sizeof(unsigned long long))) != MMC_OK) return bail(st);
-  if ((st = alloc((void**)&h->ctr, sizeof(SweepCounters))) != MMC_OK) return bail(st);
+  if ((st = alloc((void**)&h->ctr, CTR_SLOTS * sizeof(SweepCounters))) != MMC_OK) return bail(st);
   if ((st = alloc((void**)&h->stage64, 3 * g.n * sizeof(double))) != MMC_OK) return bail(st);
   if ((st = alloc((void**)&h->field64, 3 * g.n * sizeof(double))) != MMC_OK) return bail(st);
   for (auto& e : h->ev)
@@ -1275,8 +1341,6 @@ int anneal_loop(mmc_handle* h, const std::string& dir, int verbose) {
 // fills a corner of it.  Replicas may differ in material, field, seed and
 // temperature; the tensor spectrum is shared.  Optional parallel-tempering
 // ladders swap temperatures on the device every `swap_interval` sweeps.
-constexpr int CTR_SLOTS = 32;
-
 struct mmc_batch {
   mmc_handle* base = nullptr;  // geometry, plans, tensor (replica 0's config)
   int R = 0;
@@ -1313,9 +1377,11 @@ struct mmc_batch {
   double* d_replica_T = nullptr;
   unsigned int* d_round = nullptr;
   unsigned long long* d_counts = nullptr;
+  bool split = false;  // m and h are in the colour-split order (inside a run only)
   cudaGraphExec_t gexec = nullptr;
   int graph_len = 0;
   bool graph_pt = false;
+  bool graph_split = false, lead_split = false;
   // tempering: the graph of one swap interval whose first sweep also makes the
   // previous interval's swap (batch_sweep_lead)
   cudaGraphExec_t gexec_lead = nullptr;
@@ -1367,13 +1433,30 @@ int batch_upload_coefs(mmc_batch* b) {
   return MMC_OK;
 }
 
+// The Metropolis form of this run's sweeps, the order of m and h it needs, and
+// the change between the orders (h is rewritten by every sweep and every energy
+// evaluation before it is read: it needs no conversion).
+int batch_form(const mmc_batch* b) { return b->split ? MC_FORM_SPLIT : b->tun.mc_form; }
+bool batch_wants_split(const mmc_batch* b, long long nsweeps) {
+  const mmc_handle* h = b->base;
+  return h->prec == 32 && b->rows_band == 0 && b->tun.mc_form == MC_FORM_QUAD && nsweeps >= MC_SPLIT_SWEEPS &&
+         h->cfg.cal_demag_flag && (long long)b->R * 3 * h->g.ny * h->g.nz < (1LL << 31) &&
+         mc_split_eligible(h->g, h->px.p);
+}
+cudaError_t batch_set_split(mmc_batch* b, bool split) {
+  if (b->split == split) return cudaSuccess;
+  const cudaError_t e = launch_split_rows(b->base->g, (float*)b->m, b->R, split, b->base->st);
+  if (e == cudaSuccess) b->split = split;
+  return e;
+}
+
 // The demag field of every replica from m (default: the batch's m).
 cudaError_t batch_demag(mmc_batch* b, cudaEvent_t* ev = nullptr, const void* m = nullptr) {
   mmc_handle* h = b->base;
   if (!m) m = b->m;
   if (h->prec == 32)
     return launch_demag<float>(h->g, h->px.p, h->py.p, h->pz.p, b->tun, (const float*)m, (float*)b->h, b->spec,
-                               h->khat, h->st, b->R, ev);
+                               h->khat, h->st, b->R, ev, b->split);
   return launch_demag<double>(h->g, h->px.p, h->py.p, h->pz.p, b->tun, (const double*)m, (double*)b->h, b->spec,
                               h->khat, h->st, b->R, ev);
 }
@@ -1461,14 +1544,14 @@ cudaError_t batch_sweep_part(mmc_batch* b, int r0, int nr, cudaStream_t st, int 
   cudaError_t e = cudaSuccess;
   if (h->cfg.cal_demag_flag)
     e = launch_demag<T>(h->g, h->px.p, h->py.p, h->pz.p, b->tun, m, hh,
-                        (char*)b->spec + (size_t)r0 * ss * 2 * sizeof(T), h->khat, st, nr);
+                        (char*)b->spec + (size_t)r0 * ss * 2 * sizeof(T), h->khat, st, nr, nullptr, b->split);
   if (e != cudaSuccess) return e;
   if (strip) {
     T* mo = (T*)(parity ? b->m : b->m2) + r0 * ms;
     return launch_mc_strip<T>(h->g, (const McCoef<T>*)b->coef + r0, m, mo, hh, b->ctr + slot, b->acc + r0, st, nr);
   }
   return launch_mc<T>(h->g, (const McCoef<T>*)b->coef + r0, m, hh, b->ctr + slot, -1, b->acc + r0, st, nr,
-                      b->tun.mc_form);
+                      batch_form(b));
 }
 
 // One sweep reading counter slot `slot` (the caller advances the counters);
@@ -1512,7 +1595,7 @@ cudaError_t batch_sweep(mmc_batch* b, cudaEvent_t* ev, int slot, int parity) {
                                                 (const double*)b->h, b->ctr + slot, b->acc, h->st, b->R);
   else
     e = h->prec == 32 ? launch_mc<float>(h->g, (const McCoef<float>*)b->coef, (float*)b->m, (const float*)b->h,
-                                         b->ctr + slot, -1, b->acc, h->st, b->R, b->tun.mc_form)
+                                         b->ctr + slot, -1, b->acc, h->st, b->R, batch_form(b))
                       : launch_mc<double>(h->g, (const McCoef<double>*)b->coef, (double*)b->m, (const double*)b->h,
                                           b->ctr + slot, -1, b->acc, h->st, b->R, b->tun.mc_form);
   if (e != cudaSuccess) return e;
@@ -1546,7 +1629,7 @@ cudaError_t batch_sweep_lead(mmc_batch* b, int slot) {
                                                    (double*)b->m2, (const double*)b->h, b->ctr + slot, b->acc, h->st,
                                                    b->R);
   return h->prec == 32 ? launch_mc<float>(h->g, (const McCoef<float>*)b->coef, (float*)b->m, (const float*)b->h,
-                                          b->ctr + slot, -1, b->acc, h->st, b->R, b->tun.mc_form)
+                                          b->ctr + slot, -1, b->acc, h->st, b->R, batch_form(b))
                        : launch_mc<double>(h->g, (const McCoef<double>*)b->coef, (double*)b->m, (const double*)b->h,
                                            b->ctr + slot, -1, b->acc, h->st, b->R, b->tun.mc_form);
 }
@@ -1584,7 +1667,7 @@ cudaError_t batch_energy_kernels(mmc_batch* b, bool swap, bool with_demag) {
   if (with_demag && h->cfg.cal_demag_flag && (e = batch_demag(b)) != cudaSuccess) return e;
   const bool dm = h->cfg.cal_demag_flag != 0;
   return h->prec == 32 ? launch_energy<float>(h->g, b->ecoef, (const float*)b->m, dm ? (const float*)b->h : nullptr,
-                                              b->partials, h->npartials, b->red, h->st, b->R, with_q)
+                                              b->partials, h->npartials, b->red, h->st, b->R, with_q, b->split)
                        : launch_energy<double>(h->g, b->ecoef, (const double*)b->m,
                                                dm ? (const double*)b->h : nullptr, b->partials, h->npartials,
                                                b->red, h->st, b->R, with_q);
@@ -1600,7 +1683,7 @@ cudaError_t batch_swap(mmc_batch* b) {
 // The graph of one swap interval of `len` sweeps whose first sweep makes the
 // pending swap (batch_sweep_lead).
 int batch_graph_lead(mmc_batch* b, int len) {
-  if (b->gexec_lead && b->lead_len == len) return MMC_OK;
+  if (b->gexec_lead && b->lead_len == len && b->lead_split == b->split) return MMC_OK;
   if (b->gexec_lead) cudaGraphExecDestroy(b->gexec_lead);
   b->gexec_lead = nullptr;
   mmc_handle* h = b->base;
@@ -1615,6 +1698,7 @@ int batch_graph_lead(mmc_batch* b, int len) {
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("batch graph: ") + cudaGetErrorString(e));
   b->lead_len = len;
+  b->lead_split = b->split;
   return MMC_OK;
 }
 
@@ -1629,7 +1713,7 @@ void batch_drop_graphs(mmc_batch* b) {
 }
 
 int batch_graph(mmc_batch* b, int len, bool pt) {
-  if (b->gexec && b->graph_len == len && b->graph_pt == pt) return MMC_OK;
+  if (b->gexec && b->graph_len == len && b->graph_pt == pt && b->graph_split == b->split) return MMC_OK;
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   b->gexec = nullptr;
   mmc_handle* h = b->base;
@@ -1648,6 +1732,7 @@ int batch_graph(mmc_batch* b, int len, bool pt) {
   if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("batch graph: ") + cudaGetErrorString(e));
   b->graph_len = len;
   b->graph_pt = pt;
+  b->graph_split = b->split;
   return MMC_OK;
 }
 
@@ -1673,6 +1758,7 @@ int batch_run_begin(mmc_batch* b, BatchRun& r, long long stage, long long sweep0
   TRY(h->prec == 32 ? batch_upload_coefs<float>(b) : batch_upload_coefs<double>(b));
   CU(batch_set_counters(b, stage, sweep0));
   CU(cudaEventRecord(h->ev[0], h->st));
+  CU(batch_set_split(b, batch_wants_split(b, nsweeps)));
   if (b->rows_band > 0) CU(batch_demag(b));  // the row kernel starts from the spectrum of m
   r = BatchRun{stage, sweep0, nsweeps, 0, 0};
   if (b->interval == 0 && nsweeps >= BATCH_GRAPH_SWEEPS) TRY(batch_graph(b, BATCH_GRAPH_SWEEPS, false));
@@ -1732,6 +1818,7 @@ int batch_run_end(mmc_batch* b, BatchRun& r) {
     CU(batch_swap(b));
     r.swap_pending = false;
   }
+  CU(batch_set_split(b, false));
   CU(cudaEventRecord(h->ev[1], h->st));
   CU(cudaStreamSynchronize(h->st));
   if (b->tun.mc_form == MC_FORM_PIPE && mc_pipe_error_take())
@@ -1743,16 +1830,24 @@ int batch_run_end(mmc_batch* b, BatchRun& r) {
   return batch_sync_temperatures(b);
 }
 
+// Puts m back into the natural order after a run that ended early.
+int batch_run_abandon(mmc_batch* b, int status) {
+  if (b->split && batch_set_split(b, false) != cudaSuccess) cudaGetLastError();
+  return status;
+}
+
 int batch_run(mmc_batch* b, long long stage, long long sweep0, long long nsweeps) {
   BatchRun r;
-  TRY(batch_run_begin(b, r, stage, sweep0, nsweeps));
-  for (bool fin = false; !fin;) {
-    TRY(batch_run_piece(b, r, &fin));
-    if (b->stop.load()) return fail(MMC_ERR_INTERRUPTED, "stop requested");
+  int status = batch_run_begin(b, r, stage, sweep0, nsweeps);
+  for (bool fin = false; status == MMC_OK && !fin;) {
+    status = batch_run_piece(b, r, &fin);
+    if (status == MMC_OK && b->stop.load()) status = fail(MMC_ERR_INTERRUPTED, "stop requested");
     // bound the queued work so that a stop request takes effect quickly
-    if (r.pieces % 64 == 0) CU(cudaStreamSynchronize(b->base->st));
+    if (status == MMC_OK && r.pieces % 64 == 0 && cudaStreamSynchronize(b->base->st) != cudaSuccess)
+      status = fail(MMC_ERR_CUDA, "stream synchronisation failed in a batch run");
   }
-  return batch_run_end(b, r);
+  if (status == MMC_OK) status = batch_run_end(b, r);
+  return batch_run_abandon(b, status);
 }
 
 // Times every launch shape the batch can run with -- the row kernel with each
@@ -1795,6 +1890,8 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
     b->tun = cd.tun;
     b->streams = cd.streams;
     e = cudaMemcpyAsync(b->m, saved, mbytes, cudaMemcpyDeviceToDevice, h->st);
+    b->split = false;
+    if (e == cudaSuccess) e = batch_set_split(b, batch_wants_split(b, BATCH_GRAPH_SWEEPS));
     if (e == cudaSuccess) e = batch_set_counters(b, 0, 0);
     if (e == cudaSuccess && b->rows_band > 0) e = batch_demag(b);
     // timed the way runs execute: replays of a captured graph of
@@ -1862,16 +1959,11 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
         }
     }
   }
-  // the column pass held in registers (films with y lengths 64 and 256):
-  // col_lean = 2 all three components per thread, 3 one component per thread
-  if (h->cfg.cal_demag_flag && g.nzp == 1 && h->py.p.warp_a == h->py.p.warp_b &&
-      (h->py.p.warp_a == 8 || h->py.p.warp_a == 16)) {
-    const Cand base = best;
-    for (int form = 2; form <= 3; ++form) {
-      Cand c = base;
-      c.tun.col_lean = form;
-      trial(c);
-    }
+  // the pipelined film column pass (FP32, y lengths 32 to 256)
+  if (h->cfg.cal_demag_flag && h->prec == 32 && g.nzp == 1 && col_pipe_eligible(h->py.p) && best.tun.col_lean < 2) {
+    Cand c = best;
+    c.tun.col_lean = 2;
+    trial(c);
   }
   {
     std::vector<int> forms;
@@ -1910,6 +2002,7 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
     b->streams = best.streams;
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(b->m, saved, mbytes, cudaMemcpyDeviceToDevice, h->st);
+  b->split = false;
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->acc, acc0.data(), b->R * sizeof(unsigned long long), cudaMemcpyHostToDevice, h->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
@@ -2524,6 +2617,8 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
     if (e == cudaSuccess && (nsweeps & 1)) e = batch_rows_settle(b);
     if (e != cudaSuccess) status = fail(MMC_ERR_CUDA, cudaGetErrorString(e));
   }
+  if (batch_set_split(b, batch_wants_split(b, nsweeps)) != cudaSuccess)
+    status = fail(MMC_ERR_CUDA, "row order conversion failed");
   for (long long s = 0; b->rows_band == 0 && s < nsweeps && status == MMC_OK; ++s) {
     cudaError_t e = batch_sweep(b, ev, 0, (int)(s & 1));
     if (e == cudaSuccess) e = launch_advance(b->ctr, 1, h->st, CTR_SLOTS);
@@ -2539,6 +2634,7 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
     cudaError_t e = batch_strip_settle(b);
     if (e != cudaSuccess) status = fail(MMC_ERR_CUDA, cudaGetErrorString(e));
   }
+  batch_run_abandon(b, status);
   for (auto& e : ev) cudaEventDestroy(e);
   if (status != MMC_OK) return status;
   CU(cudaStreamSynchronize(h->st));
@@ -2646,11 +2742,7 @@ int mmc_farm_create(mmc_batch* const* batches, int nbatches, mmc_farm** out) {
 
 void mmc_farm_destroy(mmc_farm* f) { delete f; }
 
-int mmc_farm_run_sweeps(mmc_farm* f, long long stage, long long sweep0, long long nsweeps) {
-  if (!f) return fail(MMC_ERR_INVALID, "null farm");
-  if (nsweeps < 0 || stage < 0 || sweep0 < 0) return fail(MMC_ERR_INVALID, "negative counter");
-  TRY(set_dev(f->batches[0]->base));
-  f->stop.store(0);
+static int farm_run(mmc_farm* f, long long stage, long long sweep0, long long nsweeps) {
   const auto t0 = std::chrono::steady_clock::now();
   const size_t nb = f->batches.size();
   std::vector<BatchRun> runs(nb);
@@ -2676,6 +2768,16 @@ int mmc_farm_run_sweeps(mmc_farm* f, long long stage, long long sweep0, long lon
   for (size_t i = 0; i < nb; ++i) TRY(batch_run_end(f->batches[i], runs[i]));
   f->last_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return MMC_OK;
+}
+
+int mmc_farm_run_sweeps(mmc_farm* f, long long stage, long long sweep0, long long nsweeps) {
+  if (!f) return fail(MMC_ERR_INVALID, "null farm");
+  if (nsweeps < 0 || stage < 0 || sweep0 < 0) return fail(MMC_ERR_INVALID, "negative counter");
+  TRY(set_dev(f->batches[0]->base));
+  f->stop.store(0);
+  const int status = farm_run(f, stage, sweep0, nsweeps);
+  for (mmc_batch* b : f->batches) batch_run_abandon(b, status);
+  return status;
 }
 
 int mmc_farm_last_run_ms(mmc_farm* f, double* ms) {
