@@ -178,6 +178,98 @@ __device__ __forceinline__ void load_twiddles(const FftPlan& p, C<T>* dst) {
   for (int i = threadIdx.x; i < p.tw_total; i += blockDim.x) dst[i] = src[i];
 }
 
+// One stage of an odd radix R >= 7: the direct R-point DFT with R known at
+// compile time, so that the R values stay in registers and the matrix of roots
+// [q][t] is read from global memory, the same word for a whole warp.  (One loop
+// over a run-time R held them in local memory: the demag convolution of an open
+// 512^2 film, lines of 1023 = 3 11 31, took 423 us in FP32 and 5601 us in FP64;
+// now 199 and 1506 us.)  Bound by the R^2 multiply-adds per butterfly.  FP32
+// products are contracted as they were in that loop, written out.
+__device__ __forceinline__ float2 odd_mul(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+template <bool INV, typename V>
+__device__ __forceinline__ V odd_twiddle(V a, V b) {
+  if constexpr (sizeof(V) == sizeof(float2)) return INV ? tmulc(a, b) : odd_mul(a, b);
+  return INV ? cmulc(a, b) : cmul(a, b);
+}
+template <bool INV, typename V>
+__device__ __forceinline__ V odd_mac(V acc, V a, V b) {
+  if constexpr (sizeof(V) == sizeof(float2)) return padd(acc, INV ? tmulc(a, b) : odd_mul(a, b));
+  return INV ? cmacc(acc, a, b) : cmac(acc, a, b);
+}
+template <typename T, bool INV, int R>
+__device__ __noinline__ void odd_stage(const C<T>* src, C<T>* dst, int total, int stride, int nb, int Ns, FastDiv dnb,
+                                       FastDiv dns, const C<T>* W, const C<T>* __restrict__ mat) {
+  using V = C<T>;
+  // long radices leave few butterflies (99 for three lines of 1023 in radix 31):
+  // `parts` threads share one, each taking a range of its outputs
+  const int parts = min(8, max(1, (2 * (int)blockDim.x + total - 1) / total)), per = (R + parts - 1) / parts;
+  for (int idx0 = threadIdx.x; idx0 < total * parts; idx0 += blockDim.x) {
+    const int part = idx0 / total, idx = idx0 - part * total;
+    const int line = dnb.div(idx), j = idx - line * nb, k = j - dns.div(j) * Ns;
+    const V* in = src + (long long)line * stride + j;
+    V* out = dst + (long long)line * stride + (j - k) * R + k;
+    V v[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = in[t * nb];
+    if (k) {
+#pragma unroll
+      for (int t = 1; t < R; ++t) v[t] = odd_twiddle<INV>(v[t], W[(t - 1) * Ns + k]);
+    }
+    if constexpr (fused_mul<V>) {
+      // FP64: the values t and R - t in their sum a and difference b, which give
+      // the outputs q and R - q together, X = (v0 + sum a cos) -+ i sum b sin:
+      // (R - 1)^2 operations instead of 4 R (R - 1)
+      constexpr int H = (R - 1) / 2;
+      V s0 = v[0];
+#pragma unroll
+      for (int t = 1; t <= H; ++t) {
+        const V a = cadd(v[t], v[R - t]), b = csub(v[t], v[R - t]);
+        v[t] = a;
+        v[R - t] = b;
+        s0 = cadd(s0, a);
+      }
+      const int perh = (H + parts - 1) / parts, p1 = min(H, (part + 1) * perh);
+      if (part == 0) out[0] = s0;
+#pragma unroll 1
+      for (int q = 1 + part * perh; q <= p1; ++q) {
+        const V* row = mat + q * R;
+        V P = v[0], S = cmk<V>(0, 0);
+#pragma unroll
+        for (int t = 1; t <= H; ++t) {
+          const V w = row[t];
+          P = cmk<V>(fma_rn(v[t].x, w.x, P.x), fma_rn(v[t].y, w.x, P.y));
+          S = cmk<V>(fma_rn(v[R - t].x, w.y, S.x), fma_rn(v[R - t].y, w.y, S.y));
+        }
+        const V u = cmk<V>(P.x - S.y, P.y + S.x), d = cmk<V>(P.x + S.y, P.y - S.x);  // P + i S, P - i S
+        out[q * Ns] = INV ? d : u;
+        out[(R - q) * Ns] = INV ? u : d;
+      }
+      continue;
+    }
+    const int q1 = min(R, (part + 1) * per);
+#pragma unroll 1
+    for (int q = part * per; q < q1; ++q) {
+      const V* row = mat + q * R;
+      V acc = v[0];
+#pragma unroll
+      for (int t = 1; t < R; ++t) acc = odd_mac<INV>(acc, v[t], row[t]);
+      out[q * Ns] = acc;
+    }
+  }
+}
+template <typename T, bool INV>
+__device__ __forceinline__ void odd_stages(const C<T>* src, C<T>* dst, int total, int stride, int R, int nb, int Ns,
+                                           FastDiv dnb, FastDiv dns, const C<T>* W, const C<T>* mat) {
+  switch (R) {
+#define MMC_ODD(R_) \
+  case R_: odd_stage<T, INV, R_>(src, dst, total, stride, nb, Ns, dnb, dns, W, mat); break;
+    MMC_ODD(7) MMC_ODD(11) MMC_ODD(13) MMC_ODD(17) MMC_ODD(19) MMC_ODD(23) MMC_ODD(29) MMC_ODD(31)
+#undef MMC_ODD
+  }
+}
+
 // Transforms `nlines` lines of length p.n; line l starts at buf + l*stride.
 // `a` holds the input, `b` is scratch of the same shape.  Returns the buffer
 // holding the result (a or b).  All threads of the block must call it.
@@ -193,7 +285,8 @@ __device__ __noinline__ C<T>* fft_lines(C<T>* a, C<T>* b, int nlines, int stride
     const FastDiv dnb = p.dnb[s], dns = p.dns[s];
     const V* W = tw + p.tw_off[s];
     const int total = nlines * nb;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+    if (R >= 7) odd_stages<T, INV>(src, dst, total, stride, R, nb, Ns, dnb, dns, W, plan_tw<T>(p) + p.odd_off[s]);
+    for (int idx = threadIdx.x; R < 7 && idx < total; idx += blockDim.x) {
       const int line = dnb.div(idx);
       const int j = idx - line * nb;
       const int k = j - dns.div(j) * Ns;
@@ -277,25 +370,6 @@ __device__ __noinline__ C<T>* fft_lines(C<T>* a, C<T>* b, int nlines, int stride
         out[2 * Ns] = cadd(a2, mb2);
         out[3 * Ns] = csub(a2, mb2);
         out[4 * Ns] = csub(a1, mb1);
-      } else {
-        // generic odd radix: direct R-point DFT with the stage's roots of unity
-        const V* RT = tw + p.root_off[s];
-        V v[FFT_MAX_RADIX];
-        for (int t = 0; t < R; ++t) {
-          V x = in[t * nb];
-          if (t && k) x = INV ? cmulc(x, W[(t - 1) * Ns + k]) : cmul(x, W[(t - 1) * Ns + k]);
-          v[t] = x;
-        }
-        for (int q = 0; q < R; ++q) {
-          V acc = v[0];
-          int e = 0;
-          for (int t = 1; t < R; ++t) {
-            e += q;
-            if (e >= R) e -= R;
-            acc = INV ? cmacc(acc, v[t], RT[e]) : cmac(acc, v[t], RT[e]);
-          }
-          out[q * Ns] = acc;
-        }
       }
     }
     __syncthreads();
@@ -618,6 +692,16 @@ __device__ __forceinline__ void fft_warp_call(C<T>* buf, int nlines, int stride,
 // plan with warp_a == 32 must only reach those (the host checks).
 // PAD: the warp-level transforms use padded transpose rows (stride >=
 // n + warp_a - 1).
+// The wide shapes alone (kernels that only plans with warp_a == 32 reach).
+template <typename T, bool INV, bool INL, bool PAD>
+__device__ __forceinline__ void fft_wide(C<T>* a, int nlines, int stride, const FftPlan& p, const C<T>* tw) {
+  if (p.warp_b == 32)
+    fft_warp_call<T, INV, 32, 32, INL, PAD>(a, nlines, stride, tw + p.full_off);
+  else
+    fft_warp_call<T, INV, 32, 16, INL, PAD>(a, nlines, stride, tw + p.full_off);
+  __syncthreads();
+}
+
 template <typename T, bool INV, bool INL = false, bool WIDE = false, bool PAD = false>
 __device__ C<T>* fft_run(C<T>* a, C<T>* b, int nlines, int stride, const FftPlan& p, const C<T>* tw) {
   if constexpr (WIDE) {

@@ -571,7 +571,9 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
   V* cur = bufA;
   V* oth = bufB;
   if (flags & PASS_FWD) {
-    V* r = fft_run<T, false, INL, WIDE, true>(cur, oth, nlines, stride, p, tw);
+    V* r = cur;
+    if constexpr (WIDE) fft_wide<T, false, INL, true>(cur, nlines, stride, p, tw);
+    else r = fft_run<T, false, INL, false, true>(cur, oth, nlines, stride, p, tw);
     if (r != cur) {
       oth = cur;
       cur = r;
@@ -600,7 +602,9 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
     __syncthreads();
   }
   if (flags & PASS_INV) {
-    V* r = fft_run<T, true, INL, WIDE, true>(cur, oth, nlines, stride, p, tw);
+    V* r = cur;
+    if constexpr (WIDE) fft_wide<T, true, INL, true>(cur, nlines, stride, p, tw);
+    else r = fft_run<T, true, INL, false, true>(cur, oth, nlines, stride, p, tw);
     if (r != cur) {
       oth = cur;
       cur = r;

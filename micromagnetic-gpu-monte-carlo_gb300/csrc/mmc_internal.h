@@ -36,15 +36,13 @@ constexpr int FFT_MAX_RADIX = 31;  // largest prime factor an FFT length may hav
 // Mixed-radix Stockham plan for one transform length.  Stage s has radix
 // radix[s] and ns[s] = product of the earlier radices.  Twiddles of stage s
 // live at tw_off[s]: entry (t-1)*ns + k = exp(-2 pi i t k / (ns*radix)) for
-// t in [1, radix), k in [0, ns); the radix-th roots of unity exp(-2 pi i m /
-// radix) live at root_off[s].
+// t in [1, radix), k in [0, ns).
 struct FftPlan {
   int n;
   int nstages;
   int radix[FFT_MAX_STAGES];
   int ns[FFT_MAX_STAGES];
   int tw_off[FFT_MAX_STAGES];
-  int root_off[FFT_MAX_STAGES];
   int tw_total;
   // Warp-level transform for power-of-two lengths n = A * B (A values per lane,
   // B lanes per line): warp_a = A (0 = use the Stockham stages), and the n
@@ -53,6 +51,7 @@ struct FftPlan {
   int full_off;
   int lane_off;  // the roots in the order the lanes of a line take them: [ka][b] = root b ka, ka < A, b < B
                  // (behind tw_total: only the FP32 x passes load it)
+  int odd_off[FFT_MAX_STAGES];  // radix 7 and above: the radix-point DFT's matrix [q][t] = root q t (behind tw_total)
   FastDiv dn;  // n
   FastDiv dnb[FFT_MAX_STAGES];  // n / radix[s]
   FastDiv dns[FFT_MAX_STAGES];  // ns[s]

@@ -141,14 +141,6 @@ int make_plan(int n, PlanHost* ph) {
         tw.push_back(c);
         tw.push_back(sn);
       }
-    p.root_off[s] = (int)(tw.size() / 2);
-    if (R != 2 && R != 3 && R != 4)
-      for (int q = 0; q < R; ++q) {
-        double c, sn;
-        unit_root(q, R, &c, &sn);
-        tw.push_back(c);
-        tw.push_back(sn);
-      }
     ns *= R;
   }
   p.nstages = (int)rad.size();
@@ -182,6 +174,18 @@ int make_plan(int n, PlanHost* ph) {
       tw.push_back(c);
       tw.push_back(sn);
     }
+  for (size_t s = 0; s < rad.size(); ++s) {
+    const int R = rad[s];
+    p.odd_off[s] = (int)(tw.size() / 2);
+    if (R < 7) continue;
+    for (int q = 0; q < R; ++q)
+      for (int t = 0; t < R; ++t) {
+        double c, sn;
+        unit_root((long long)q * t, R, &c, &sn);
+        tw.push_back(c);
+        tw.push_back(sn);
+      }
+  }
   size_t cnt = tw.size() / 2;
   if (cnt == 0) cnt = 1, tw.push_back(1.0), tw.push_back(0.0);
   std::vector<float> tw32(tw.size());
