@@ -111,7 +111,17 @@ int transform_len(int t, bool open) {
   return has_mixed_radix_plan(t) ? t : p;
 }
 
-int make_plan(int n, PlanHost* ph) {
+// A small host array to the device, ordered with the work of stream st.  The
+// streams here do not wait for the legacy stream, on which a plain cudaMemcpy or
+// cudaMemset returns before its bytes are in place (seen when several processes
+// share the GPU: sweeps ran with the previous coefficients); and the source is
+// often a local object, so the copy is waited for.
+cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
+int make_plan(int n, PlanHost* ph, cudaStream_t st) {
   FftPlan& p = ph->p;
   p = FftPlan{};
   p.n = n;
@@ -168,12 +178,11 @@ int make_plan(int n, PlanHost* ph) {
   p.tw_total = (int)(tw.size() / 2);
   p.lane_off = p.tw_total;
   for (int ka = 0; ka < p.warp_a; ++ka)
-    for (int b = 0; b < p.warp_b; ++b) {
-      double c, sn;
-      unit_root((long long)b * ka, n, &c, &sn);
-      tw.push_back(c);
-      tw.push_back(sn);
-    }
+    for (int b = 0; b < p.warp_b; ++b)
+      for (int q = 0; q < 2; ++q) {
+        const double v = tw[2 * (size_t)(p.full_off + b * ka % n) + q];
+        tw.push_back(v);
+      }
   for (size_t s = 0; s < rad.size(); ++s) {
     const int R = rad[s];
     p.odd_off[s] = (int)(tw.size() / 2);
@@ -192,8 +201,8 @@ int make_plan(int n, PlanHost* ph) {
   for (size_t i = 0; i < tw.size(); ++i) tw32[i] = (float)tw[i];
   CU(cudaMalloc(&ph->d64, cnt * sizeof(double2)));
   CU(cudaMalloc(&ph->d32, cnt * sizeof(float2)));
-  CU(cudaMemcpy(ph->d64, tw.data(), cnt * sizeof(double2), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(ph->d32, tw32.data(), cnt * sizeof(float2), cudaMemcpyHostToDevice));
+  CU(upload(ph->d64, tw.data(), cnt * sizeof(double2), st));
+  CU(upload(ph->d32, tw32.data(), cnt * sizeof(float2), st));
   p.tw64 = ph->d64;
   p.tw32 = ph->d32;
   return MMC_OK;
@@ -633,7 +642,7 @@ int setup_engine(mmc_handle* h, int nsm) {
       h->fused_blocks = blocks;
       void* p = nullptr;
       CU(cudaMalloc(&p, grid_barrier_bytes()));
-      CU(cudaMemset(p, 0, grid_barrier_bytes()));
+      CU(cudaMemsetAsync(p, 0, grid_barrier_bytes(), h->st));
       h->bar = (GridBarrier*)p;
       CU(cudaMalloc(&h->m2, 3 * (size_t)g.n * h->tsize));
       CU(cudaMalloc(&h->spec2, 3 * (size_t)g.nspec * 2 * h->tsize));
@@ -794,7 +803,7 @@ int build_demag_impl(mmc_handle* h, const char* cache_dir) {
   int status = MMC_OK;
   do {
     if (loaded) {
-      cudaError_t e = cudaMemcpy(k6, h->tensor.data(), 6 * (size_t)g.tnp * sizeof(double), cudaMemcpyHostToDevice);
+      cudaError_t e = upload(k6, h->tensor.data(), 6 * (size_t)g.tnp * sizeof(double), h->st);
       if (e != cudaSuccess) {
         status = fail(MMC_ERR_CUDA, cudaGetErrorString(e));
         break;
@@ -1113,9 +1122,9 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
   if (cudaStreamCreateWithFlags(&h->st_own, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(MMC_ERR_CUDA, "stream creation failed"));
   h->st = h->st_own;
-  if ((st = make_plan(g.nxp, &h->px)) != MMC_OK) return bail(st);
-  if ((st = make_plan(g.nyp, &h->py)) != MMC_OK) return bail(st);
-  if ((st = make_plan(g.nzp, &h->pz)) != MMC_OK) return bail(st);
+  if ((st = make_plan(g.nxp, &h->px, h->st)) != MMC_OK) return bail(st);
+  if ((st = make_plan(g.nyp, &h->py, h->st)) != MMC_OK) return bail(st);
+  if ((st = make_plan(g.nzp, &h->pz, h->st)) != MMC_OK) return bail(st);
   int nsm = 148, optin = 48 * 1024;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -1156,10 +1165,10 @@ int create_impl(const mmc_config* cfg, int device, mmc_handle** out) {
     if (cudaEventCreate(&e) != cudaSuccess) return bail(fail(MMC_ERR_CUDA, "event creation failed"));
   if (cudaMallocHost(&h->red_host, NQ * sizeof(double)) != cudaSuccess)
     return bail(fail(MMC_ERR_OOM, "pinned allocation failed"));
-  if (cudaMemset(h->acc, 0, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemset(h->h, 0, 3 * g.n * h->tsize) != cudaSuccess ||
-      (h->spec && cudaMemset(h->spec, 0, 3 * g.nspec * csize) != cudaSuccess) ||
-      (h->khat && cudaMemset(h->khat, 0, 6 * g.nspec * csize) != cudaSuccess))
+  if (cudaMemsetAsync(h->acc, 0, sizeof(unsigned long long), h->st) != cudaSuccess ||
+      cudaMemsetAsync(h->h, 0, 3 * g.n * h->tsize, h->st) != cudaSuccess ||
+      (h->spec && cudaMemsetAsync(h->spec, 0, 3 * g.nspec * csize, h->st) != cudaSuccess) ||
+      (h->khat && cudaMemsetAsync(h->khat, 0, 6 * g.nspec * csize, h->st) != cudaSuccess))
     return bail(fail(MMC_ERR_CUDA, "memset failed"));
   if ((st = setup_engine(h, nsm)) != MMC_OK) return bail(st);
   // initial magnetisation (src/main.cu:289-333)
@@ -1432,8 +1441,8 @@ int batch_upload_coefs(mmc_batch* b) {
     p[r] = make_mc_params(b->cfgs[r], b->base->k0, b->seeds[r]);
     c[r] = mc_coef_from<T>(p[r], b->T[r]);
   }
-  CU(cudaMemcpy(b->params, p.data(), b->R * sizeof(McParams), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(b->coef, c.data(), b->R * sizeof(McCoef<T>), cudaMemcpyHostToDevice));
+  CU(upload(b->params, p.data(), b->R * sizeof(McParams), b->base->st));
+  CU(upload(b->coef, c.data(), b->R * sizeof(McCoef<T>), b->base->st));
   return MMC_OK;
 }
 
@@ -2103,9 +2112,9 @@ int batch_create_impl(const mmc_config* cfgs, int R, int device, mmc_batch** out
   if ((st = alloc((void**)&b->ctr, CTR_SLOTS * sizeof(SweepCounters))) != MMC_OK) return bail(st);
   if (cudaMallocHost(&b->red_host, (size_t)R * NQ * sizeof(double)) != cudaSuccess)
     return bail(fail(MMC_ERR_OOM, "pinned allocation failed"));
-  if (cudaMemset(b->acc, 0, R * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemset(b->h, 0, (size_t)R * 3 * g.n * ts) != cudaSuccess ||
-      (b->spec && cudaMemset(b->spec, 0, (size_t)R * 3 * g.nspec * cs) != cudaSuccess))
+  if (cudaMemsetAsync(b->acc, 0, R * sizeof(unsigned long long), h->st) != cudaSuccess ||
+      cudaMemsetAsync(b->h, 0, (size_t)R * 3 * g.n * ts, h->st) != cudaSuccess ||
+      (b->spec && cudaMemsetAsync(b->spec, 0, (size_t)R * 3 * g.nspec * cs, h->st) != cudaSuccess))
     return bail(fail(MMC_ERR_CUDA, "memset failed"));
   std::vector<EnCoef> ec(R);
   for (int r = 0; r < R; ++r) {
@@ -2113,7 +2122,7 @@ int batch_create_impl(const mmc_config* cfgs, int R, int device, mmc_batch** out
     tmp.cfg = cfgs[r];
     ec[r] = make_en_coef(&tmp);
   }
-  if (cudaMemcpy(b->ecoef, ec.data(), R * sizeof(EnCoef), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload(b->ecoef, ec.data(), R * sizeof(EnCoef), h->st) != cudaSuccess)
     return bail(fail(MMC_ERR_CUDA, "coefficient upload failed"));
   // initial states: random from each replica's seed, or its OVF file
   for (int r = 0; r < R; ++r) {
@@ -2128,7 +2137,7 @@ int batch_create_impl(const mmc_config* cfgs, int R, int device, mmc_batch** out
                          mm.data() + g.n, mm.data() + 2 * g.n)) != MMC_OK)
         return bail(st);
       if ((st = unit_vectors(mm.data(), g.n, cfgs[r].ovf_filename)) != MMC_OK) return bail(st);
-      if (cudaMemcpy(h->stage64, mm.data(), 3 * g.n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+      if (upload(h->stage64, mm.data(), 3 * g.n * sizeof(double), h->st) != cudaSuccess)
         return bail(fail(MMC_ERR_CUDA, "upload failed"));
       cudaError_t e = h->prec == 32 ? launch_from_f64<float>(3 * g.n, h->stage64, (float*)b->m + off, h->st)
                                     : launch_from_f64<double>(3 * g.n, h->stage64, (double*)b->m + off, h->st);
@@ -2473,7 +2482,7 @@ int mmc_profile_fused(mmc_handle* h, double temperature, long long stage, long l
   TRY(upload_coef(h, temperature));
   unsigned long long* d = nullptr;
   CU(cudaMalloc(&d, FUSED_STAMP_WORDS * sizeof(unsigned long long)));
-  cudaError_t e = cudaMemset(d, 0, FUSED_STAMP_WORDS * sizeof(unsigned long long));
+  cudaError_t e = cudaMemsetAsync(d, 0, FUSED_STAMP_WORDS * sizeof(unsigned long long), h->st);
   if (e == cudaSuccess)
     e = h->prec == 32 ? fused_chunk<float>(h, stage, sweep0, (int)nsweeps, d)
                       : fused_chunk<double>(h, stage, sweep0, (int)nsweeps, d);
@@ -2517,7 +2526,7 @@ int mmc_batch_set_temperatures(mmc_batch* b, const double* T) {
   b->T.assign(T, T + b->R);
   if (b->interval > 0) {
     TRY(set_dev(b->base));
-    CU(cudaMemcpy(b->d_replica_T, b->T.data(), b->R * sizeof(double), cudaMemcpyHostToDevice));
+    CU(upload(b->d_replica_T, b->T.data(), b->R * sizeof(double), b->base->st));
   }
   return MMC_OK;
 }
@@ -2555,11 +2564,11 @@ int mmc_batch_set_ladders(mmc_batch* b, int nladders, int per_ladder, const int*
   TRY(re((void**)&b->d_round, sizeof(unsigned int)));
   TRY(re((void**)&b->d_counts, 2 * sizeof(unsigned long long)));
   for (size_t i = 0; i < nk; ++i) b->T[replicas[i]] = temps[i];
-  CU(cudaMemcpy(b->d_replica_at, replicas, nk * sizeof(int), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(b->d_temps, temps, nk * sizeof(double), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(b->d_replica_T, b->T.data(), b->R * sizeof(double), cudaMemcpyHostToDevice));
-  CU(cudaMemset(b->d_round, 0, sizeof(unsigned int)));
-  CU(cudaMemset(b->d_counts, 0, 2 * sizeof(unsigned long long)));
+  CU(upload(b->d_replica_at, replicas, nk * sizeof(int), b->base->st));
+  CU(upload(b->d_temps, temps, nk * sizeof(double), b->base->st));
+  CU(upload(b->d_replica_T, b->T.data(), b->R * sizeof(double), b->base->st));
+  CU(cudaMemsetAsync(b->d_round, 0, sizeof(unsigned int), b->base->st));
+  CU(cudaMemsetAsync(b->d_counts, 0, 2 * sizeof(unsigned long long), b->base->st));
   b->pt.nladders = nladders;
   b->pt.K = per_ladder;
   b->pt.replica_at = b->d_replica_at;
@@ -2837,9 +2846,9 @@ int mmc_batch_set_m(mmc_batch* b, int r, const double* mx, const double* my, con
   mmc_handle* h = b->base;
   TRY(set_dev(h));
   const long long n = h->g.n;
-  CU(cudaMemcpy(h->stage64, mx, n * sizeof(double), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(h->stage64 + n, my, n * sizeof(double), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(h->stage64 + 2 * n, mz, n * sizeof(double), cudaMemcpyHostToDevice));
+  CU(upload(h->stage64, mx, n * sizeof(double), h->st));
+  CU(upload(h->stage64 + n, my, n * sizeof(double), h->st));
+  CU(upload(h->stage64 + 2 * n, mz, n * sizeof(double), h->st));
   CU(h->prec == 32 ? launch_from_f64<float>(3 * n, h->stage64, (float*)b->m + off, h->st)
                    : launch_from_f64<double>(3 * n, h->stage64, (double*)b->m + off, h->st));
   CU(cudaStreamSynchronize(h->st));
