@@ -816,67 +816,90 @@ inline cudaError_t launch_col_pipe(const FftPlan& p, float2* S, long long nspec,
 }
 
 // Column pass for short lines (n <= 16: the padded z axis of thin 3-D
-// lattices, short y axes): one thread per column (kx, plane) holding the three
-// component lines in registers, transformed by ThreadDft -- no shared-memory
-// staging, no barriers, and loads and stores coalesced across the threads'
-// consecutive kx.  Same flags, product and tensor layout as k_col_pass.
+// lattices, short y axes): csh_cols columns (kx, plane) per CTA, one thread per
+// column and component with the line in registers, transformed by ThreadDft.
+// For the product the threads exchange their lines through shared memory, each
+// taking all three components of every third position, so that every word of
+// the tensor is read once, its loads issued before the transform.
+// Bound by the traffic of the tensor and the spectrum.  (One thread per column
+// with all three lines: 255 registers, two CTAs per SM.)  Demag field of a
+// 512 x 512 x 8 slab: 144 -> 98 us in FP32 (106 without the early tensor loads),
+// 2122 -> 1215 us in FP64 with lines64.cuh's passes; 128 x 128 x 4: 23.4 -> 19.2 us.
+// Same flags, product and tensor layout as k_col_pass.
+template <typename T>
+constexpr int csh_cols = sizeof(T) == 4 ? 64 : 32;
 template <typename T, int N>
-__global__ void __launch_bounds__(128) k_col_short(FftPlan p, C<T>* __restrict__ S, long long nspec,
-                                                   const C<T>* __restrict__ khat, int hx, long long plane_stride,
-                                                   long long pos_stride, int load_lim, int store_lim, int flags,
-                                                   T inv_n, long long s_rstride) {
+__global__ void __launch_bounds__(3 * csh_cols<T>, sizeof(T) == 4 ? 2 : 1)
+    k_col_short(FftPlan p, C<T>* __restrict__ S, long long nspec, const C<T>* __restrict__ khat, FastDiv dhx, int hx,
+                int total, long long plane_stride, long long pos_stride, int load_lim, int store_lim, int flags,
+                T inv_n, long long s_rstride) {
   using V = C<T>;
+  constexpr int CSH_COLS = csh_cols<T>, ZN = (N + 2) / 3;
+  constexpr bool PRE = sizeof(T) == 4;
   __shared__ V rt[N];
+  __shared__ V line[3][N][CSH_COLS];
   S += blockIdx.z * s_rstride;
   {
     const V* src = plan_tw<T>(p) + p.full_off;
     for (int i = threadIdx.x; i < N; i += blockDim.x) rt[i] = src[i];
   }
+  const int c = threadIdx.x / CSH_COLS, j = threadIdx.x - c * CSH_COLS;
+  const int col = blockIdx.x * CSH_COLS + j;
+  const bool mine = col < total;
+  const int plane = mine ? dhx.div(col) : 0, kx = mine ? col - plane * hx : 0;
+  const long long base = plane * plane_stride + kx;
+  V kk[PRE ? ZN : 1][6];
+  if (PRE && (flags & PASS_MUL)) {
+#pragma unroll
+    for (int q = 0; q < ZN; ++q)
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+        if (c + 3 * q < N) kk[q][i] = khat[i * nspec + base + (c + 3 * q) * pos_stride];
+  }
   pdl_wait();
   __syncthreads();
-  const int kx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (kx >= hx) return;
-  const long long base = (long long)blockIdx.y * plane_stride + kx;
-  V v[3][N];
+  V* s0 = S + c * nspec + base;
+  V v[N];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int z = 0; z < N; ++z) v[c][z] = z < load_lim ? S[c * nspec + base + z * pos_stride] : cmk<V>(0, 0);
-  if (flags & PASS_FWD) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) ThreadDft<T, false, N, 1>::run(v[c], rt);
-  }
+  for (int z = 0; z < N; ++z) v[z] = z < load_lim ? s0[z * pos_stride] : cmk<V>(0, 0);
+  if (flags & PASS_FWD) ThreadDft<T, false, N, 1>::run(v, rt);
   if (flags & PASS_MUL) {
 #pragma unroll
-    for (int z = 0; z < N; ++z) {
-      const V* kk = khat + base + z * pos_stride;
-      V kxx = kk[0], kxy = kk[nspec], kxz = kk[2 * nspec];
-      V kyy = kk[3 * nspec], kyz = kk[4 * nspec], kzz = kk[5 * nspec];
-      if (flags & PASS_SYM) kxx.y = kxy.y = kxz.y = kyy.y = kyz.y = kzz.y = (T)0;
-      const V mx = v[0][z], my = v[1][z], mz = v[2][z];
-      const V hx_ = tensor_row(mx, my, mz, kxx, kxy, kxz);
-      const V hy_ = tensor_row(mx, my, mz, kxy, kyy, kyz);
-      const V hz_ = tensor_row(mx, my, mz, kxz, kyz, kzz);
-      v[0][z] = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
-      v[1][z] = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
-      v[2][z] = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
+    for (int z = 0; z < N; ++z) line[c][z][j] = v[z];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ZN; ++q) {
+      const int z = c + 3 * q;
+      if (z < N) {
+        V k[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          k[i] = PRE ? kk[PRE ? q : 0][i] : khat[i * nspec + base + z * pos_stride];
+          if (flags & PASS_SYM) k[i].y = (T)0;
+        }
+        const V mx = line[0][z][j], my = line[1][z][j], mz = line[2][z][j];
+        const V hx_ = tensor_row(mx, my, mz, k[0], k[1], k[2]);
+        const V hy_ = tensor_row(mx, my, mz, k[1], k[3], k[4]);
+        const V hz_ = tensor_row(mx, my, mz, k[2], k[4], k[5]);
+        line[0][z][j] = cmk<V>(hx_.x * inv_n, hx_.y * inv_n);
+        line[1][z][j] = cmk<V>(hy_.x * inv_n, hy_.y * inv_n);
+        line[2][z][j] = cmk<V>(hz_.x * inv_n, hz_.y * inv_n);
+      }
     }
+    __syncthreads();
+#pragma unroll
+    for (int z = 0; z < N; ++z) v[z] = line[c][z][j];
   }
-  if (flags & PASS_INV) {
+  if (flags & PASS_INV) ThreadDft<T, true, N, 1>::run(v, rt);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ThreadDft<T, true, N, 1>::run(v[c], rt);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int z = 0; z < N; ++z)
-      if (z < store_lim) S[c * nspec + base + z * pos_stride] = v[c][z];
+  for (int z = 0; z < N; ++z)
+    if (mine && z < store_lim) s0[z * pos_stride] = v[z];
 }
 
 // The short-line kernel for length n, or null.
 template <typename T>
-using ColShortFn = void (*)(FftPlan, C<T>*, long long, const C<T>*, int, long long, long long, int, int, int, T,
-                            long long);
+using ColShortFn = void (*)(FftPlan, C<T>*, long long, const C<T>*, FastDiv, int, int, long long, long long, int, int,
+                            int, T, long long);
 template <typename T>
 ColShortFn<T> col_short_kernel(int n) {
   switch (n) {
@@ -1159,14 +1182,13 @@ __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&
 // The Metropolis decision for one cell from its neighbour values, its own m,
 // its demag field h and its proposal.  Shared by every sweep kernel so that
 // all paths round identically.
-// SEP (FP32): the products of the first two neighbours are rounded before they
-// are added, where the chain of multiply-adds rounds the second with the sum.
-// The vectorised forms have always taken the first of a thread's two cells this
-// way (see mc_sep), the others the chain; written out, it does not depend on
-// what the compiler makes of the code around.
+// SEP (FP32): in the components of this mask the second neighbour's product is
+// rounded before it is added, where the chain of multiply-adds rounds it with the
+// sum.  The scalar forms take the chain, the vectorised ones what mc_sep says;
+// written out, it does not depend on what the compiler makes of the code around.
 template <typename T>
 __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy,
-                                                  T hz, T px, T py, T pz, T ua, bool sep = false) {
+                                                  T hz, T px, T py, T pz, T ua, int sep = 0) {
   T Fx = 0, Fy = 0, Fz = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -1175,15 +1197,10 @@ __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs
       if (!nb.has[a][s]) continue;
       if constexpr (sizeof(T) == 4) {
         const float w = c.wex[a], x = nb.v[a][s][0], y = nb.v[a][s][1], z = nb.v[a][s][2];
-        if (sep && a == 0 && s == 1) {
-          Fx = __fadd_rn(Fx, __fmul_rn(w, x));
-          Fy = __fadd_rn(Fy, __fmul_rn(w, y));
-          Fz = __fadd_rn(Fz, __fmul_rn(w, z));
-        } else {
-          Fx = __fmaf_rn(w, x, Fx);
-          Fy = __fmaf_rn(w, y, Fy);
-          Fz = __fmaf_rn(w, z, Fz);
-        }
+        const bool second = a == 0 && s == 1;
+        Fx = second && (sep & 1) ? __fadd_rn(Fx, __fmul_rn(w, x)) : __fmaf_rn(w, x, Fx);
+        Fy = second && (sep & 2) ? __fadd_rn(Fy, __fmul_rn(w, y)) : __fmaf_rn(w, y, Fy);
+        Fz = second && (sep & 4) ? __fadd_rn(Fz, __fmul_rn(w, z)) : __fmaf_rn(w, z, Fz);
         continue;
       }
       Fx = Fx + c.wex[a] * nb.v[a][s][0];
@@ -1245,7 +1262,7 @@ __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs
 // The decision; p's direction is the new m where it is true.
 template <typename T>
 __device__ __forceinline__ bool mc_accept(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy, T hz,
-                                          const Proposal<T>& p, bool sep = false) {
+                                          const Proposal<T>& p, int sep = 0) {
   if constexpr (sizeof(T) == 8) {
     float v[3][2][3];
 #pragma unroll
@@ -1534,12 +1551,16 @@ __device__ __forceinline__ void st4(T* p, const Vec4<T>& r) {
   }
 }
 
-// Whether the vectorised forms round the first exchange products separately
-// (mc_accept_formula) for cell q of a thread's two: the first one, on thick
-// lattices with an open x or y axis only in the layer that has none above it.
+// The components whose second exchange product the vectorised forms round
+// separately (mc_accept_formula; bit 0 = x) for cell q of a thread's two, at x
+// offset p0 + 2 q of its u-th segment.  This is how these forms have rounded
+// from the beginning: one trial in 1e10 is decided by it, and it keeps a seed's
+// run the same.
 template <bool ALLB, bool Z3>
-__device__ __forceinline__ bool mc_sep(int q, bool hzu) {
-  return q == 0 && (!Z3 || ALLB || !hzu);
+__device__ __forceinline__ int mc_sep(int q, int u, int p0) {
+  if (q) return 0;
+  if (ALLB) return !Z3 || u == 1 ? 7 : p0;
+  return u == 1 || p0 == 0 ? 7 : Z3 ? 0 : 4;
 }
 
 // The decisions of the two cells at offsets P0 and P0 + 2 of a segment.
@@ -1551,7 +1572,7 @@ template <typename T, int P0, bool ALLB, bool Z3 = false>
 __device__ __forceinline__ bool quad_cells(const McCoef<T>& c, Vec4<T> (&own)[3], const Vec4<T> (&up)[3],
                                            const Vec4<T> (&dn)[3], const T (&lft)[3], const T (&rgt)[3],
                                            const Vec4<T> (&hh)[3], bool hl, bool hr, bool hd, bool hu,
-                                           uint32_t cell0, uint32_t stage, uint32_t sweep, unsigned int& mine,
+                                           uint32_t cell0, uint32_t stage, uint32_t sweep, unsigned int& mine, int u,
                                            const Vec4<T> (&zd)[3], const Vec4<T> (&zu)[3], bool hzd, bool hzu) {
   if constexpr (ALLB) hl = hr = hd = hu = true;
   if constexpr (!Z3) hzd = hzu = false;
@@ -1579,7 +1600,7 @@ __device__ __forceinline__ bool quad_cells(const McCoef<T>& c, Vec4<T> (&own)[3]
     }
     const Proposal<T> pr = mc_propose<T>(c, cell0 + (uint32_t)o, stage, sweep);
     if (mc_accept<T>(c, nb, own[0].v[o], own[1].v[o], own[2].v[o], hh[0].v[o], hh[1].v[o], hh[2].v[o], pr,
-                     mc_sep<ALLB, Z3>(q, hzu))) {
+                     mc_sep<ALLB, Z3>(q, u, P0))) {
       pr.get(own[0].v[o], own[1].v[o], own[2].v[o]);
       changed = true;
       ++mine;
@@ -1681,10 +1702,10 @@ __global__ void __launch_bounds__(256) k_mc_quad(Geom g, const McCoef<T>* __rest
       bool changed;
       if (p0 == 0)
         changed = quad_cells<T, 0, ALLB, Z3>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0),
-                                             ctr->stage, ctr->sweep, mine, zdn, zup, hzd, hzu);
+                                             ctr->stage, ctr->sweep, mine, u, zdn, zup, hzd, hzu);
       else
         changed = quad_cells<T, 1, ALLB, Z3>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0),
-                                             ctr->stage, ctr->sweep, mine, zdn, zup, hzd, hzu);
+                                             ctr->stage, ctr->sweep, mine, u, zdn, zup, hzd, hzu);
       if (changed) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) st4<T>(m + k * n + rowb + x0, own[k]);
@@ -1815,7 +1836,7 @@ __global__ void __launch_bounds__(MCSP_THREADS, 6) k_mc_split(Geom g, const McCo
       float& oy = q ? own[1].y : own[1].x;
       float& oz = q ? own[2].y : own[2].x;
       if (mc_accept<float>(c, nb, ox, oy, oz, q ? hh[0].y : hh[0].x, q ? hh[1].y : hh[1].x, q ? hh[2].y : hh[2].x,
-                           pr, mc_sep<ALLB, Z3>(q, hzu))) {
+                           pr, mc_sep<ALLB, Z3>(q, u, p))) {
         pr.get(ox, oy, oz);
         changed = true;
         ++mine;
@@ -1918,10 +1939,10 @@ __device__ __forceinline__ void band_segments(const Geom& g, const McCoef<T>& c,
     bool changed;
     if (p0 == 0)
       changed = quad_cells<T, 0, ALLB>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0), stage,
-                                       sweep, mine, own, own, false, false);
+                                       sweep, mine, 1, own, own, false, false);
     else
       changed = quad_cells<T, 1, ALLB>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0), stage,
-                                       sweep, mine, own, own, false, false);
+                                       sweep, mine, 1, own, own, false, false);
     if (changed) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) st4<T>(m + k * n + rowb + x0, own[k]);
@@ -2986,12 +3007,14 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
                          int planes, long long plane_stride, long long pos_stride, int load_lim, int store_lim,
                          int flags, T inv_n, int tx, int threads, cudaStream_t st, int nrep = 1,
                          long long s_rstride = 0, bool inl = false, bool lean = false, int regs = 0) {
-  if (ncomp == 3 && p.n <= 16 && p.full_off > 0) {  // short lines: one thread per column
+  if (ncomp == 3 && p.n <= 16 && p.full_off > 0) {  // short lines: one thread per column and component
     const ColShortFn<T> ks = col_short_kernel<T>(p.n);
-    if (ks) {
-      dim3 grid((hx + 127) / 128, planes, nrep);
-      return launch_pdl(ks, grid, dim3(128), 0, st, p, S, nspec, khat, hx, plane_stride, pos_stride, load_lim,
-                        store_lim, flags, inv_n, s_rstride);
+    constexpr int CSH_COLS = csh_cols<T>;
+    if (ks && (long long)hx * planes < INT_MAX - CSH_COLS) {
+      const int total = hx * planes;
+      dim3 grid((total + CSH_COLS - 1) / CSH_COLS, 1, nrep);
+      return launch_pdl(ks, grid, dim3(3 * CSH_COLS), 0, st, p, S, nspec, khat, FastDiv((uint32_t)hx), hx, total,
+                        plane_stride, pos_stride, load_lim, store_lim, flags, inv_n, s_rstride);
     }
   }
   if constexpr (__is_same(T, double)) {
