@@ -815,6 +815,80 @@ inline cudaError_t launch_col_pipe(const FftPlan& p, float2* S, long long nspec,
   return f(p, S, nspec, khat, hx, pitch, load_lim, store_lim, sym, inv_n, nrep, st);
 }
 
+// One direction of an FP32 transform along y (or z), without the product:
+// cl_tx columns of one component per CTA.  The lines go from global memory into
+// the registers in the order the transform takes them and back from them, so
+// shared memory is passed once, by the transpose, and the components and tiles
+// are CTAs of their own whose loads, transforms and stores overlap.
+// Bound by the latency of its loads with 16 warps per SM.  Against tiles of all
+// three components staged in shared memory (k_col_pass, k_col_pass_wide), the
+// demag field of a 512 x 512 x 8 slab: 97.9 -> 78.2 us, of 128 x 128 x 4 19.2 ->
+// 14.1 us, of 64 x 64 x 2 14.5 -> 11.8 us.  (16 columns at length 512: the same; 4:
+// 81 us; 5 CTAs per SM: 81 us.)
+template <int B>
+constexpr int cl_tx = B == 32 ? 4 : B == 16 ? 8 : 16;
+template <bool INV, int A, int B>
+__global__ void __launch_bounds__(cl_tx<B> * B, 4)
+    k_col_lines(const __grid_constant__ FftPlan p, float2* __restrict__ S, long long nspec, int hx,
+                long long plane_stride, long long pos_stride, int load_lim, int store_lim, long long s_rstride) {
+  constexpr int TX = cl_tx<B>, Q = A / B, RW = B * TX + TX / Q;  // transpose row: conflict-free both ways
+  __shared__ float2 reg[A * RW];
+  const int rep = blockIdx.z / 3, c = blockIdx.z - 3 * rep;
+  const int t = threadIdx.x & (TX - 1), b = threadIdx.x / TX, kx = blockIdx.x * TX + t;
+  const bool mine = kx < hx;
+  float2* s0 = S + rep * s_rstride + c * nspec + blockIdx.y * plane_stride + (mine ? kx : 0);
+  const float2* tw = p.tw32 + p.lane_off + b;
+  pdl_wait();
+  float2 v[A];
+#pragma unroll
+  for (int a = 0; a < A; ++a) {
+    const int pos = b + B * a;
+    v[a] = mine && pos < load_lim ? s0[pos * pos_stride] : make_float2(0.0f, 0.0f);
+  }
+  RegDft<float, INV, A>::run(v);
+#pragma unroll
+  for (int ka = 1; ka < A; ++ka) {
+    const float2 w = tw[ka * B];
+    v[ka] = INV ? tmulc(v[ka], w) : tmul(v[ka], w);
+  }
+#pragma unroll
+  for (int ka = 0; ka < A; ++ka) reg[ka * RW + b * TX + t] = v[ka];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+#pragma unroll
+    for (int bb = 0; bb < B; ++bb) v[q * B + bb] = reg[(b * Q + q) * RW + bb * TX + t];
+    RegDft<float, INV, B>::run(v + q * B);
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+#pragma unroll
+    for (int kb = 0; kb < B; ++kb) {
+      const int pos = b * Q + q + A * kb;
+      if (mine && pos < store_lim) s0[pos * pos_stride] = v[q * B + kb];
+    }
+}
+template <bool INV, int A, int B>
+cudaError_t launch_col_lines_ab(const FftPlan& p, float2* S, long long nspec, int hx, int planes,
+                                long long plane_stride, long long pos_stride, int load_lim, int store_lim,
+                                long long s_rstride, int nrep, cudaStream_t st) {
+  constexpr int TX = cl_tx<B>;
+  return launch_pdl(k_col_lines<INV, A, B>, dim3((hx + TX - 1) / TX, planes, 3 * nrep), dim3(TX * B), 0, st, p, S,
+                    nspec, hx, plane_stride, pos_stride, load_lim, store_lim, s_rstride);
+}
+template <bool INV>
+cudaError_t launch_col_lines(const FftPlan& p, float2* S, long long nspec, int hx, int planes, long long plane_stride,
+                             long long pos_stride, int load_lim, int store_lim, long long s_rstride, int nrep,
+                             cudaStream_t st) {
+  auto f = p.n == 1024  ? launch_col_lines_ab<INV, 32, 32>
+           : p.n == 512 ? launch_col_lines_ab<INV, 32, 16>
+           : p.n == 256 ? launch_col_lines_ab<INV, 16, 16>
+           : p.n == 128 ? launch_col_lines_ab<INV, 16, 8>
+           : p.n == 64  ? launch_col_lines_ab<INV, 8, 8>
+                        : launch_col_lines_ab<INV, 8, 4>;
+  return f(p, S, nspec, hx, planes, plane_stride, pos_stride, load_lim, store_lim, s_rstride, nrep, st);
+}
+
 // Column pass for short lines (n <= 16: the padded z axis of thin 3-D
 // lattices, short y axes): csh_cols columns (kx, plane) per CTA, one thread per
 // column and component with the line in registers, transformed by ThreadDft.
@@ -3027,6 +3101,11 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
     }
   }
   if constexpr (sizeof(T) == 4) {
+    if (ncomp == 3 && p.warp_a && (flags == PASS_FWD || flags == PASS_INV) && planes <= 65535 && nrep <= 21845)
+      return flags == PASS_FWD ? launch_col_lines<false>(p, S, nspec, hx, planes, plane_stride, pos_stride, load_lim,
+                                                         store_lim, s_rstride, nrep, st)
+                               : launch_col_lines<true>(p, S, nspec, hx, planes, plane_stride, pos_stride, load_lim,
+                                                        store_lim, s_rstride, nrep, st);
     if (regs && ncomp == 3 && planes == 1 && (flags & ~PASS_SYM) == (PASS_FWD | PASS_MUL | PASS_INV) &&
         pos_stride < (1LL << 31) && (nrep == 1 || s_rstride == 3 * nspec) && col_pipe_ok(p))
       return launch_col_pipe(p, S, nspec, khat, hx, (int)pos_stride, load_lim, store_lim, (flags & PASS_SYM) ? 1 : 0,
