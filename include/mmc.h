@@ -226,7 +226,10 @@ int mmc_compute_demag(mmc_handle* h);
  * handle's tensor spectrum.  mdev and hdev hold 3*nx*ny*nz values of the
  * handle's precision (float for precision 32, double for 64), SoA, x fastest;
  * hdev is dimensionless (H_demag = ms * hdev).  scratch is a caller-owned
- * device buffer of at least mmc_demag_scratch_bytes() bytes.  The work is
+ * device buffer of at least mmc_demag_scratch_bytes() bytes, aligned to a
+ * complex value (8 bytes for precision 32, 16 for 64; MMC_ERR_INVALID
+ * otherwise); on 16 bytes, FP32 films with y lengths of 32 to 256 take the
+ * faster column pass (the results are the same bits).  The work is
  * enqueued on `stream` (a cudaStream_t; NULL means the handle's stream) and
  * the call returns without synchronising. */
 int mmc_demag_scratch_bytes(mmc_handle* h, size_t* bytes);

@@ -3107,7 +3107,8 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
                                : launch_col_lines<true>(p, S, nspec, hx, planes, plane_stride, pos_stride, load_lim,
                                                         store_lim, s_rstride, nrep, st);
     if (regs && ncomp == 3 && planes == 1 && (flags & ~PASS_SYM) == (PASS_FWD | PASS_MUL | PASS_INV) &&
-        pos_stride < (1LL << 31) && (nrep == 1 || s_rstride == 3 * nspec) && col_pipe_ok(p))
+        pos_stride < (1LL << 31) && (nrep == 1 || s_rstride == 3 * nspec) && col_pipe_ok(p) &&
+        (reinterpret_cast<uintptr_t>(S) & 15) == 0)  // its copies are of 16 bytes; a caller's scratch may lie on 8
       return launch_col_pipe(p, S, nspec, khat, hx, (int)pos_stride, load_lim, store_lim, (flags & PASS_SYM) ? 1 : 0,
                              inv_n, nrep, st);
   }

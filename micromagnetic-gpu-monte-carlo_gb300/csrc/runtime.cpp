@@ -2317,6 +2317,8 @@ int mmc_demag_apply(mmc_handle* h, const void* mdev, void* hdev, void* scratch, 
   if (!h || !mdev || !hdev || !scratch) return fail(MMC_ERR_INVALID, "null argument");
   if (!h->cfg.cal_demag_flag) return fail(MMC_ERR_STATE, "cal_demag_flag is off");
   if (scratch_bytes < 3 * (size_t)h->g.nspec * 2 * h->tsize) return fail(MMC_ERR_INVALID, "scratch too small");
+  if (reinterpret_cast<uintptr_t>(scratch) % (2 * h->tsize))
+    return fail(MMC_ERR_INVALID, "scratch must be aligned to a complex value (8 bytes for precision 32, 16 for 64)");
   TRY(set_dev(h));
   TRY(ensure_demag(h));
   cudaStream_t st = stream ? (cudaStream_t)stream : h->st;
