@@ -405,13 +405,20 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
  * transform in place reading the tensor from global memory (1; 2 and 3 the
  * same, with FP32 film y lines of length 32 to 256 by the pipelined pass, other
  * lines as 1),
- * and the number of streams (1-4) the batch's replicas are split over. */
+ * and the number of streams (1-4) the batch's replicas are split over.  Some
+ * passes have shapes of their own and do not read a setting: the pipelined
+ * pass and the y passes of FP32 3-D lattices with power-of-two y transforms of
+ * 32 to 1024 the columns and threads, FP32 x passes of such lengths the in-line
+ * flag, FP64 passes of such lengths all of them, and films the columns of the z
+ * pass.  Every shape reported here or chosen by the autotuner is one that
+ * mmc_batch_set_launch_shape accepts. */
 int mmc_batch_launch_shape(mmc_batch* b, int out[10]);
-/* Autotuner: times each launch shape this batch can run with (the film row
+/* Autotuner: times the launch shapes this batch can run with (the film row
  * kernel with each band that fits; the pass kernels with 1-16 rows per x-pass
  * CTA and 1-8 kx columns per column-pass tile, then -- one dimension at a
- * time from the fastest so far -- the transforms in and out of line, the
- * in-place column passes, every Metropolis form, 2-4 streams) for `sweeps`
+ * time from the fastest so far -- the other column-pass forms, the transforms
+ * in and out of line, every Metropolis form, 2-4 streams; settings that none
+ * of a shape's kernels read are not varied) for `sweeps`
  * sweeps (the faster of two repetitions; replays of the 32-sweep graph that
  * runs execute, so `sweeps` is rounded up to a multiple of 32) from the
  * current state, keeps the fastest and restores m and the acceptance

@@ -294,7 +294,7 @@ DemagTuning choose_tuning(const Geom& g, const FftPlan& px, const FftPlan& py, c
     return tx;
   };
   t.col_tx = pick(py, g.nzp == 1 ? 1 : g.nz, g.nzp == 1);
-  t.col_tx_z = pick(pz, g.nyp, true);
+  t.col_tx_z = g.nzp == 1 ? t.col_tx : pick(pz, g.nyp, true);  // (films have no z pass)
   t.col_threads = col_threads_for(g, py, pz, t.col_tx, t.col_tx_z);
   // FP32 with at least 8 x 256^2 trials per launch (batches of 8 films, a
   // 512x512x8 slab): the vectorised per-colour sweep, measured faster there
@@ -1863,6 +1863,28 @@ int batch_run(mmc_batch* b, long long stage, long long sweep0, long long nsweeps
   return batch_run_abandon(b, status);
 }
 
+// Whether the kernels take a launch shape (mmc_batch_set_launch_shape's rule
+// but for the band and the streams).
+bool batch_shape_ok(const mmc_batch* b, const DemagTuning& t, int band) {
+  const mmc_handle* h = b->base;
+  const Geom& g = h->g;
+  const size_t cs = 2 * h->tsize;
+  auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
+  return !(!pow2(t.x_rows_per_cta) || t.x_rows_per_cta > 16 ||
+           x_pass_smem(h->px.p, t.x_rows_per_cta, cs) > smem_limit() || !pow2(t.col_tx) || t.col_tx > 64 ||
+           col_pass_smem(h->py.p, t.col_tx, cs, t.col_lean != 0) > smem_limit() || !pow2(t.col_tx_z) ||
+           t.col_tx_z > 64 || col_pass_smem(h->pz.p, t.col_tx_z, cs, t.col_lean != 0) > smem_limit() ||
+           t.col_threads % t.col_tx != 0 || t.col_threads % t.col_tx_z != 0 ||
+           (t.x_threads != 128 && t.x_threads != 256) || t.col_threads < 32 || t.col_threads > 512 ||
+           t.col_threads % 32 != 0 || t.mc_form < MC_FORM_SCALAR || t.mc_form > MC_FORM_PIPE ||
+           (t.mc_form == MC_FORM_TILE && !mc_tile_eligible(g)) || (t.mc_form == MC_FORM_QUAD && !mc_quad_eligible(g)) ||
+           (t.mc_form == MC_FORM_BAND && !mc_band_eligible(g)) ||
+           (t.mc_form == MC_FORM_STRIP && (!mc_strip_eligible(g) || band != 0 ||
+                                           mc_strip_smem_bytes(g, h->tsize) > smem_limit())) ||
+           (t.mc_form == MC_FORM_PIPE && (!mc_pipe_eligible(g) || mc_pipe_smem_bytes(g, h->tsize) > smem_limit())) ||
+           (t.fft_inline != 0 && t.fft_inline != 1) || t.col_lean < 0 || t.col_lean > 3);
+}
+
 // Times every launch shape the batch can run with -- the row kernel with each
 // band that fits, the pass kernels with each x-pass row count and column-pass
 // width -- for `sweeps` sweeps from the current state, keeps the fastest and
@@ -1895,6 +1917,8 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
   // times one candidate from the saved state; keeps it when it is the fastest
   auto trial = [&](const Cand& cd) {
     if (e != cudaSuccess || status != MMC_OK) return;
+    // a shape that could not be set again is no candidate (the first one is what the batch has)
+    if (tried && !batch_shape_ok(b, cd.tun, cd.rows_band)) return;
     if (cd.rows_band > 0 && (status = batch_alloc_rows(b)) != MMC_OK) return;
     if (cd.streams > 1 && (status = batch_alloc_streams(b)) != MMC_OK) return;
     if (cd.tun.mc_form == MC_FORM_STRIP && (status = batch_alloc_m2(b)) != MMC_OK) return;
@@ -1933,50 +1957,69 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
     }
   };
   // coordinate search: the pass-kernel tiling first, then one dimension at a
-  // time from the best so far; the row kernel bands are whole alternatives
+  // time from the best so far; the row kernel bands are whole alternatives.
+  // A setting that no kernel of the shape reads is left as it is: the FP64
+  // passes of power-of-two lengths have shapes of their own (lines64.cuh), and so
+  // has the pipelined column pass.
+  const bool film = g.nzp == 1, own64 = h->prec == 64;
+  const bool pipe = !own64 && film && col_pipe_eligible(h->py.p);
+  auto general_cols = [&](const DemagTuning& t) {  // whether a column pass reads col_tx or col_threads
+    if (h->py.p.warp_a == 0) return true;
+    return !own64 && (film ? !(pipe && t.col_lean >= 2) : h->pz.p.warp_a != 0);
+  };
+  auto with_tx = [&](DemagTuning t, int tx) {
+    t.col_tx = tx;
+    if (film) t.col_tx_z = tx;
+    t.col_threads = col_threads_for(g, h->py.p, h->pz.p, tx, t.col_tx_z);
+    return t;
+  };
   trial({0, base});
   if (h->cfg.cal_demag_flag) {
     const long long rows = (long long)g.ny * g.nz;
     for (int r : {1, 2, 4, 8, 16}) {
       if (r > rows || x_pass_smem(h->px.p, r, cs) > smem_limit()) continue;
+      if (own64 && h->px.p.warp_a && r != base.x_rows_per_cta) continue;
       for (int tx : {1, 2, 4, 8}) {
+        if (!general_cols(base) && tx != 1) break;
         // a tile the copying form cannot hold is tried in place
         const bool fits = col_pass_smem(h->py.p, tx, cs, base.col_lean != 0) <= smem_limit();
         const bool fits_lean = col_pass_smem(h->py.p, tx, cs, true) <= smem_limit();
         if (tx > g.hx || !(fits || fits_lean)) continue;
-        if (r == base.x_rows_per_cta && tx == base.col_tx) continue;
-        DemagTuning t = base;
+        DemagTuning t = general_cols(base) ? with_tx(base, tx) : base;
         t.x_rows_per_cta = r;
-        t.col_tx = tx;
+        if (r == base.x_rows_per_cta && t.col_tx == base.col_tx) continue;
         if (!fits) t.col_lean = 1;
-        t.col_threads = col_threads_for(g, h->py.p, h->pz.p, tx, t.col_tx_z);
         trial({0, t});
       }
     }
-    Cand c = best;
-    c.tun.fft_inline = 1 - c.tun.fft_inline;
-    trial(c);
-    // the other column-pass form (in place or with copies) with the full and
-    // half thread count, and the half thread count of the current form
-    if (h->py.p.warp_a) {
+    // the other column-pass forms (with copies, in place, pipelined), the first
+    // two with the full and the half thread count, and with each width where the
+    // grid above left it alone
+    if (!own64 && (film ? h->py.p.warp_a : h->pz.p.warp_a)) {
       const Cand cur = best;
-      for (int flip = 0; flip < 2; ++flip)
-        for (int half = 0; half < 2; ++half) {
-          if (!flip && !half) continue;
-          Cand d = cur;
-          if (flip) d.tun.col_lean = 1 - cur.tun.col_lean;
-          if (half) d.tun.col_threads = std::max(64, cur.tun.col_threads / 2);
-          if (half && d.tun.col_threads == cur.tun.col_threads) continue;
-          if (col_pass_smem(h->py.p, d.tun.col_tx, cs, d.tun.col_lean != 0) > smem_limit()) continue;
-          trial(d);
-        }
+      const bool widths_left = film && !general_cols(cur.tun);
+      for (int form = 0; form <= (pipe ? 2 : 1); ++form) {
+        std::vector<int> widths{cur.tun.col_tx};
+        if (form < 2 && widths_left) widths = {1, 2, 4, 8};
+        for (int tx : widths)
+          for (int half = 0; half < (form == 2 ? 1 : 2); ++half) {
+            if (tx > g.hx || (form == cur.tun.col_lean && !half)) continue;
+            Cand d = cur;
+            if (tx != cur.tun.col_tx) d.tun = with_tx(cur.tun, tx);
+            d.tun.col_lean = form;
+            const int full = d.tun.col_threads;
+            if (half) d.tun.col_threads = std::max(64, full / 2);
+            if (half && d.tun.col_threads == full) continue;
+            trial(d);
+          }
+      }
     }
-  }
-  // the pipelined film column pass (FP32, y lengths 32 to 256)
-  if (h->cfg.cal_demag_flag && h->prec == 32 && g.nzp == 1 && col_pipe_eligible(h->py.p) && best.tun.col_lean < 2) {
-    Cand c = best;
-    c.tun.col_lean = 2;
-    trial(c);
+    // in-line transforms, where a warp-shaped line runs in a general column pass
+    if (!own64 && (film ? h->py.p.warp_a && general_cols(best.tun) : h->pz.p.warp_a != 0)) {
+      Cand c = best;
+      c.tun.fft_inline = 1 - c.tun.fft_inline;
+      trial(c);
+    }
   }
   {
     std::vector<int> forms;
@@ -2007,6 +2050,7 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
       Cand c = best;
       c.rows_band = bd;
       c.streams = 1;
+      if (c.tun.mc_form == MC_FORM_STRIP) c.tun.mc_form = base.mc_form;  // (the row kernel sweeps by itself)
       trial(c);
     }
   if (e == cudaSuccess && status == MMC_OK && best_t >= 0) {
@@ -2661,31 +2705,14 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
 
 int mmc_batch_set_launch_shape(mmc_batch* b, const int shape[10]) {
   if (!b || !shape) return fail(MMC_ERR_INVALID, "null argument");
-  mmc_handle* h = b->base;
-  const Geom& g = h->g;
-  const size_t cs = 2 * h->tsize;
   DemagTuning t{shape[0], shape[1], shape[2], shape[3], shape[4], shape[6], shape[7], shape[8]};
   const int streams = shape[9];
   if (streams < 1 || streams > 4) return fail(MMC_ERR_INVALID, "streams must be in [1, 4]");
   const int band = shape[5];
-  auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
-  if (!pow2(t.x_rows_per_cta) || t.x_rows_per_cta > 16 || x_pass_smem(h->px.p, t.x_rows_per_cta, cs) > smem_limit() ||
-      !pow2(t.col_tx) || t.col_tx > 64 || col_pass_smem(h->py.p, t.col_tx, cs, t.col_lean != 0) > smem_limit() ||
-      !pow2(t.col_tx_z) || t.col_tx_z > 64 || col_pass_smem(h->pz.p, t.col_tx_z, cs, t.col_lean != 0) > smem_limit() ||
-      t.col_threads % t.col_tx != 0 ||
-      t.col_threads % t.col_tx_z != 0 ||
-      (t.x_threads != 128 && t.x_threads != 256) || t.col_threads < 32 || t.col_threads > 512 ||
-      t.col_threads % 32 != 0 || t.mc_form < MC_FORM_SCALAR || t.mc_form > MC_FORM_PIPE ||
-      (t.mc_form == MC_FORM_TILE && !mc_tile_eligible(g)) || (t.mc_form == MC_FORM_QUAD && !mc_quad_eligible(g)) ||
-      (t.mc_form == MC_FORM_BAND && !mc_band_eligible(g)) ||
-      (t.mc_form == MC_FORM_STRIP && (!mc_strip_eligible(g) || shape[5] != 0 ||
-                                      mc_strip_smem_bytes(g, h->tsize) > smem_limit())) ||
-      (t.mc_form == MC_FORM_PIPE && (!mc_pipe_eligible(g) || mc_pipe_smem_bytes(g, h->tsize) > smem_limit())) ||
-      (t.fft_inline != 0 && t.fft_inline != 1) || t.col_lean < 0 || t.col_lean > 3)
-    return fail(MMC_ERR_INVALID, "launch shape outside the supported range");
+  if (!batch_shape_ok(b, t, band)) return fail(MMC_ERR_INVALID, "launch shape outside the supported range");
   if (band != 0 && std::find(b->row_bands.begin(), b->row_bands.end(), band) == b->row_bands.end())
     return fail(MMC_ERR_UNSUPPORTED, "row-kernel band not available for this batch");
-  TRY(set_dev(h));
+  TRY(set_dev(b->base));
   if (band > 0) TRY(batch_alloc_rows(b));
   if (streams > 1) TRY(batch_alloc_streams(b));
   if (t.mc_form == MC_FORM_STRIP) TRY(batch_alloc_m2(b));
