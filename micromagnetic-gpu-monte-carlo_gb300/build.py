@@ -70,10 +70,13 @@ def _compile(unit):
     src, extra, comp = unit
     obj = os.path.join(BUILD, src + ".o")
     if comp == "nvcc":
-        cmd = [NVCC] + NVCC_COMMON + extra + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [NVCC] + NVCC_COMMON + ["-Xptxas", "-v"] + extra + ["-c", os.path.join(CSRC, src), "-o", obj]
     else:
         cmd = GXX_COMMON + extra + ["-c", os.path.join(CSRC, src), "-o", obj]
-    _run(cmd)
+    text = _run(cmd)
+    if comp == "nvcc":  # each kernel's registers and spills
+        with open(obj + ".ptxas", "w") as f:
+            f.write(text)
     return obj
 
 

@@ -270,10 +270,24 @@ __device__ __forceinline__ void odd_stages(const C<T>* src, C<T>* dst, int total
   }
 }
 
+// Whether a plan has a stage for odd_stage.
+inline bool plan_odd(const FftPlan& p) {
+  for (int s = 0; s < p.nstages; ++s)
+    if (p.radix[s] >= 7) return true;
+  return false;
+}
+
 // Transforms `nlines` lines of length p.n; line l starts at buf + l*stride.
 // `a` holds the input, `b` is scratch of the same shape.  Returns the buffer
 // holding the result (a or b).  All threads of the block must call it.
-template <typename T, bool INV>
+// ODD: the length may have radices of 7 and above (plan_odd).  Their stages keep
+// up to 31 values in registers and a kernel's register allocation covers
+// everything it calls, so only kernels instantiated with ODD contain them and
+// only plans that need them reach those: with them in every kernel, k_rows<float>
+// took 203 registers instead of 128 and k_col_pass<float> 127 instead of 70; us
+// per sweep with / without them: 8 x 96^2 films 32.2 / 25.1 in FP32, 93.0 / 76.8 in
+// FP64, 16 x 128^2 by the row kernel in bands of 2 57.3 / 37.5.
+template <typename T, bool INV, bool ODD>
 __device__ __noinline__ C<T>* fft_lines(C<T>* a, C<T>* b, int nlines, int stride, const FftPlan& p,
                                         const C<T>* tw) {
   using V = C<T>;
@@ -285,8 +299,10 @@ __device__ __noinline__ C<T>* fft_lines(C<T>* a, C<T>* b, int nlines, int stride
     const FastDiv dnb = p.dnb[s], dns = p.dns[s];
     const V* W = tw + p.tw_off[s];
     const int total = nlines * nb;
-    if (R >= 7) odd_stages<T, INV>(src, dst, total, stride, R, nb, Ns, dnb, dns, W, plan_tw<T>(p) + p.odd_off[s]);
-    for (int idx = threadIdx.x; R < 7 && idx < total; idx += blockDim.x) {
+    if constexpr (ODD) {
+      if (R >= 7) odd_stages<T, INV>(src, dst, total, stride, R, nb, Ns, dnb, dns, W, plan_tw<T>(p) + p.odd_off[s]);
+    }
+    for (int idx = threadIdx.x; (!ODD || R < 7) && idx < total; idx += blockDim.x) {
       const int line = dnb.div(idx);
       const int j = idx - line * nb;
       const int k = j - dns.div(j) * Ns;
@@ -702,7 +718,8 @@ __device__ __forceinline__ void fft_wide(C<T>* a, int nlines, int stride, const 
   __syncthreads();
 }
 
-template <typename T, bool INV, bool INL = false, bool WIDE = false, bool PAD = false>
+// (ODD: see fft_lines.)
+template <typename T, bool INV, bool ODD, bool INL = false, bool WIDE = false, bool PAD = false>
 __device__ C<T>* fft_run(C<T>* a, C<T>* b, int nlines, int stride, const FftPlan& p, const C<T>* tw) {
   if constexpr (WIDE) {
     if (p.warp_a == 32) {
@@ -725,7 +742,7 @@ __device__ C<T>* fft_run(C<T>* a, C<T>* b, int nlines, int stride, const FftPlan
   } else if (p.warp_a == 8 && p.warp_b == 4) {
     fft_warp_call<T, INV, 8, 4, INL, PAD>(a, nlines, stride, tw + p.full_off);
   } else {
-    return fft_lines<T, INV>(a, b, nlines, stride, p, tw);
+    return fft_lines<T, INV, ODD>(a, b, nlines, stride, p, tw);
   }
   __syncthreads();
   return a;

@@ -135,6 +135,8 @@ __host__ __device__ inline Fused2DLayout fused2d_layout(const Geom& g, const Fft
   return L;
 }
 
+// (One instance, with the odd stages of fft_lines: the kernel takes 255 registers
+// and one CTA per SM either way, and without them it spills more: 2-3 % slower.)
 template <typename T>
 __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_constant__ Fused2D<T> P) {
   using V = C<T>;
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_const
         fa[(size_t)line * (Ly + 1) + pos] = pos < ny ? colraw[((size_t)cc * ny + pos) * 2 + t] : cmk<V>(0, 0);
       }
       __syncthreads();
-      V* cur = fft_run<T, false>(fa, fb, 6, Ly + 1, P.py, twy);
+      V* cur = fft_run<T, false, true>(fa, fb, 6, Ly + 1, P.py, twy);
       V* oth = cur == fa ? fb : fa;
       for (int idx = threadIdx.x; idx < 2 * Ly; idx += blockDim.x) {
         const int t = P.py.dn.div(idx), pos = idx - t * Ly;
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_const
         *qz = cmk<V>(hz_.x * P.inv_n, hz_.y * P.inv_n);
       }
       __syncthreads();
-      V* r = fft_run<T, true>(cur, oth, 6, Ly + 1, P.py, twy);
+      V* r = fft_run<T, true, true>(cur, oth, 6, Ly + 1, P.py, twy);
       for (int idx = threadIdx.x; idx < 3 * ny; idx += blockDim.x) {
         const int cc = g.dny.div(idx), y = idx - cc * ny;
         V* dst = S + cc * nspec + (long long)y * hxp + kx0;
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_const
     __syncthreads();
   }
   R.So = P.S;
-  row_forward<T>(R);
+  row_forward<T, true>(R);
   if (!grid_sync(P.bar, target, &s_flag)) return;
   column_phase(-1, P.S);
   if (!grid_sync(P.bar, target, &s_flag)) return;
@@ -282,13 +284,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_fused2d(const __grid_const
     stamp(sw, 0);
     row_load<T>(R, c, P.stage, sweep, sw == 0);  // later sweeps' proposals were made during barrier 2
     stamp(sw, 1);
-    row_field<T>(R);
+    row_field<T, true>(R);
     stamp(sw, 2);
     my_acc += row_sweep<T>(R, c);
     stamp(sw, 3);
     row_store<T>(R, last);
     if (last) break;
-    row_forward<T>(R);
+    row_forward<T, true>(R);
     stamp(sw, 4);
     if (!grid_sync(P.bar, target, &s_flag)) return;
     stamp(sw, 5);
@@ -376,11 +378,17 @@ size_t rows_smem_bytes(const Geom& g, const FftPlan& px, int band) {
 }
 
 template <typename T>
+auto rows_kernel(const FftPlan& px) {
+  return plan_odd(px) ? k_rows<T, true> : k_rows<T, false>;
+}
+
+template <typename T>
 cudaError_t rows_prepare(const Geom& g, const FftPlan& px, int band, int* blocks_per_sm) {
   const size_t smem = rows_smem_bytes<T>(g, px, band);
-  cudaError_t e = raise_smem_limit((const void*)k_rows<T>);
+  const void* kern = (const void*)rows_kernel<T>(px);
+  cudaError_t e = raise_smem_limit(kern);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, (const void*)k_rows<T>, 256, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, 256, smem);
 }
 
 template <typename T>
@@ -390,9 +398,9 @@ cudaError_t launch_rows(const Geom& g, const FftPlan& px, const McCoef<T>* coef,
   if (m == mo || spec == spec_out) return cudaErrorInvalidValue;  // halo rows must not be overwritten
   const size_t smem = rows_smem_bytes<T>(g, px, band);
   dim3 grid((g.ny + band - 1) / band, 1, nrep);
-  k_rows<T><<<grid, 256, smem, st>>>(g, px, coef, m, mo, h, reinterpret_cast<const C<T>*>(spec),
-                                     reinterpret_cast<C<T>*>(spec_out), acc, ctr, band, with_h ? 1 : 0,
-                                     do_forward ? 1 : 0);
+  rows_kernel<T>(px)<<<grid, 256, smem, st>>>(g, px, coef, m, mo, h, reinterpret_cast<const C<T>*>(spec),
+                                              reinterpret_cast<C<T>*>(spec_out), acc, ctr, band, with_h ? 1 : 0,
+                                              do_forward ? 1 : 0);
   return cudaGetLastError();
 }
 

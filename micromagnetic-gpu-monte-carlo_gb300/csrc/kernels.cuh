@@ -64,9 +64,18 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Real rows in[c][row][x] (x < xdata, zero up to p.n) -> S[c][z][y][kx], kx < hx.
 // NC: components (3 for m, 6 for the tensor), fixed at compile time so the
-// per-element work covers only the components that exist.
-template <typename T, bool INL, int NC>
-__global__ void k_x_forward(FftPlan p, int xdata, FastDiv dyd, int nrows, const T* __restrict__ in,
+// per-element work covers only the components that exist.  Three components
+// come in lengths without a warp-level plan only (k_x_forward_w and its like take
+// those).  ODD: see fft_lines.
+// (Register budget in FP32: 64 per thread, 128 with the odd stages, whose 130
+// left three CTAs of 128 threads per SM instead of four: 211 us for the demag
+// field of an open 512^2 film instead of 199.)
+template <typename T, bool ODD>
+constexpr int x_min_blocks() {
+  return sizeof(T) == 8 ? 1 : ODD ? 2 : 4;
+}
+template <typename T, int NC, bool ODD>
+__global__ void __launch_bounds__(256, x_min_blocks<T, ODD>()) k_x_forward(FftPlan p, int xdata, FastDiv dyd, int nrows, const T* __restrict__ in,
                             long long in_cstride, C<T>* __restrict__ S, long long nspec, int nyp, FastDiv dhx,
                             int pitch, int rows_per_cta, long long in_rstride, long long s_rstride) {
   constexpr int ncomp = NC;
@@ -109,7 +118,11 @@ __global__ void k_x_forward(FftPlan p, int xdata, FastDiv dyd, int nrows, const 
     }
   }
   __syncthreads();
-  V* res = fft_run<T, false, INL, NC == 6>(bufA, bufB, nr * npairs, L, p, tw);
+  V* res;
+  if constexpr (NC == 6)
+    res = fft_run<T, false, ODD, false, true>(bufA, bufB, nr * npairs, L, p, tw);
+  else
+    res = fft_lines<T, false, ODD>(bufA, bufB, nr * npairs, L, p, tw);
   for (int idx = threadIdx.x; idx < nr * npairs * hx; idx += blockDim.x) {
     const int rest = dhx.div(idx);
     const int k = idx - rest * hx;
@@ -127,8 +140,8 @@ __global__ void k_x_forward(FftPlan p, int xdata, FastDiv dyd, int nrows, const 
 }
 
 // Half spectra S[0..2][z][y][kx] -> real rows out[c][row][x], x < xout.
-template <typename T, bool INL>
-__global__ void k_x_inverse(FftPlan p, const C<T>* __restrict__ S, long long nspec, int nyp, int hx, int pitch,
+template <typename T, bool ODD>
+__global__ void __launch_bounds__(256, x_min_blocks<T, ODD>()) k_x_inverse(FftPlan p, const C<T>* __restrict__ S, long long nspec, int nyp, int hx, int pitch,
                             FastDiv dxo, FastDiv dyo, int nrows, T* __restrict__ out, long long out_cstride,
                             int rows_per_cta, long long s_rstride, long long out_rstride) {
   const int xout = (int)dxo.d, yout = (int)dyo.d;
@@ -173,7 +186,7 @@ __global__ void k_x_inverse(FftPlan p, const C<T>* __restrict__ S, long long nsp
     }
   }
   __syncthreads();
-  V* res = fft_run<T, true, INL>(bufA, bufB, nr * 2, L, p, tw);
+  V* res = fft_lines<T, true, ODD>(bufA, bufB, nr * 2, L, p, tw);
   for (int idx = threadIdx.x; idx < nr * xout; idx += blockDim.x) {
     const int rr = dxo.div(idx), x = idx - rr * xout;
     const long long o = (long long)(row0 + rr) * xout + x;
@@ -495,7 +508,7 @@ enum : int { PASS_FWD = 1, PASS_MUL = 2, PASS_INV = 4, PASS_SYM = 8 };
 // pos*pos_stride + kx0 + col].  Loads pos < load_lim (zero above), stores
 // pos < store_lim.  With PASS_MUL the tile is multiplied by the symmetric
 // tensor spectrum (K^ . M^ / N, calHexchangeKernel) between the transforms.
-template <typename T, bool INL, bool WIDE>
+template <typename T, bool INL, bool WIDE, bool ODD>
 __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>* __restrict__ S, long long nspec,
                                               const C<T>* __restrict__ khat, int hx, long long plane_stride,
                                               long long pos_stride, int load_lim, int store_lim, int flags, T inv_n,
@@ -573,7 +586,7 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
   if (flags & PASS_FWD) {
     V* r = cur;
     if constexpr (WIDE) fft_wide<T, false, INL, true>(cur, nlines, stride, p, tw);
-    else r = fft_run<T, false, INL, false, true>(cur, oth, nlines, stride, p, tw);
+    else r = fft_run<T, false, ODD, INL, false, true>(cur, oth, nlines, stride, p, tw);
     if (r != cur) {
       oth = cur;
       cur = r;
@@ -604,7 +617,7 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
   if (flags & PASS_INV) {
     V* r = cur;
     if constexpr (WIDE) fft_wide<T, true, INL, true>(cur, nlines, stride, p, tw);
-    else r = fft_run<T, true, INL, false, true>(cur, oth, nlines, stride, p, tw);
+    else r = fft_run<T, true, ODD, INL, false, true>(cur, oth, nlines, stride, p, tw);
     if (r != cur) {
       oth = cur;
       cur = r;
@@ -619,11 +632,11 @@ __device__ __forceinline__ void col_pass_body(const FftPlan& p, int ncomp, C<T>*
   }
 }
 
-template <typename T, bool INL>
+template <typename T, bool INL, bool ODD>
 __global__ void k_col_pass(FftPlan p, int ncomp, C<T>* __restrict__ S, long long nspec,
                            const C<T>* __restrict__ khat, int hx, long long plane_stride, long long pos_stride,
                            int load_lim, int store_lim, int flags, T inv_n, int tx, long long s_rstride, int lean) {
-  col_pass_body<T, INL, false>(p, ncomp, S, nspec, khat, hx, plane_stride, pos_stride, load_lim, store_lim, flags,
+  col_pass_body<T, INL, false, ODD>(p, ncomp, S, nspec, khat, hx, plane_stride, pos_stride, load_lim, store_lim, flags,
                                inv_n, tx, s_rstride, lean);
 }
 // The same for the 32-value warp shapes (lengths 512 and 1024), at most 256
@@ -633,7 +646,7 @@ __global__ void __launch_bounds__(256) k_col_pass_wide(FftPlan p, int ncomp, C<T
                                                        const C<T>* __restrict__ khat, int hx, long long plane_stride,
                                                        long long pos_stride, int load_lim, int store_lim, int flags,
                                                        T inv_n, int tx, long long s_rstride, int lean) {
-  col_pass_body<T, INL, true>(p, ncomp, S, nspec, khat, hx, plane_stride, pos_stride, load_lim, store_lim, flags,
+  col_pass_body<T, INL, true, false>(p, ncomp, S, nspec, khat, hx, plane_stride, pos_stride, load_lim, store_lim, flags,
                               inv_n, tx, s_rstride, lean);
 }
 
@@ -2984,16 +2997,17 @@ inline size_t x_pass_w_smem(const FftPlan& p, int rows, int threads, size_t csiz
 // inside a stream capture.
 template <typename T>
 cudaError_t prepare_passes(int max_dyn_smem) {
-  const void* fns[] = {(const void*)k_x_forward<T, false, 3>, (const void*)k_x_forward<T, true, 3>,
-                       (const void*)k_x_inverse<T, false>,    (const void*)k_x_inverse<T, true>,
-                       (const void*)k_col_pass<T, false>,     (const void*)k_col_pass<T, true>};
+  const void* fns[] = {(const void*)k_x_forward<T, 3, false>,    (const void*)k_x_forward<T, 3, true>,
+                       (const void*)k_x_inverse<T, false>,       (const void*)k_x_inverse<T, true>,
+                       (const void*)k_col_pass<T, false, false>, (const void*)k_col_pass<T, true, false>,
+                       (const void*)k_col_pass<T, false, true>};
   for (const void* f : fns) MMC_TRY_ATTR(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
   if constexpr (__is_same(T, double)) return l64_prepare(max_dyn_smem);
   else {
     const void* wide[] = {(const void*)k_col_pass_wide<T, false>, (const void*)k_col_pass_wide<T, true>};
     for (const void* f : wide) MMC_TRY_ATTR(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
     if constexpr (__is_same(T, f64s))  // the tensor's six blocks
-      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_x_forward<T, false, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
+      MMC_TRY_ATTR(cudaFuncSetAttribute((const void*)k_x_forward<T, 6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem));
     for (int s = 0; s < 7; ++s) {
       FftPlan p{};
       const int ab[7][2] = {{32, 32}, {32, 16}, {16, 16}, {16, 8}, {8, 8}, {16, 2}, {8, 4}};
@@ -3047,7 +3061,7 @@ template <typename T>
 cudaError_t run_x_forward(const FftPlan& p, int ncomp, int xdata, int ydata, int nrows, const T* in,
                           long long in_cstride, C<T>* S, long long nspec, int nyp, int hx, int pitch, int rpc,
                           int threads, cudaStream_t st, int nrep = 1, long long in_rstride = 0,
-                          long long s_rstride = 0, bool inl = false, bool split = false) {
+                          long long s_rstride = 0, bool split = false) {
   if (ncomp == 3) {
     XPassW<T> w = x_pass_w<T>(p);
     if constexpr (sizeof(T) == 4) {
@@ -3060,13 +3074,13 @@ cudaError_t run_x_forward(const FftPlan& p, int ncomp, int xdata, int ydata, int
                         s_rstride);
     }
   }
-  if (ncomp == 3 && p.warp_a == 32) return cudaErrorInvalidValue;  // handled by k_x_forward_w above
+  if (ncomp == 3 && p.warp_a == 32) return cudaErrorInvalidValue;  // the wide shapes have warp-shaped x passes
   const int lines = (ncomp + 1) / 2;
   size_t sm = x_pass_smem(p, lines, rpc, sizeof(C<T>));
   dim3 grid((nrows + rpc - 1) / rpc, 1, nrep);
-  auto kern = inl ? k_x_forward<T, true, 3> : k_x_forward<T, false, 3>;
+  auto kern = plan_odd(p) ? k_x_forward<T, 3, true> : k_x_forward<T, 3, false>;
   if constexpr (__is_same(T, f64s)) {
-    if (ncomp == 6) kern = k_x_forward<T, false, 6>;  // the tensor's six blocks
+    if (ncomp == 6) kern = k_x_forward<T, 6, true>;  // the tensor's six blocks
   }
   if (ncomp != 3 && !(ncomp == 6 && __is_same(T, f64s))) return cudaErrorInvalidValue;
   kern<<<grid, threads, sm, st>>>(p, xdata, FastDiv((uint32_t)ydata), nrows, in, in_cstride, S, nspec, nyp,
@@ -3129,7 +3143,7 @@ cudaError_t run_col_pass(const FftPlan& p, int ncomp, C<T>* S, long long nspec, 
     }
   }
   dim3 grid((hx + tx - 1) / tx, planes, nrep);
-  auto kern = inl ? k_col_pass<T, true> : k_col_pass<T, false>;
+  auto kern = plan_odd(p) ? k_col_pass<T, false, true> : inl ? k_col_pass<T, true, false> : k_col_pass<T, false, false>;
   if constexpr (!__is_same(T, double)) {
     if (p.warp_a == 32) kern = inl ? k_col_pass_wide<T, true> : k_col_pass_wide<T, false>;
   }
@@ -3174,7 +3188,7 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   }
   if (!x64)
     MMC_TRY(run_x_forward<T>(px, 3, g.nx, g.ny, rows, m, g.n, S, ns, g.nyp, g.hx, g.hxp, tun.x_rows_per_cta,
-                           tun.x_threads, st, nrep, mr, sr, tun.fft_inline != 0, split));
+                           tun.x_threads, st, nrep, mr, sr, split));
   if (ev) MMC_TRY(cudaEventRecord(ev[1], st));
   const long long ystride = g.hxp, yplane = (long long)g.nyp * g.hxp;
   if (g.nzp == 1) {
@@ -3210,7 +3224,7 @@ cudaError_t demag_impl(const Geom& g, const FftPlan& px, const FftPlan& py, cons
   } else {
     if (px.warp_a == 32) return cudaErrorInvalidValue;  // the wide shapes have warp-shaped x passes
     size_t sm = x_pass_smem(px, 2, rpc, sizeof(C<T>));
-    auto kinv = tun.fft_inline ? k_x_inverse<T, true> : k_x_inverse<T, false>;
+    auto kinv = plan_odd(px) ? k_x_inverse<T, true> : k_x_inverse<T, false>;
     kinv<<<grid, tun.x_threads, sm, st>>>(px, S, ns, g.nyp, g.hx, g.hxp, g.dnx, g.dny, rows, h, g.n, rpc, sr, mr);
   }
   MMC_TRY(cudaGetLastError());

@@ -143,7 +143,7 @@ __device__ __forceinline__ void row_load(const RowPhase<T>& R, const McCoef<T>& 
 }
 
 // inverse x-FFT of the work rows -> hsm
-template <typename T>
+template <typename T, bool ODD>
 __device__ __forceinline__ void row_field(const RowPhase<T>& R) {
   using V = C<T>;
   const int nx = R.g.nx, hx = R.g.hx, hxp = R.g.hx + (R.g.hx & 1), L = R.px->n;
@@ -170,7 +170,7 @@ __device__ __forceinline__ void row_field(const RowPhase<T>& R) {
     R.fa[(size_t)(2 * w + 1) * L + k] = B;
   }
   __syncthreads();
-  V* res = fft_run<T, true>(R.fa, R.fb, 2 * nwork, L, *R.px, R.twx);
+  V* res = fft_run<T, true, ODD>(R.fa, R.fb, 2 * nwork, L, *R.px, R.twx);
   for (int idx = threadIdx.x; idx < nwork * nx; idx += blockDim.x) {
     const int w = R.g.dnx.div(idx), x = idx - w * nx;
     const V a = res[(size_t)(2 * w) * L + x];
@@ -257,7 +257,7 @@ __device__ __forceinline__ void row_store(const RowPhase<T>& R, bool with_h) {
 }
 
 // forward x-FFT of the band rows held in msm -> spectrum rows
-template <typename T>
+template <typename T, bool ODD>
 __device__ __forceinline__ void row_forward(const RowPhase<T>& R) {
   using V = C<T>;
   const int nx = R.g.nx, hx = R.g.hx, hxp = R.g.hxp, L = R.px->n;
@@ -275,7 +275,7 @@ __device__ __forceinline__ void row_forward(const RowPhase<T>& R) {
     R.fa[(size_t)(2 * rr + 1) * L + x] = b;
   }
   __syncthreads();
-  V* res = fft_run<T, false>(R.fa, R.fb, 2 * R.nb, L, *R.px, R.twx);
+  V* res = fft_run<T, false, ODD>(R.fa, R.fb, 2 * R.nb, L, *R.px, R.twx);
   for (int idx = threadIdx.x; idx < R.nb * hx; idx += blockDim.x) {
     const int rr = R.g.dhx.div(idx), k = idx - rr * hx;
     const V* la = res + (size_t)(2 * rr) * L;
@@ -291,9 +291,11 @@ __device__ __forceinline__ void row_forward(const RowPhase<T>& R) {
 }
 
 // Batched row kernel: one CTA per (band, replica).  A batched film sweep is
-// this kernel (m, S) -> (mo, So) followed by the column pass on So.
-template <typename T>
-__global__ void __launch_bounds__(256) k_rows(Geom g, const __grid_constant__ FftPlan px,
+// this kernel (m, S) -> (mo, So) followed by the column pass on So.  FP32: two
+// CTAs per SM, at 128 registers (203 without the bound in the instance with the
+// odd stages: 16 x 88^2 in bands of 8, 57.9 us per sweep instead of 44.2).
+template <typename T, bool ODD>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_rows(Geom g, const __grid_constant__ FftPlan px,
                                               const McCoef<T>* __restrict__ coef, const T* m, T* mo, T* h,
                                               const C<T>* S, C<T>* So, unsigned long long* acc,
                                               const SweepCounters* ctr, int band, int with_h, int do_forward) {
@@ -321,10 +323,10 @@ __global__ void __launch_bounds__(256) k_rows(Geom g, const __grid_constant__ Ff
   load_twiddles<T>(px, R.twx);
   __syncthreads();
   row_load<T>(R, c, ctr->stage, ctr->sweep);
-  row_field<T>(R);
+  row_field<T, ODD>(R);
   unsigned int a = row_sweep<T>(R, c);
   row_store<T>(R, with_h != 0);
-  if (do_forward) row_forward<T>(R);
+  if (do_forward) row_forward<T, ODD>(R);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
   if ((threadIdx.x & 31) == 0 && a) atomicAdd(&s_acc, a);
