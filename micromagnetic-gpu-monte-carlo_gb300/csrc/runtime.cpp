@@ -267,6 +267,11 @@ DemagTuning choose_tuning(const Geom& g, const FftPlan& px, const FftPlan& py, c
   // (FP32 warp-shaped passes: a CTA's warps work on their own, and full CTAs are
   // as fast as single rows on one 64^2 film, faster from 32 of them on)
   while (r > 1 && !(csize == 8 && px.warp_a) && ((rows + r - 1) / r) * nrep < want) r /= 2;
+  // (but lines of 512 and 1024 spread better in half-full CTAs where full ones do
+  // not cover the SMs: 512 x 48 22.2 us per sweep with 8 rows per CTA, 19.7 with 4;
+  // 512 x 512 in 64 CTAs of 8 rows or 128 of 4 35.7 / 34.4, two of them 41.1 / 40.9,
+  // three of them 46.6 / 50.2; 16 of 1024 x 64 37.5 with 4 rows, 40.7 with 2)
+  if (csize == 8 && px.warp_a == 32 && ((rows + r - 1) / r) * nrep < nsm) r /= 2;
   while (r > 1 && xsm(r) > 96 * 1024) r /= 2;
   t.x_rows_per_cta = r;
   // in-place column passes reading K^ from global memory for the long

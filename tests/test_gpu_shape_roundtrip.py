@@ -27,3 +27,13 @@ def test_reported_shapes_are_accepted(M, prec, nx, ny, nz, R):
         a.run_sweeps(0, 0, 40)
         b.run_sweeps(0, 0, 40)
         assert all(np.array_equal(a.get_m(r), b.get_m(r)) for r in range(R))
+
+
+@pytest.mark.parametrize("nx,ny,nz,R,rows", [(512, 48, 1, 1, 4), (1024, 16, 1, 1, 2), (512, 512, 1, 4, 8),
+                                             (256, 48, 1, 1, 4)])
+def test_long_lines_on_few_rows_spread_over_the_sms(M, nx, ny, nz, R, rows):
+    """FP32 x passes of 512 and 1024 take half as many rows per CTA where full
+    CTAs would not cover the SMs."""
+    cfgs = [M.Config.defaults(nx=nx, ny=ny, nz=nz, pbc_x=1, pbc_y=1, pbc_z=0, precision=32) for _ in range(R)]
+    with M.Batch(cfgs) as b:
+        assert b.launch_shape()[0] == rows
