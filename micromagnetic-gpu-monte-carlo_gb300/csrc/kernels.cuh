@@ -1638,14 +1638,16 @@ __device__ __forceinline__ void st4(T* p, const Vec4<T>& r) {
   }
 }
 
-// The components whose second exchange product the vectorised forms round
+// The components whose second exchange product a vectorised form rounds
 // separately (mc_accept_formula; bit 0 = x) for cell q of a thread's two, at x
-// offset p0 + 2 q of its u-th segment.  This is how these forms have rounded
-// from the beginning: one trial in 1e10 is decided by it, and it keeps a seed's
-// run the same.
+// offset p0 + 2 q of its u-th segment.  This is how each form has rounded from
+// the beginning, and it keeps a seed's run the same; about two trials in 1e10 are
+// decided by it, so a long run in one of these forms leaves the scalar forms'
+// path there.  u < 0: the scalar forms' chain (k_mc_band); k_mc_pipe takes u = 1;
+// k_mc_quad and k_mc_split the number of the thread's segment.
 template <bool ALLB, bool Z3>
 __device__ __forceinline__ int mc_sep(int q, int u, int p0) {
-  if (q) return 0;
+  if (q || u < 0) return 0;
   if (ALLB) return !Z3 || u == 1 ? 7 : p0;
   return u == 1 || p0 == 0 ? 7 : Z3 ? 0 : 4;
 }
@@ -1989,7 +1991,7 @@ template <typename T, bool ALLB>
 __device__ __forceinline__ void band_segments(const Geom& g, const McCoef<T>& c, const T* ms, const T* hs,
                                               T* __restrict__ m, int y0, int nb, int color, bool dm,
                                               const FastDiv& dseg, uint32_t stage, uint32_t sweep,
-                                              unsigned int& mine) {
+                                              unsigned int& mine, int u) {
   const int nx = g.nx, ny = g.ny;
   const long long n = g.n;
   const int nseg = (int)dseg.d;
@@ -2026,10 +2028,10 @@ __device__ __forceinline__ void band_segments(const Geom& g, const McCoef<T>& c,
     bool changed;
     if (p0 == 0)
       changed = quad_cells<T, 0, ALLB>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0), stage,
-                                       sweep, mine, 1, own, own, false, false);
+                                       sweep, mine, u, own, own, false, false);
     else
       changed = quad_cells<T, 1, ALLB>(c, own, up, dn, lft, rgt, hh, hl, hr, hd, hu, (uint32_t)(rowb + x0), stage,
-                                       sweep, mine, 1, own, own, false, false);
+                                       sweep, mine, u, own, own, false, false);
     if (changed) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) st4<T>(m + k * n + rowb + x0, own[k]);
@@ -2078,7 +2080,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_mc_band(Geom g,
   cp_async_wait_all();
   __syncthreads();
   unsigned int mine = 0;
-  band_segments<T, ALLB>(g, c, ms, hs, m, y0, nb, color, dm, dseg, ctr->stage, ctr->sweep, mine);
+  band_segments<T, ALLB>(g, c, ms, hs, m, y0, nb, color, dm, dseg, ctr->stage, ctr->sweep, mine, -1);
   unsigned int v = mine;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -2271,7 +2273,7 @@ __global__ void __launch_bounds__(MCP_THREADS, 2)
       }
       const T* ms = buf0 + s * selems;
       band_segments<T, ALLB>(g, c, ms, ms + (size_t)(band + 2) * 3 * g.nx, m + (long long)r * 3 * n, y0,
-                             min(band, g.ny - y0), color, c.cd != (T)0, dseg, stage, sweep, mine);
+                             min(band, g.ny - y0), color, c.cd != (T)0, dseg, stage, sweep, mine, 1);
     }
     __syncthreads();  // buffer s is free; abort_s is final for this item
     if (abort_s) {
