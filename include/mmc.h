@@ -394,10 +394,10 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
  * passes, kx columns per tile of the y and z passes, threads of the column
  * passes, the band of the film row kernel (0 when sweeps use one kernel per
  * pass), and the Metropolis form: 0 one launch per colour, 1 both colours of
- * a film in one tile launch, 2 one vectorised launch per colour (films with
+ * a film in one tile launch (from one copy of m to another), 2 one vectorised launch per colour (films with
  * nx a multiple of 4), 3 the same with each CTA's rows staged in shared
  * memory by asynchronous copies (nx also at most 1024), 4 both colours of a
- * film in one launch over strips of rows (nx a multiple of 4, at most 2048,
+ * film in one launch over strips of rows (as 1; nx a multiple of 4, at most 2048,
  * row kernel off), 5 the staged form run by persistent CTAs with the rows
  * fetched by bulk asynchronous copies (as 3; a run whose buffer wait runs out
  * of its time limit returns MMC_ERR_TIMEOUT), whether the pass kernels expand their transforms in

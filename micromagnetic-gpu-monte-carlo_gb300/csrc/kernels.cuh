@@ -2300,9 +2300,11 @@ __global__ void __launch_bounds__(MCP_THREADS, 2)
 // ring cells belong to neighbouring tiles, and this CTA repeats, bit for bit,
 // the decisions their owners make -- same inputs, same Philox counter -- so
 // that colour 1 on the tile sees exactly the colour-0 state of the two-launch
-// sweep.  Only tile cells are written back and counted.  Periodic axes must be
-// whole tiles and at least two tiles long, so the margin never wraps onto the
-// tile itself.
+// sweep.  Only tile cells are written and counted, to the other copy of m: a
+// neighbour that starts later (another wave of CTAs, a cold instruction cache)
+// still has to read this tile's margin as it was before the sweep.  Periodic
+// axes must be whole tiles and at least two tiles long, so the margin never wraps
+// onto the tile itself.
 constexpr int MCT = 32;
 
 // One 4- or 8-byte global -> shared copy through the async path (no register
@@ -2328,7 +2330,8 @@ __host__ __device__ inline size_t mc_tile_smem() {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_mc_tile(Geom g, const McCoef<T>* __restrict__ cp, T* __restrict__ m,
+__global__ void __launch_bounds__(256) k_mc_tile(Geom g, const McCoef<T>* __restrict__ cp,
+                                                 const T* __restrict__ m, T* __restrict__ mo,
                                                  const T* __restrict__ h, const SweepCounters* __restrict__ ctr,
                                                  unsigned long long* acc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2338,6 +2341,7 @@ __global__ void __launch_bounds__(256) k_mc_tile(Geom g, const McCoef<T>* __rest
   const McCoef<T> c = cp[blockIdx.z];
   const long long n = g.n;
   m += blockIdx.z * 3 * n;
+  mo += blockIdx.z * 3 * n;
   h += blockIdx.z * 3 * n;
   acc += blockIdx.z;
   const uint32_t stage = ctr->stage, sweep = ctr->sweep;
@@ -2430,7 +2434,7 @@ __global__ void __launch_bounds__(256) k_mc_tile(Geom g, const McCoef<T>* __rest
     const int cc = idx / (MCT * MCT), r = idx - cc * MCT * MCT, ty = r / MCT, tx = r - ty * MCT;
     const int gx = colx[tx + 2], gy = rowy[ty + 2];
     if (gx >= 0 && gy >= 0 && x0 + tx < g.nx && y0 + ty < g.ny)
-      m[cc * n + (long long)gy * g.nx + gx] = sm[cc * BB + (ty + 2) * MCT_B + tx + 2];
+      mo[cc * n + (long long)gy * g.nx + gx] = sm[cc * BB + (ty + 2) * MCT_B + tx + 2];
   }
   unsigned int v = mine;
 #pragma unroll
@@ -3238,14 +3242,8 @@ template <typename T>
 cudaError_t mc_impl(const Geom& g, const McCoef<T>* c, T* m, const T* h, const SweepCounters* ctr, int color,
                     unsigned long long* acc, cudaStream_t st, int nrep, int form) {
   const int threads = 256;
-  // form: MC_FORM_TILE both colours in one tile launch, MC_FORM_QUAD one
-  // vectorised launch per colour, else one scalar launch per colour
+  // the forms that work in place, one launch per colour (the others: launch_mc_out)
   if (color < 0) {  // every colour of the sweep
-    if (form == MC_FORM_TILE && mc_tile_ok(g)) {
-      dim3 grid((unsigned)((g.nx + MCT - 1) / MCT), (unsigned)((g.ny + MCT - 1) / MCT), nrep);
-      k_mc_tile<T><<<grid, threads, mc_tile_smem<T>(), st>>>(g, c, m, h, ctr, acc);
-      return cudaGetLastError();
-    }
     for (int col = 0; col < g.ncolors; ++col) MMC_TRY(mc_impl<T>(g, c, m, h, ctr, col, acc, st, nrep, form));
     return cudaSuccess;
   }
@@ -3394,9 +3392,16 @@ cudaError_t launch_mc(const Geom& g, const McCoef<T>* c, T* m, const T* h, const
   return mc_impl<T>(g, c, m, h, ctr, color, acc, st, nrep, form);
 }
 template <typename T>
-cudaError_t launch_mc_strip(const Geom& g, const McCoef<T>* c, const T* m_in, T* m_out, const T* h,
-                            const SweepCounters* ctr, unsigned long long* acc, cudaStream_t st, int nrep) {
-  if (!mc_strip_ok(g) || m_in == m_out) return cudaErrorInvalidValue;
+cudaError_t launch_mc_out(const Geom& g, const McCoef<T>* c, const T* m_in, T* m_out, const T* h,
+                          const SweepCounters* ctr, unsigned long long* acc, cudaStream_t st, int nrep, int form) {
+  if (m_in == m_out) return cudaErrorInvalidValue;
+  if (form == MC_FORM_TILE) {
+    if (!mc_tile_ok(g)) return cudaErrorInvalidValue;
+    dim3 grid((unsigned)((g.nx + MCT - 1) / MCT), (unsigned)((g.ny + MCT - 1) / MCT), nrep);
+    k_mc_tile<T><<<grid, 256, mc_tile_smem<T>(), st>>>(g, c, m_in, m_out, h, ctr, acc);
+    return cudaGetLastError();
+  }
+  if (form != MC_FORM_STRIP || !mc_strip_ok(g)) return cudaErrorInvalidValue;
   const int rows = mc_strip_rows(g);
   dim3 grid((unsigned)((g.ny + rows - 1) / rows), 1, nrep);
   auto kern = mc_all_bonds(g) ? k_mc_strip<T, true> : k_mc_strip<T, false>;
@@ -3459,8 +3464,8 @@ cudaError_t launch_khat_store(long long count, const double2* spec64, void* khat
                                            const DemagTuning&, const T*, T*, void*, const void*, cudaStream_t); \
   template cudaError_t launch_mc<T>(const Geom&, const McCoef<T>*, T*, const T*, const SweepCounters*, int,   \
                                     unsigned long long*, cudaStream_t, int, int);                             \
-  template cudaError_t launch_mc_strip<T>(const Geom&, const McCoef<T>*, const T*, T*, const T*,             \
-                                          const SweepCounters*, unsigned long long*, cudaStream_t, int);       \
+  template cudaError_t launch_mc_out<T>(const Geom&, const McCoef<T>*, const T*, T*, const T*,               \
+                                        const SweepCounters*, unsigned long long*, cudaStream_t, int, int);    \
   template cudaError_t launch_energy<T>(const Geom&, const EnCoef*, const T*, const T*, double*, int, double*, \
                                         cudaStream_t, int, int, bool);                                         \
   template cudaError_t launch_field<T>(const Geom&, const HCoef&, int, const T*, const T*, double*,            \

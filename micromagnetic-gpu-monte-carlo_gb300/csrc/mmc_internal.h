@@ -175,13 +175,12 @@ cudaError_t launch_demag(const Geom& g, const FftPlan& px, const FftPlan& py, co
                          const DemagTuning& tun, const T* m, T* h, void* spec, const void* khat,
                          cudaStream_t st, int nrep = 1, cudaEvent_t* ev = nullptr, bool split = false);
 // (split: m and h in the colour-split order, see MC_FORM_SPLIT.)
-// Metropolis kernel forms (all make the same decisions): one scalar launch
-// per colour; both colours of a film in one tile launch; one vectorised launch
-// per colour for films with nx a multiple of 4.
+// Metropolis kernel forms (mc_sep says where their decisions part): one scalar launch
+// per colour; one vectorised launch per colour for films with nx a multiple of 4.
 // (MC_FORM_BAND: the vectorised form with the CTA's rows staged in shared
-// memory by asynchronous copies.)  MC_FORM_STRIP: both colours of a film in
-// one launch by strips of rows, reading m from one buffer and writing the
-// other (launch_mc_strip; the batch alternates its two copies of m).
+// memory by asynchronous copies.)  MC_FORM_TILE and MC_FORM_STRIP: both colours
+// of a film in one launch by tiles or strips of rows, reading m from one buffer
+// and writing the other (launch_mc_out; the batch alternates its two copies of m).
 // MC_FORM_PIPE: one colour per launch by persistent CTAs, each band's rows
 // staged by bulk asynchronous copies into a ring of shared-memory buffers
 // (k_mc_pipe).
@@ -223,8 +222,8 @@ int* mc_pipe_err_word();
 int mc_pipe_error_take();
 // One sweep (both colours) in the strip form: m_in -> m_out (distinct buffers).
 template <typename T>
-cudaError_t launch_mc_strip(const Geom& g, const McCoef<T>* c, const T* m_in, T* m_out, const T* h,
-                            const SweepCounters* ctr, unsigned long long* acc, cudaStream_t st, int nrep);
+cudaError_t launch_mc_out(const Geom& g, const McCoef<T>* c, const T* m_in, T* m_out, const T* h,
+                          const SweepCounters* ctr, unsigned long long* acc, cudaStream_t st, int nrep, int form);
 constexpr int MC_TILE_SIDE = 32;
 template <typename T>
 // with_q: 1 energies, <m> and Q; 0 energies and <m> (FP64 per cell); -1 the

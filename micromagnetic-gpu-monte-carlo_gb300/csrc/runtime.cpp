@@ -1479,18 +1479,20 @@ cudaError_t batch_demag(mmc_batch* b, cudaEvent_t* ev = nullptr, const void* m =
                               h->khat, h->st, b->R, ev);
 }
 
-// The strip form (both colours in one launch) reads m from one copy and
-// writes the other: sweep q of a run reads m on even q and m2 on odd q.
-bool batch_strip(const mmc_batch* b) {
-  return b->rows_band == 0 && b->tun.mc_form == MC_FORM_STRIP && mc_strip_eligible(b->base->g);
+// The strip and tile forms (both colours in one launch) read m from one copy
+// and write the other: sweep q of a run reads m on even q and m2 on odd q.
+bool mc_two_copies(int form) { return form == MC_FORM_STRIP || form == MC_FORM_TILE; }
+bool batch_two(const mmc_batch* b) {
+  return b->rows_band == 0 && ((b->tun.mc_form == MC_FORM_STRIP && mc_strip_eligible(b->base->g)) ||
+                               (b->tun.mc_form == MC_FORM_TILE && mc_tile_eligible(b->base->g)));
 }
 int batch_alloc_m2(mmc_batch* b) {
   const mmc_handle* h = b->base;
   if (!b->m2) CU(cudaMalloc(&b->m2, (size_t)b->R * 3 * h->g.n * h->tsize));
   return MMC_OK;
 }
-// After an odd number of strip-form sweeps the state sits in m2: move it back.
-cudaError_t batch_strip_settle(mmc_batch* b) {
+// After an odd number of such sweeps the state sits in m2: move it back.
+cudaError_t batch_two_settle(mmc_batch* b) {
   mmc_handle* h = b->base;
   return cudaMemcpyAsync(b->m, b->m2, (size_t)b->R * 3 * h->g.n * h->tsize, cudaMemcpyDeviceToDevice, h->st);
 }
@@ -1551,29 +1553,30 @@ int batch_alloc_streams(mmc_batch* b) {
   return MMC_OK;
 }
 
-// One sweep of replicas [r0, r0 + nr) on stream st (parity: see batch_strip).
+// One sweep of replicas [r0, r0 + nr) on stream st (parity: see batch_two).
 template <typename T>
 cudaError_t batch_sweep_part(mmc_batch* b, int r0, int nr, cudaStream_t st, int slot, int parity) {
   mmc_handle* h = b->base;
   const long long ms = 3 * h->g.n, ss = 3 * h->g.nspec;
-  const bool strip = batch_strip(b);
-  T* m = (T*)(strip && parity ? b->m2 : b->m) + r0 * ms;
+  const bool two = batch_two(b);
+  T* m = (T*)(two && parity ? b->m2 : b->m) + r0 * ms;
   T* hh = (T*)b->h + r0 * ms;
   cudaError_t e = cudaSuccess;
   if (h->cfg.cal_demag_flag)
     e = launch_demag<T>(h->g, h->px.p, h->py.p, h->pz.p, b->tun, m, hh,
                         (char*)b->spec + (size_t)r0 * ss * 2 * sizeof(T), h->khat, st, nr, nullptr, b->split);
   if (e != cudaSuccess) return e;
-  if (strip) {
+  if (two) {
     T* mo = (T*)(parity ? b->m : b->m2) + r0 * ms;
-    return launch_mc_strip<T>(h->g, (const McCoef<T>*)b->coef + r0, m, mo, hh, b->ctr + slot, b->acc + r0, st, nr);
+    return launch_mc_out<T>(h->g, (const McCoef<T>*)b->coef + r0, m, mo, hh, b->ctr + slot, b->acc + r0, st, nr,
+                            b->tun.mc_form);
   }
   return launch_mc<T>(h->g, (const McCoef<T>*)b->coef + r0, m, hh, b->ctr + slot, -1, b->acc + r0, st, nr,
                       batch_form(b));
 }
 
 // One sweep reading counter slot `slot` (the caller advances the counters);
-// parity: see batch_strip.
+// parity: see batch_two.
 cudaError_t batch_sweep(mmc_batch* b, cudaEvent_t* ev, int slot, int parity) {
   mmc_handle* h = b->base;
   cudaError_t e;
@@ -1602,15 +1605,16 @@ cudaError_t batch_sweep(mmc_batch* b, cudaEvent_t* ev, int slot, int parity) {
     }
     return cudaSuccess;
   }
-  const bool strip = batch_strip(b);
-  void* mi = strip && parity ? b->m2 : b->m;
+  const bool two = batch_two(b);
+  void* mi = two && parity ? b->m2 : b->m;
   void* mo = parity ? b->m : b->m2;
   if (h->cfg.cal_demag_flag && (e = batch_demag(b, ev, mi)) != cudaSuccess) return e;
-  if (strip)
-    e = h->prec == 32 ? launch_mc_strip<float>(h->g, (const McCoef<float>*)b->coef, (const float*)mi, (float*)mo,
-                                               (const float*)b->h, b->ctr + slot, b->acc, h->st, b->R)
-                      : launch_mc_strip<double>(h->g, (const McCoef<double>*)b->coef, (const double*)mi, (double*)mo,
-                                                (const double*)b->h, b->ctr + slot, b->acc, h->st, b->R);
+  if (two)
+    e = h->prec == 32 ? launch_mc_out<float>(h->g, (const McCoef<float>*)b->coef, (const float*)mi, (float*)mo,
+                                               (const float*)b->h, b->ctr + slot, b->acc, h->st, b->R, b->tun.mc_form)
+                      : launch_mc_out<double>(h->g, (const McCoef<double>*)b->coef, (const double*)mi, (double*)mo,
+                                                (const double*)b->h, b->ctr + slot, b->acc, h->st, b->R,
+                                                b->tun.mc_form);
   else
     e = h->prec == 32 ? launch_mc<float>(h->g, (const McCoef<float>*)b->coef, (float*)b->m, (const float*)b->h,
                                          b->ctr + slot, -1, b->acc, h->st, b->R, batch_form(b))
@@ -1640,12 +1644,13 @@ cudaError_t batch_sweep_lead(mmc_batch* b, int slot) {
   if (h->cfg.cal_demag_flag && (e = batch_demag(b)) != cudaSuccess) return e;
   if ((e = batch_energy_kernels(b, true, false)) != cudaSuccess) return e;
   if ((e = batch_swap(b)) != cudaSuccess) return e;
-  if (batch_strip(b))
-    return h->prec == 32 ? launch_mc_strip<float>(h->g, (const McCoef<float>*)b->coef, (const float*)b->m,
-                                                  (float*)b->m2, (const float*)b->h, b->ctr + slot, b->acc, h->st, b->R)
-                         : launch_mc_strip<double>(h->g, (const McCoef<double>*)b->coef, (const double*)b->m,
+  if (batch_two(b))
+    return h->prec == 32 ? launch_mc_out<float>(h->g, (const McCoef<float>*)b->coef, (const float*)b->m,
+                                                  (float*)b->m2, (const float*)b->h, b->ctr + slot, b->acc, h->st, b->R,
+                                                  b->tun.mc_form)
+                         : launch_mc_out<double>(h->g, (const McCoef<double>*)b->coef, (const double*)b->m,
                                                    (double*)b->m2, (const double*)b->h, b->ctr + slot, b->acc, h->st,
-                                                   b->R);
+                                                   b->R, b->tun.mc_form);
   return h->prec == 32 ? launch_mc<float>(h->g, (const McCoef<float>*)b->coef, (float*)b->m, (const float*)b->h,
                                           b->ctr + slot, -1, b->acc, h->st, b->R, batch_form(b))
                        : launch_mc<double>(h->g, (const McCoef<double>*)b->coef, (double*)b->m, (const double*)b->h,
@@ -1665,7 +1670,7 @@ cudaError_t batch_sweeps(mmc_batch* b, long long k, bool lead_swap = false) {
       e = launch_advance(b->ctr, (uint32_t)(slot + 1), b->base->st, CTR_SLOTS);
   }
   if (e == cudaSuccess && b->rows_band > 0 && (k & 1)) e = batch_rows_settle(b);
-  if (e == cudaSuccess && batch_strip(b) && (k & 1)) e = batch_strip_settle(b);
+  if (e == cudaSuccess && batch_two(b) && (k & 1)) e = batch_two_settle(b);
   return e;
 }
 
@@ -1926,7 +1931,10 @@ int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
     if (tried && !batch_shape_ok(b, cd.tun, cd.rows_band)) return;
     if (cd.rows_band > 0 && (status = batch_alloc_rows(b)) != MMC_OK) return;
     if (cd.streams > 1 && (status = batch_alloc_streams(b)) != MMC_OK) return;
-    if (cd.tun.mc_form == MC_FORM_STRIP && (status = batch_alloc_m2(b)) != MMC_OK) return;
+    if (mc_two_copies(cd.tun.mc_form) && batch_alloc_m2(b) != MMC_OK) {  // no room for the second copy: not tried
+      cudaGetLastError();
+      return;
+    }
     ++tried;
     b->rows_band = cd.rows_band;
     b->tun = cd.tun;
@@ -2694,8 +2702,8 @@ int mmc_batch_profile_sweeps(mmc_batch* b, long long stage, long long sweep0, lo
     }
     if (e != cudaSuccess) status = fail(MMC_ERR_CUDA, cudaGetErrorString(e));
   }
-  if (status == MMC_OK && batch_strip(b) && (nsweeps & 1)) {
-    cudaError_t e = batch_strip_settle(b);
+  if (status == MMC_OK && batch_two(b) && (nsweeps & 1)) {
+    cudaError_t e = batch_two_settle(b);
     if (e != cudaSuccess) status = fail(MMC_ERR_CUDA, cudaGetErrorString(e));
   }
   batch_run_abandon(b, status);
@@ -2720,7 +2728,7 @@ int mmc_batch_set_launch_shape(mmc_batch* b, const int shape[10]) {
   TRY(set_dev(b->base));
   if (band > 0) TRY(batch_alloc_rows(b));
   if (streams > 1) TRY(batch_alloc_streams(b));
-  if (t.mc_form == MC_FORM_STRIP) TRY(batch_alloc_m2(b));
+  if (mc_two_copies(t.mc_form)) TRY(batch_alloc_m2(b));
   b->tun = t;
   b->rows_band = band;
   b->streams = streams;
