@@ -308,7 +308,8 @@ int mmc_run_sweeps(mmc_handle* h, double temperature, long long stage, long long
                    long long nsweeps);
 
 /* The sweep engine chosen at creation: out[0] = enum mmc_engine (never AUTO),
- * out[1] = rows per CTA of the fused engine, out[2] = its CTA count. */
+ * out[1] = rows per CTA of the fused engine, out[2] = its CTA count (0 where
+ * sweeps do not use it, until mmc_profile_fused sets it up). */
 int mmc_engine_info(mmc_handle* h, int out[3]);
 
 /* Device time, in ms, of the last mmc_run_sweeps() call: CUDA events recorded
@@ -322,7 +323,8 @@ int mmc_last_run_ms(mmc_handle* h, double* ms);
 int mmc_profile_sweeps(mmc_handle* h, double temperature, long long stage, long long sweep0, long long nsweeps,
                        double out_ms[3]);
 
-/* Profiling hook of the fused film engine: runs nsweeps (<= 1024) sweeps in
+/* Profiling hook of the fused film engine (of handles that use it, and of films
+ * that MMC_ENGINE_AUTO runs on the pass kernels): runs nsweeps (<= 1024) sweeps in
  * one launch and returns device timestamps (ns) of the phase boundaries of the
  * first 16 sweeps for the first and the last CTA: stamps[(s*9 + p)*2 + c],
  * points p = 0 row phase start, 1 copies landed, 2 demag field ready,

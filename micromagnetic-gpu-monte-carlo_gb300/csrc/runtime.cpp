@@ -600,15 +600,55 @@ int run_fused(mmc_handle* h, long long stage, long long sweep0, long long nsweep
   return MMC_OK;
 }
 
-// Picks the film engine's band (rows per CTA) and CTA count: the smallest band
-// from the preference list whose grid is co-resident.
+// Films with demag and two colours whose m rows are whole 16-byte chunks.
+bool film_eligible(const mmc_handle* h) {
+  const Geom& g = h->g;
+  return h->cfg.cal_demag_flag && g.nz == 1 && g.nzp == 1 && g.ncolors == 2 && ((size_t)g.nx * h->tsize) % 16 == 0 &&
+         g.ny >= 1 && h->px.p.warp_a != 32 && h->py.p.warp_a != 32;
+}
+
+// Picks the film engine's band (rows per CTA) and CTA count -- the smallest band
+// from the preference list whose grid is co-resident -- and allocates its
+// buffers.  h->fused_blocks stays 0 when no band fits.
+int film_setup(mmc_handle* h, int nsm) {
+  const mmc_config& c = h->cfg;
+  const Geom& g = h->g;
+  if (h->fused_blocks > 0) return MMC_OK;
+  int optin = 48 * 1024;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+  std::vector<int> bands;
+  if (c.fused_band > 0) bands.push_back(c.fused_band);
+  else bands = {2, 1, 3, 4, 6, 8, 12, 16, 24, 32, 48, 60};
+  for (int b : bands) {
+    const size_t smem = h->prec == 32 ? fused2d_smem_bytes<float>(g, h->px.p, h->py.p, b)
+                                      : fused2d_smem_bytes<double>(g, h->px.p, h->py.p, b);
+    if (smem > (size_t)optin) continue;
+    int per_sm = 0;
+    cudaError_t e = h->prec == 32 ? fused2d_blocks_per_sm<float>(g, h->px.p, h->py.p, b, &per_sm)
+                                  : fused2d_blocks_per_sm<double>(g, h->px.p, h->py.p, b, &per_sm);
+    if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
+    const int blocks = (g.ny + b - 1) / b;
+    if (per_sm > 0 && blocks <= per_sm * nsm) {
+      if (!h->bar) {
+        void* p = nullptr;
+        CU(cudaMalloc(&p, grid_barrier_bytes()));
+        h->bar = (GridBarrier*)p;
+        CU(cudaMemsetAsync(p, 0, grid_barrier_bytes(), h->st));
+      }
+      if (!h->m2) CU(cudaMalloc(&h->m2, 3 * (size_t)g.n * h->tsize));
+      if (!h->spec2) CU(cudaMalloc(&h->spec2, 3 * (size_t)g.nspec * 2 * h->tsize));
+      h->fused_band = b;
+      h->fused_blocks = blocks;
+      return MMC_OK;
+    }
+  }
+  return MMC_OK;
+}
+
 int setup_engine(mmc_handle* h, int nsm) {
   const mmc_config& c = h->cfg;
   const Geom& g = h->g;
-  // films with demag and two colours whose m rows are whole 16-byte chunks
-  const bool eligible = c.cal_demag_flag && g.nz == 1 && g.nzp == 1 && g.ncolors == 2 &&
-                        ((size_t)g.nx * h->tsize) % 16 == 0 && g.ny >= 1 && h->px.p.warp_a != 32 &&
-                        h->py.p.warp_a != 32;
+  const bool eligible = film_eligible(h);
   // FP64 films: the film engine's CTAs transform and sweep their halo rows again
   // and leave most of the SM's FP64 issue idle, while the pass kernels spread
   // the operations (lines64.cuh).  us per sweep, pass kernels / film engine: 32^2
@@ -627,32 +667,10 @@ int setup_engine(mmc_handle* h, int nsm) {
     return fail(MMC_ERR_UNSUPPORTED,
                 "the fused engine needs a film (nz = 1), demag on, an even or open lattice, nx * sizeof(real) "
                 "a multiple of 16 bytes and padded sides other than 512 and 1024");
-  int optin = 48 * 1024;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-  std::vector<int> bands;
-  if (c.fused_band > 0) bands.push_back(c.fused_band);
-  else bands = {2, 1, 3, 4, 6, 8, 12, 16, 24, 32, 48, 60};
-  for (int b : bands) {
-    const size_t smem = h->prec == 32 ? fused2d_smem_bytes<float>(g, h->px.p, h->py.p, b)
-                                      : fused2d_smem_bytes<double>(g, h->px.p, h->py.p, b);
-    if (smem > (size_t)optin) continue;
-    int per_sm = 0;
-    cudaError_t e = h->prec == 32 ? fused2d_blocks_per_sm<float>(g, h->px.p, h->py.p, b, &per_sm)
-                                  : fused2d_blocks_per_sm<double>(g, h->px.p, h->py.p, b, &per_sm);
-    if (e != cudaSuccess) return fail(MMC_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
-    const int blocks = (g.ny + b - 1) / b;
-    if (per_sm > 0 && blocks <= per_sm * nsm) {
-      h->engine = MMC_ENGINE_FUSED;
-      h->fused_band = b;
-      h->fused_blocks = blocks;
-      void* p = nullptr;
-      CU(cudaMalloc(&p, grid_barrier_bytes()));
-      CU(cudaMemsetAsync(p, 0, grid_barrier_bytes(), h->st));
-      h->bar = (GridBarrier*)p;
-      CU(cudaMalloc(&h->m2, 3 * (size_t)g.n * h->tsize));
-      CU(cudaMalloc(&h->spec2, 3 * (size_t)g.nspec * 2 * h->tsize));
-      return MMC_OK;
-    }
+  TRY(film_setup(h, nsm));
+  if (h->fused_blocks > 0) {
+    h->engine = MMC_ENGINE_FUSED;
+    return MMC_OK;
   }
   if (c.sweep_engine == MMC_ENGINE_FUSED)
     return fail(MMC_ERR_UNSUPPORTED, "no film-engine band fits this lattice on this device");
@@ -2534,9 +2552,13 @@ int mmc_engine_info(mmc_handle* h, int out[3]) {
 int mmc_profile_fused(mmc_handle* h, double temperature, long long stage, long long sweep0, long long nsweeps,
                       unsigned long long* stamps) {
   if (!h || !stamps) return fail(MMC_ERR_INVALID, "null argument");
-  if (h->engine != MMC_ENGINE_FUSED) return fail(MMC_ERR_STATE, "the handle does not use the fused engine");
+  // a lattice that AUTO runs on the pass kernels may be profiled on this engine too
+  const bool ours = h->engine == MMC_ENGINE_FUSED || (h->cfg.sweep_engine == MMC_ENGINE_AUTO && film_eligible(h));
+  if (!ours) return fail(MMC_ERR_STATE, "the handle does not use the fused engine");
   if (nsweeps < 1 || nsweeps > 1024) return fail(MMC_ERR_INVALID, "nsweeps must be in [1, 1024]");
   TRY(set_dev(h));
+  TRY(film_setup(h, h->nsm));
+  if (h->fused_blocks == 0) return fail(MMC_ERR_STATE, "the handle does not use the fused engine");
   TRY(ensure_demag(h));
   TRY(upload_coef(h, temperature));
   unsigned long long* d = nullptr;
