@@ -374,8 +374,8 @@ def run_ours(args):
     batch = M.Batch(cfgs, device=local)
     batch.build_demag(CACHE_DIR)
     setup_s = time.perf_counter() - t0
-    # launch shape: the fastest of all shapes on this device (bit-identical
-    # results), or the one given (to profile the shape a plain run chose)
+    # launch shape: the fastest of all shapes on this device, or the one given (to
+    # profile the shape a plain run chose)
     batch.set_temperatures(np.full(R, stage_temperature(0)))
     t0 = time.perf_counter()
     if args.launch_shape:

@@ -424,8 +424,10 @@ int mmc_batch_launch_shape(mmc_batch* b, int out[10]);
  * sweeps (the faster of two repetitions; replays of the 32-sweep graph that
  * runs execute, so `sweeps` is rounded up to a multiple of 32) from the
  * current state, keeps the fastest and restores m and the acceptance
- * counters.  Every shape gives bit-identical results, so the choice changes
- * only the speed.  best_ms_per_sweep and candidates may be NULL.  No
+ * counters.  Fields do not depend on the shape.  Decisions do not depend on it
+ * in FP64; in FP32 the Metropolis forms 2 and 5 round one product of the exchange
+ * sum by itself, forms 0, 1, 3, 4 and the row kernel with the sum, which decides
+ * about two trials in 1e10.  (FP32 runs of one seed repeat with one form.)  best_ms_per_sweep and candidates may be NULL.  No
  * counterpart in the reference, whose block shape is fixed in the source
  * (src/main.cu:275-286). */
 int mmc_batch_autotune(mmc_batch* b, int sweeps, double* best_ms_per_sweep, int* candidates);
@@ -436,8 +438,8 @@ int mmc_batch_autotune(mmc_batch* b, int sweeps, double* best_ms_per_sweep, int*
  * shared memory fits 220 KB in the chosen column-pass form, a row-kernel band
  * this batch offers, a Metropolis form the lattice qualifies for, 0/1 for the
  * in-line transform flag, 0-3 for the column-pass form and 1-4 streams;
- * anything else is rejected.  Results do
- * not depend on the shape.  No counterpart in the reference. */
+ * anything else is rejected.  Results depend
+ * on the shape only as said at mmc_batch_autotune.  No counterpart in the reference. */
 int mmc_batch_set_launch_shape(mmc_batch* b, const int shape[10]);
 
 /* Replica farms: batches of different lattice sizes advanced together.  One

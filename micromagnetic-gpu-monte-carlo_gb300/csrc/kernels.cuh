@@ -213,14 +213,15 @@ __device__ __forceinline__ void load_roots(const FftPlan& p, C<T>* dst) {
   for (int i = threadIdx.x; i < p.n; i += blockDim.x) dst[i] = src[i];
 }
 
-// (Register budget: 64 per thread in FP32 with 16 values per lane, so that
-// eight 128-thread CTAs fit on an SM; twice that in FP64 or with 32 values.)
-template <typename T, int A>
+// They serve the relaxation (f64s): FP32 lines have k_x_forward_r / k_x_inverse_r,
+// FP64 ones the passes of lines64.cuh.  (Register budget: 128 per thread with 16
+// values per lane, 255 with 32.)
+template <int A>
 constexpr int x_w_min_blocks() {
-  return (sizeof(T) == 4 ? 4 : 2) / (A >= 32 ? 2 : 1);
+  return A >= 32 ? 1 : 2;
 }
 template <typename T, int A, int B>
-__global__ void __launch_bounds__(256, x_w_min_blocks<T, A>()) k_x_forward_w(FftPlan p, int xdata, FastDiv dyd, int nrows, const T* __restrict__ in,
+__global__ void __launch_bounds__(256, x_w_min_blocks<A>()) k_x_forward_w(FftPlan p, int xdata, FastDiv dyd, int nrows, const T* __restrict__ in,
                               long long in_cstride, C<T>* __restrict__ S, long long nspec, int nyp, int hx,
                               int pitch, int rows_per_cta, long long in_rstride, long long s_rstride) {
   constexpr int L = A * B, GPW = 32 / B;
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(256, x_w_min_blocks<T, A>()) k_x_forward_w(Fft
 }
 
 template <typename T, int A, int B>
-__global__ void __launch_bounds__(256, x_w_min_blocks<T, A>()) k_x_inverse_w(FftPlan p, const C<T>* __restrict__ S, long long nspec, int nyp, int hx, int pitch,
+__global__ void __launch_bounds__(256, x_w_min_blocks<A>()) k_x_inverse_w(FftPlan p, const C<T>* __restrict__ S, long long nspec, int nyp, int hx, int pitch,
                               FastDiv dxo, FastDiv dyo, int nrows, T* __restrict__ out, long long out_cstride,
                               int rows_per_cta, long long s_rstride, long long out_rstride) {
   constexpr int L = A * B, GPW = 32 / B;
@@ -1185,15 +1186,23 @@ __device__ __forceinline__ Proposal<T> mc_propose(const McCoef<T>& c, uint32_t c
 //
 // The bound: with M >= every |component| of m involved (at least 1), H the
 // same for h, and G = gm M + gc + |cd| H >= |F_a| for each component of the
-// field (McFilter), dE = -d . F in the regrouped form of mc_accept<float>.  On
-// any path from an input to dE its FP32 evaluation makes at most 32 roundings of
-// 2^-24 (2 for a truncated input, 1 for a coefficient, 16 in a component of F, 3
-// in d and 3 in the dot product), each on terms that add up to at most |d|_1 G:
-// 1.9e-6 |d|_1 G.  The direction's components are off by at most 2.5e-7 (the
-// angle's rounding 9e-8, sincospif 1 ulp, 1 - z^2 as a product of two rounded
-// factors, its square root through rsqrtf), and dE changes by at most 2 G per
-// unit of each: 1.5e-6 G.  FP64 rounding is 1e-9 of either.  MC_FILTER_EPS =
-// 2.2e-6 times (|d|_1 + 1) G covers both.
+// field (McFilter), dE = -d . F in the regrouped form of mc_accept<float>.
+// - On any path from an input of F to dE the FP32 evaluation makes at most 32
+//   roundings of 2^-24 (2 for a truncated input, 1 for a coefficient, 16 in a
+//   component of F, 3 in d and 3 in the dot product), each on terms that add up to
+//   at most |d|_1 G: 1.9e-6 |d|_1 G.
+// - The direction m' and the cell's own m enter d itself, by absolute errors.  An
+//   error e of a component of either changes dE by at most e G (1 + |d|_1 / 4):
+//   through d, and through the K0 and anisotropy terms of F, whose coefficients
+//   are in G at least fourfold.  The errors add up over the components to 9.2e-7
+//   for m' (rsqrtf 2 ulp, t = (1 + z)(1 - z) from two rounded factors and their
+//   product, r = t / sqrt(t): 3.9e-7 of r, at most 5.5e-7 in x and y together;
+//   the angle's rounding 1.3e-7; sincospif 1 ulp each 1.2e-7; the products 9e-8; z
+//   3e-8) and to 2^-23 |m|_1 <= 2.1e-7 for m, truncated: together 1.13e-6 G +
+//   0.28e-6 |d|_1 G.
+// FP64 rounding is 1e-9 of either.  MC_FILTER_EPS = 2.2e-6 times (|d|_1 + 1) G
+// covers the sum, 2.2e-6 |d|_1 G + 1.13e-6 G, for unit vectors; the rest of its
+// constant part covers an m of another length.
 // exp: the hardware's is within 2 + 1.173 |x| ulp, 4.5e-6 for x >= -30; below
 // that the smallest uniform (2^-33) decides alone.  MC_FILTER_EXP = 2e-5 covers
 // it and the rounding of the uniform.  NaN or infinity anywhere leaves both
@@ -1267,12 +1276,13 @@ __device__ __forceinline__ McVerdict mc_filter(const McFilter& c, const float (&
 }
 
 // The Metropolis decision for one cell from its neighbour values, its own m,
-// its demag field h and its proposal.  Shared by every sweep kernel so that
-// all paths round identically.
-// SEP (FP32): in the components of this mask the second neighbour's product is
+// its demag field h and its proposal.  Shared by every sweep kernel, so that they
+// round alike but for sep.
+// sep (FP32): in the components of this mask the second neighbour's product is
 // rounded before it is added, where the chain of multiply-adds rounds it with the
-// sum.  The scalar forms take the chain, the vectorised ones what mc_sep says;
-// written out, it does not depend on what the compiler makes of the code around.
+// sum.  k_mc_quad, k_mc_split and k_mc_pipe take what mc_sep says, every other
+// form the chain; written out, it does not depend on what the compiler makes of
+// the code around.
 template <typename T>
 __device__ __forceinline__ bool mc_accept_formula(const McCoef<T>& c, const Nbrs<T>& nb, T ox, T oy, T oz, T hx, T hy,
                                                   T hz, T px, T py, T pz, T ua, int sep = 0) {
@@ -1645,6 +1655,10 @@ __device__ __forceinline__ void st4(T* p, const Vec4<T>& r) {
 // decided by it, so a long run in one of these forms leaves the scalar forms'
 // path there.  u < 0: the scalar forms' chain (k_mc_band); k_mc_pipe takes u = 1;
 // k_mc_quad and k_mc_split the number of the thread's segment.
+// The segments of a thread are a grid's threads apart, so these two fix u for every
+// cell; k_mc_quad and k_mc_split, which take runs of one seed in turn (by the
+// run's length), must share them.
+constexpr int MCQ_THREADS = 128, MCQ_UNITS = 2;
 template <bool ALLB, bool Z3>
 __device__ __forceinline__ int mc_sep(int q, int u, int p0) {
   if (q || u < 0) return 0;
@@ -1725,7 +1739,7 @@ __global__ void __launch_bounds__(256) k_mc_quad(Geom g, const McCoef<T>* __rest
   const int tstride = gridDim.x * blockDim.x;
   unsigned int mine = 0;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
+  for (int u = 0; u < MCQ_UNITS; ++u) {
     const int t = t0 + u * tstride;
     if (t < nseg * g.ny * g.nz) {
       // t / (nx / 4) == (4 t) / nx: the multiply-shift divider by nx, no run-time division
@@ -1828,7 +1842,7 @@ template <typename T>
 inline bool mc_split_ok(const Geom& g, const FftPlan& px) {
   return sizeof(T) == 4 && mc_split_geom_ok(g) && px.warp_a != 0;
 }
-constexpr int MCSP_THREADS = 128;
+constexpr int MCSP_THREADS = MCQ_THREADS;
 template <bool ALLB, bool Z3>
 __global__ void __launch_bounds__(MCSP_THREADS, 6) k_mc_split(Geom g, const McCoef<float>* __restrict__ cp,
                                                            float* __restrict__ m, const float* __restrict__ h,
@@ -3291,7 +3305,7 @@ cudaError_t mc_impl(const Geom& g, const McCoef<T>* c, T* m, const T* h, const S
     if constexpr (sizeof(T) == 4) {
       if (!mc_split_geom_ok(g)) return cudaErrorInvalidValue;
       const long long total = (long long)g.ny * g.nz * (g.nx >> 2);
-      const int upt = 2;  // units per thread (1: 28.6 us at 64 x 256^2 instead of 24.3)
+      const int upt = MCQ_UNITS;  // units per thread (1: 28.6 us at 64 x 256^2 instead of 24.3)
       dim3 grid((unsigned)((total + upt * MCSP_THREADS - 1) / (upt * MCSP_THREADS)), 1, nrep);
       auto kern = g.nz > 1 ? (mc_all_bonds(g) ? k_mc_split<true, true> : k_mc_split<false, true>)
                            : (mc_all_bonds(g) ? k_mc_split<true, false> : k_mc_split<false, false>);
@@ -3303,9 +3317,9 @@ cudaError_t mc_impl(const Geom& g, const McCoef<T>* c, T* m, const T* h, const S
   if (form == MC_FORM_QUAD && mc_quad_ok(g)) {
     // 128-thread CTAs: the same warps per SM as 256 (the registers limit
     // them), in finer pieces, measured 2 us faster per batched sweep
-    const int qthreads = 128;
+    const int qthreads = MCQ_THREADS;
     const long long total = (long long)g.ny * g.nz * (g.nx >> 2);  // segments, two per thread
-    dim3 grid((unsigned)((total + 2 * qthreads - 1) / (2 * qthreads)), 1, nrep);
+    dim3 grid((unsigned)((total + MCQ_UNITS * qthreads - 1) / (MCQ_UNITS * qthreads)), 1, nrep);
     auto kern = g.nz > 1 ? (mc_all_bonds(g) ? k_mc_quad<T, true, true> : k_mc_quad<T, false, true>)
                          : (mc_all_bonds(g) ? k_mc_quad<T, true, false> : k_mc_quad<T, false, false>);
     return launch_pdl(kern, grid, dim3(qthreads), 0, st, g, c, m, h, ctr, color, acc);

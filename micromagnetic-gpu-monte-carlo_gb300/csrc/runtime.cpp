@@ -220,8 +220,10 @@ size_t smem_limit() { return 220 * 1024; }  // below the 227 KB opt-in limit of 
 // Shared memory of an x pass with r rows per CTA, of a column pass with tx
 // columns per CTA (bytes).
 size_t x_pass_smem(const FftPlan& px, int r, size_t csize) {
-  if (px.warp_a)  // k_x_forward_w / k_x_inverse_w: the roots and 2 r padded lines
-    return ((size_t)px.n + 2 * (size_t)r * (px.n + px.warp_a)) * csize;
+  // warp-shaped lines: the roots and 2 r padded lines, as in k_x_forward_w (FP32
+  // launches hold the lines in flight only, FP64 ones have shapes of their own;
+  // this stays the limit for the rows of a launch shape)
+  if (px.warp_a) return ((size_t)px.n + 2 * (size_t)r * (px.n + px.warp_a)) * csize;
   return ((size_t)((px.tw_total + 1) & ~1) + 2 * (size_t)r * 2 * px.n) * csize;
 }
 // (lean: the in-place form, which exists for warp-shaped lengths only and
@@ -1602,7 +1604,7 @@ cudaError_t batch_sweep(mmc_batch* b, cudaEvent_t* ev, int slot, int parity) {
   // replica parts on their own streams while a graph is captured (as parallel
   // branches, kernels of different kinds overlap on the SMs); launched
   // directly, the extra launches and events cost more than they give, and
-  // every launch shape gives the same results, so direct sweeps use one stream
+  // the bits do not depend on the parts, so direct sweeps use one stream
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (parts > 1 && (e = cudaStreamIsCapturing(h->st, &cap)) != cudaSuccess) return e;
   if (parts > 1 && !ev && b->sts[0] && cap == cudaStreamCaptureStatusActive) {
@@ -1916,7 +1918,8 @@ bool batch_shape_ok(const mmc_batch* b, const DemagTuning& t, int band) {
 // Times every launch shape the batch can run with -- the row kernel with each
 // band that fits, the pass kernels with each x-pass row count and column-pass
 // width -- for `sweeps` sweeps from the current state, keeps the fastest and
-// puts the state back.  All shapes give bit-identical results.
+// puts the state back.  All shapes sample the same chain (mc_sep says which
+// Metropolis forms may round a trial in 1e10 apart).
 int batch_autotune(mmc_batch* b, int sweeps, double* best_ms, int* ncand) {
   mmc_handle* h = b->base;
   TRY(ensure_demag(h));
