@@ -345,8 +345,9 @@ __global__ void __launch_bounds__(256, x_w_min_blocks<A>()) k_x_inverse_w(FftPla
 // and read back twice), and the inverse's rows go straight to global memory.
 // Shared memory carries the transposes only, so the kernel has no barrier after
 // its table of roots, which it holds in the lanes' order (the products b ka of
-// the plain order meet in the same banks).  What bounded k_x_forward_w was the
-// shared-memory pipe (84 % busy at 64 x 256^2).
+// the plain order meet in the same banks).  64 x 256^2: 26.9 -> 23.7 us forward
+// and 28.5 -> 26.8 back; bound by the latency of its loads with the L1 path 70 to
+// 74 % busy (56 and 51 % issue).
 // SPLIT: m and h rows in the colour-split order (see k_mc_split): cell x of row
 // (y, z) at split_pos(x, y + z, nx); a lane's values have one parity (B and A
 // are even), so its addresses stay a base plus a compile-time step.
@@ -1832,7 +1833,7 @@ __global__ void __launch_bounds__(256) k_mc_quad(Geom g, const McCoef<T>* __rest
 // half were cells of no use to it.  Runs of at least MC_SPLIT_SWEEPS sweeps
 // convert m once at either end (k_split_rows); the x passes read and write the
 // split order at no cost.  Decisions: mc_propose / mc_accept on the same inputs
-// as every other form.  Latency and issue share the bound (58 % issue, loads the
+// as every other form but for mc_sep.  Latency and issue share the bound (58 % issue, loads the
 // top stall): the coefficients stay in shared memory so that 80 registers hold 24
 // warps per SM (102 registers and 16 warps with them in registers: 29 us; one
 // cell per thread, 32 warps: 31 us for its index work).  128 x 64^2: 17.6 -> 13.3
